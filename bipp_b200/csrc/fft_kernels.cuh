@@ -335,9 +335,9 @@ __global__ void __launch_bounds__(512, 2) fft_lines_kernel(FftLinePlan pl, FftLi
 
 using FftLinesKernel = void (*)(FftLinePlan, FftLines, const float2*);
 
-// Compiled radix sequences: the power of two 2^a (a = 4..9) as 4 x 4, 8 x 4, 16 x 4,
-// 16 x 8, 16 x 16, 16 x 8 x 4, or one odd radix 3, 5 or 7 followed by 16, 8 x 4, 16 x 4,
-// 16 x 8, 16 x 16, 16 x 8 x 4. Null when the sequence has no compiled kernel (the caller
+// Compiled radix sequences: the power of two 2^a (a = 4..10) as 4 x 4, 8 x 4, 16 x 4,
+// 16 x 8, 16 x 16, 16 x 8 x 4, 16 x 16 x 4, or one odd radix 3, 5 or 7 followed by 16,
+// 8 x 4, 16 x 4, 16 x 8, 16 x 16, 16 x 8 x 4, 16 x 16 x 4. Null when the sequence has no compiled kernel (the caller
 // then transforms with cuFFT).
 inline FftLinesKernel fft_lines_kernel_for(const int* radix, int ns, bool lineFast) {
   struct Entry {
@@ -347,9 +347,10 @@ inline FftLinesKernel fft_lines_kernel_for(const int* radix, int ns, bool lineFa
 #define B2_FFT_ENTRY(...) {{__VA_ARGS__}, fft_lines_kernel<false, __VA_ARGS__>, fft_lines_kernel<true, __VA_ARGS__>}
 #define B2_FFT_ODD(f)                                                                                          \
   B2_FFT_ENTRY(f, 16), B2_FFT_ENTRY(f, 8, 4), B2_FFT_ENTRY(f, 16, 4), B2_FFT_ENTRY(f, 16, 8),                 \
-      B2_FFT_ENTRY(f, 16, 16), B2_FFT_ENTRY(f, 16, 8, 4)
+      B2_FFT_ENTRY(f, 16, 16), B2_FFT_ENTRY(f, 16, 8, 4), B2_FFT_ENTRY(f, 16, 16, 4)
   static const Entry table[] = {B2_FFT_ENTRY(4, 4),  B2_FFT_ENTRY(8, 4),      B2_FFT_ENTRY(16, 4),
                                 B2_FFT_ENTRY(16, 8), B2_FFT_ENTRY(16, 16),    B2_FFT_ENTRY(16, 8, 4),
+                                B2_FFT_ENTRY(16, 16, 4),
                                 B2_FFT_ODD(3),       B2_FFT_ODD(5),           B2_FFT_ODD(7)};
 #undef B2_FFT_ODD
 #undef B2_FFT_ENTRY
