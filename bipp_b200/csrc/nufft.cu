@@ -335,10 +335,14 @@ void NufftCore::set_corr(bool on, double su, double sv) {
 void NufftCore::begin(double wmin, double wmax) {
   g_.wc = 0.5 * (wmin + wmax);
   const double Xw = std::max(0.5 * (wmax - wmin), 0.0);
-  g_.jc = (int)std::ceil(Xw / g_.hw + 0.5 * g_.W) + 1;
-  int nw = 2 * g_.jc + 1;
-  nw = ((nw + kTW - 1) / kTW) * kTW;
-  g_.nw = nw;
+  // Supports start at ceil(jc + t / hw - W / 2) for |t| <= Xw: jc is the smallest index
+  // whose lowest support starts at plane 0, and planes() counts up to the highest support's
+  // end (1e-6 of a plane covers the rounding of t). Planes past planes() of the last tile
+  // layer hold no point and are neither transformed nor summed.
+  const double xw = Xw / g_.hw;
+  g_.jc = std::max(0, (int)std::ceil(xw + 0.5 * g_.W - 1.0 + 1e-6));
+  planes_ = (int)std::ceil(g_.jc + xw - 0.5 * g_.W + 1e-6) + g_.W;
+  g_.nw = ((planes_ + kTW - 1) / kTW) * kTW;
   g_.ntx = g_.nx / kTX;
   g_.nty = g_.ny / kTY;
   g_.ntw = g_.nw / kTW;
@@ -584,11 +588,15 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
           {{launch_spread_tc<8, 1, false, false>, launch_spread_tc<8, 2, false, false>},
            {launch_spread_tc<8, 1, true, false>, launch_spread_tc<8, 2, true, false>},
            {launch_spread_tc<8, 1, false, true>, launch_spread_tc<8, 2, false, true>}}};
-      const L launch = table[nch_ <= 4 ? 0 : 1][operands][two ? 1 : 0];
-      launch(g_, nItems, ctx_->stream, offsets_.get<int>(), rec_.get<PtRec>(), vals_.get<float2>(), valStride_, nch_,
-             items_.get<SpreadItem>() + slabBegin[sl], tw0, slabPlanes, grid_.get<float2>(), errFlag_.get<int>(),
-             dynamic ? workCounters_.get<int>() + sl : nullptr, valScale_.get<unsigned>());
-      B2_CHECK_LAUNCH();
+      for (int c0 = 0, grp = 0; c0 < nch_; c0 += kTcMaxChan, ++grp) {
+        const int nc = std::min(kTcMaxChan, nch_ - c0);
+        const L launch = table[nc <= 4 ? 0 : 1][operands][two ? 1 : 0];
+        launch(g_, nItems, ctx_->stream, offsets_.get<int>(), rec_.get<PtRec>(), vals_.get<float2>() + c0, nch_, nc,
+               items_.get<SpreadItem>() + slabBegin[sl], tw0, slabPlanes,
+               grid_.get<float2>() + slab_index(g_, nch_, slabPlanes, c0, 0, 0, 0), errFlag_.get<int>(),
+               dynamic ? workCounters_.get<int>() + sl + grp * nslab : nullptr, valScale_.get<unsigned>() + c0);
+        B2_CHECK_LAUNCH();
+      }
     } else if (nItems > 0) {
       const SpreadItem* it = items_.get<SpreadItem>() + slabBegin[sl];
       if (nch_ <= 4)
@@ -600,12 +608,13 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
       B2_CHECK_LAUNCH();
     }
     if (stageMs) B2_CUDA(cudaEventRecord(ev[1], ctx_->stream));
-    inverse_fft(slabPlanes, tiles * kTW, grid_.get<float2>(), prunedFft);
+    const int planesUsed = std::min(tiles * kTW, planes_ - tw0 * kTW);
+    inverse_fft(slabPlanes, planesUsed, grid_.get<float2>(), prunedFft);
     if (stageMs) B2_CUDA(cudaEventRecord(ev[2], ctx_->stream));
     const int blocks = (int)std::min<long long>((P + 255) / 256, 65535);
     count_launch();
     auto wk = nch_ <= 4 ? wsum_kernel<4> : wsum_kernel<kMaxChan>;
-    wk<<<blocks, 256, 0, ctx_->stream>>>(g_, grid_.get<float2>(), nch_, slabPlanes, tw0 * kTW, tiles * kTW,
+    wk<<<blocks, 256, 0, ctx_->stream>>>(g_, grid_.get<float2>(), nch_, slabPlanes, tw0 * kTW, planesUsed,
                                          nTilde_.get<double>(), acc_.get<float2>(), P, prunedFft ? 1 : 0);
     B2_CHECK_LAUNCH();
     if (stageMs) {

@@ -91,6 +91,7 @@ private:
   bool fftPlansOk_ = false;
   DevBuf fftTw_;
   int slabTiles_ = 1;
+  int planes_ = 0;    // w-planes that supports of the current transform reach
   // inverse 2-D FFT of the first planesUsed planes of every channel of the slab: pruned
   // (cell (a, b) of a plane then holds pixel (a, b)'s output) or in full by cuFFT
   void inverse_fft(int slabPlanes, int planesUsed, float2* slab, bool pruned);
