@@ -401,7 +401,7 @@ static void launch_spread(const NufftGeom& g, int nItems, size_t smem, cudaStrea
 // memory allows
 template <int CH, int STAGES, bool AT, bool F16>
 static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, const int* offs, const PtRec* rec,
-                             const float2* vals, long long vs, int nch, const SpreadItem* items, int tw0,
+                             const float2* vals, int chStride, int nch, const SpreadItem* items, int tw0,
                              int slabPlanes, float2* out, int* errFlag, int* workCounter, const unsigned* valScale) {
   using S = TcShape<CH, STAGES, AT, F16>;
   int dev = 0, sms = 148;
@@ -413,14 +413,16 @@ static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, co
   const int grid = std::max(1, std::min(nItems, sms * std::min(S::MinBlocks, tuned("spread.ctas_per_sm"))));
   count_launch();
   spread_tc_kernel<CH, STAGES, AT, F16><<<grid, kTcThreads, S::Smem, st>>>(
-      g, offs, rec, vals, vs, nch, items, nItems, tw0, slabPlanes, out, errFlag, workCounter, valScale);
+      g, offs, rec, vals, chStride, nch, items, nItems, tw0, slabPlanes, out, errFlag, workCounter, valScale);
 }
 
-// BIPP_B200_SPREAD=warp selects the shared-memory-atomic spreader for every channel count
-static bool use_tensor_core_spread(int nch) {
+// BIPP_B200_SPREAD=warp selects the shared-memory-atomic spreader for every channel count.
+// More than 8 channels (four images with their first-order lattice channels: 12) take one
+// tensor-core launch of 8 and one of 4; the points' kernel values are then formed twice,
+// which still leaves the atomics of the other spreader far behind.
+static bool use_tensor_core_spread() {
   const char* e = std::getenv("BIPP_B200_SPREAD");
-  if (e && std::string(e) == "warp") return false;
-  return nch <= kTcMaxChan;
+  return !(e && std::string(e) == "warp");
 }
 
 
@@ -466,7 +468,7 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
   // the tensor-core spreader writes every tile it spreads in one part; the other tiles of a
   // slab (empty, or split into parts that accumulate with atomics) are cleared first from
   // a compact list; the warp spreader works on a cleared slab
-  const bool tc = use_tensor_core_spread(nch_);
+  const bool tc = use_tensor_core_spread();
   const bool prunedFft = fftPlansOk_ && tuned("nufft.fft") == 1;
   const int tb = std::min(8192, (ntiles + 255) / 256);
   clearFlag_.ensure(ctx_, (size_t)ntiles * sizeof(int));
@@ -528,8 +530,10 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
                                             itemsAlt_.get<SpreadItem>(), nItemsAll, 0, endBit, ctx_->stream));
     B2_CUDA(cudaMemcpyAsync(items_.get(), itemsAlt_.get(), (size_t)nItemsAll * sizeof(SpreadItem),
                             cudaMemcpyDeviceToDevice, ctx_->stream));
-    workCounters_.ensure(ctx_, (size_t)std::max(1, nslab) * sizeof(int));
-    B2_CUDA(cudaMemsetAsync(workCounters_.get(), 0, (size_t)std::max(1, nslab) * sizeof(int), ctx_->stream));
+    // a counter per slab and channel group
+    const size_t counters = (size_t)std::max(1, nslab) * ((nch_ + kTcMaxChan - 1) / kTcMaxChan);
+    workCounters_.ensure(ctx_, counters * sizeof(int));
+    B2_CUDA(cudaMemsetAsync(workCounters_.get(), 0, counters * sizeof(int), ctx_->stream));
   }
   {
     int total = 0, split = 0;

@@ -26,7 +26,7 @@ constexpr int kTcThreads = 128;
 constexpr int kTcVisits = 16;                 // visits per phase
 constexpr int kTcSteps = kTcVisits / 8;       // MMA K-steps per phase (K = 8 for tf32)
 constexpr int kTcM = kTX * kTY;               // 128 accumulator rows (cells)
-constexpr int kTcMaxChan = 8;                 // channels handled by the tensor-core kernel
+constexpr int kTcMaxChan = 8;                 // channels of one launch of the tensor-core kernel
 // shared-memory layout (bytes); one K-step of A is 128 rows x 8 tf32
 constexpr int kTcAStep = kTcM * 8 * 4;
 // per-visit kernel values at every tile position (zero outside the support) and the
@@ -119,12 +119,15 @@ __device__ __forceinline__ int tc_range_pair(int j) {
   return -1;
 }
 
+// The nch <= CH channels of one launch are consecutive ones of chStride channels per point:
+// more than 8 channels are spread by several launches, vals, valScale and grid pointing at
+// each launch's first channel.
 // Persistent: each CTA takes work items blockIdx.x, blockIdx.x + gridDim.x, ... or, with
 // a work counter, the next item of the (load-ordered) list whenever it is free
 template <int CH, int STAGES, bool AT = false, bool F16 = false>
 static __global__ void __launch_bounds__(kTcThreads, TcShape<CH, STAGES, AT, F16>::MinBlocks)
 spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __restrict__ rec,
-                 const float2* __restrict__ vals, long long valStride, int nch, const SpreadItem* __restrict__ items,
+                 const float2* __restrict__ vals, int chStride, int nch, const SpreadItem* __restrict__ items,
                  int nItems, int tw0, int slabPlanes, float2* __restrict__ grid, int* __restrict__ errFlag,
                  int* __restrict__ workCounter, const unsigned* __restrict__ valScale = nullptr) {
   using S = TcShape<CH, STAGES, AT, F16>;
@@ -255,7 +258,7 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
 #pragma unroll
           for (int cc = 0; cc < CPR; ++cc) {
             const int c = CPR * (pa - 6) + cc;
-            pfX[cc] = (c < nch) ? vals[(long long)p * nch + c] : make_float2(0.f, 0.f);
+            pfX[cc] = (c < nch) ? vals[(long long)p * chStride + c] : make_float2(0.f, 0.f);
           }
         }
       }
