@@ -1,0 +1,117 @@
+"""Kernels at the sizes where they can go wrong (tile edges, remainders, the smallest and
+largest of a range), against FP64 numpy/scipy of the same definition."""
+import math
+
+import numpy as np
+import pytest
+
+from oracle import bluebild as bb
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel_l2(a, b):
+    return np.linalg.norm(np.asarray(a, np.float64) - b) / max(np.linalg.norm(b), 1e-300)
+
+
+def _points(rng, n, umax, wmax, images):
+    u, v = rng.uniform(-umax, umax, (2, n))
+    w = rng.uniform(-wmax, wmax, n) if wmax else np.zeros(n)
+    c = rng.standard_normal((n, images)) + 1j * rng.standard_normal((n, images))
+    return np.stack([u, v, w], 1).astype(np.float32), c.astype(np.complex64)
+
+
+def _check_nufft(ctx, lmn, uvw, c, tol, bound):
+    import bipp_b200 as bipp
+
+    plan = bipp.NufftSynthesis(ctx, bipp.NufftSynthesisOptions().set_tolerance(tol), lmn, c.shape[1], uvw.shape[0])
+    plan.add(uvw, c)
+    l64, uvw64 = lmn.astype(np.float64), uvw.astype(np.float64)
+    pix = np.random.default_rng(3).choice(lmn.shape[0], min(lmn.shape[0], 3000), replace=False)
+    for i in range(c.shape[1]):
+        ref = bb.nuft_sum(1.0, c[:, i].astype(np.complex128), uvw64[:, 0], uvw64[:, 1], uvw64[:, 2], l64[pix, 0],
+                          l64[pix, 1], l64[pix, 2])
+        assert _rel_l2(plan.get_image(i)[pix], ref) <= bound, i
+    plan.close()
+
+
+@pytest.mark.parametrize("images", [3, 4])
+@pytest.mark.parametrize("tol", [1e-3, 1e-5, 1e-7])
+def test_spread_more_than_eight_channels(ctx, images, tol):
+    """9 and 12 channels (3 and 4 images with their first-order lattice channels): two
+    tensor-core spreading launches. Bound as for up to 8 channels: 20 tolerances, at least 2e-6."""
+    from bipp_b200 import simulate as sim
+
+    rng = np.random.default_rng(21)
+    lmn = sim.make_lmn_grid(45, math.radians(12.0)).astype(np.float32)
+    uvw, c = _points(rng, 900, 4000.0, 200.0, images)
+    _check_nufft(ctx, lmn, uvw, c, tol, max(20 * tol, 2e-6))
+
+
+@pytest.mark.parametrize("px", [585, 1755, 2926, 4096])
+def test_fft_lines_with_factor_1024(ctx, px):
+    """Image widths whose fine grid is 1024 times 1, 3, 5 or 7 (radices .., 16, 16, 4)."""
+    rng = np.random.default_rng(22)
+    na = 9
+    a, b = np.meshgrid(np.arange(na), np.arange(px), indexing="ij")
+    for transposed in (False, True):
+        l = (b.reshape(-1) - px / 2 + 0.5) * (0.2 / px)
+        m = (a.reshape(-1) - na / 2 + 0.25) * (0.02 / na)
+        if transposed:
+            l, m = (l.reshape(na, px).T.reshape(-1), m.reshape(na, px).T.reshape(-1))
+        lmn = np.stack([l, m, np.sqrt(1 - l * l - m * m)], 1).astype(np.float32)
+        uvw, c = _points(rng, 500, 500.0, 20.0, 1)
+        _check_nufft(ctx, lmn, uvw, c, 1e-6, 2e-5)
+
+
+@pytest.mark.parametrize("tol", [1e-2, 1e-4, 1e-5, 1e-6])
+@pytest.mark.parametrize("wmax", [0.0, 30.0, 333.0, 2500.0])
+def test_w_planes(ctx, wmax, tol):
+    """No w extent at all, and extents whose planes end at different places of a tile layer."""
+    from bipp_b200 import simulate as sim
+
+    rng = np.random.default_rng(23)
+    lmn = sim.make_lmn_grid(33, math.radians(16.0)).astype(np.float32)
+    uvw, c = _points(rng, 400, 1500.0, wmax, 1)
+    _check_nufft(ctx, lmn, uvw, c, tol, 20 * tol)
+
+
+@pytest.mark.parametrize("n_in,n_out", [(1, 1), (255, 257), (256, 256), (257, 300), (9000, 65)])
+@pytest.mark.parametrize("double", [False, True])
+def test_direct_sum_sizes(ctx, n_in, n_out, double):
+    """FP32: sine and cosine within 2^-20 each and the FP32 result, so 2e-6 of the summed
+    magnitudes. FP64: phases below 2e3 rounded to 2^-52 of that, 1e-11 of them."""
+    import bipp_b200 as bipp
+
+    rng = np.random.default_rng(n_in + n_out)
+    rt, ct = (np.float64, np.complex128) if double else (np.float32, np.complex64)
+    u = rng.uniform(-900, 900, (3, n_in)).astype(rt)
+    x = rng.uniform(-1, 1, (3, n_out)).astype(rt)
+    v = (rng.standard_normal(n_in) + 1j * rng.standard_normal(n_in)).astype(ct)
+    out = bipp.nuft_sum(rt(1.25), v, u[0], u[1], u[2], x[0], x[1], x[2], ctx=ctx)
+    ref = (np.exp(1j * 1.25 * (x.astype(np.float64).T @ u.astype(np.float64))) @ v.astype(np.complex128)).real
+    assert np.abs(out - ref).max() <= (1e-11 if double else 2e-6) * np.abs(v).sum()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e30])
+def test_direct_sum_out_of_range(ctx, bad):
+    """A non-finite input coordinate or value reaches every output as NaN; a huge finite one
+    stays finite; a non-finite pixel only its own output."""
+    import bipp_b200 as bipp
+
+    rng = np.random.default_rng(7)
+    base = [rng.uniform(-1, 1, 300).astype(np.float32) for _ in range(3)]
+    pix = [rng.uniform(-1, 1, 40).astype(np.float32) for _ in range(3)]
+    val = np.ones(300, np.complex64)
+    u = base[0].copy()
+    u[17] = bad
+    out = bipp.nuft_sum(np.float32(1.0), val, u, base[1], base[2], *pix, ctx=ctx)
+    assert np.isfinite(out).all() if bad == 1e30 else np.isnan(out).all()
+    if bad != 1e30:
+        v = val.copy()
+        v[3] = bad
+        assert not np.isfinite(bipp.nuft_sum(np.float32(1.0), v, *base, *pix, ctx=ctx)).any()
+        x = pix[0].copy()
+        x[5] = bad
+        out = bipp.nuft_sum(np.float32(1.0), val, *base, x, pix[1], pix[2], ctx=ctx)
+        assert np.isnan(out[5]) and np.isfinite(np.delete(out, 5)).all()
