@@ -265,8 +265,11 @@ void NufftCore::setup(bipp_ctx_s* ctx, const Lattice& lat, const std::vector<dou
   es_params(eps, sigma, g_.W, g_.beta);
   g_.nx = next_smooth((int)std::ceil(sigma * g_.Nb));
   g_.ny = next_smooth((int)std::ceil(sigma * g_.Na));
-  g_.nx = std::max(g_.nx, 2 * g_.W);
-  g_.ny = std::max(g_.ny, 2 * g_.W);
+  // at least two tiles along each axis: with one, a support that wraps would meet its own
+  // tile as the neighbour
+  g_.nx = std::max(g_.nx, 2 * kTX);
+  g_.ny = std::max(g_.ny, 2 * kTY);
+  static_assert(kMaxW <= kTX && kMaxW <= kTY + 1, "two tiles hold twice a support");
   g_.hx = 2.0 * M_PI / g_.nx;
   g_.hy = 2.0 * M_PI / g_.ny;
   fftPlansOk_ = make_fft_plan(g_.nx, g_.Nb, false, rowPlan_, rowKernel_) &&
@@ -419,10 +422,13 @@ static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, co
 // BIPP_B200_SPREAD=warp selects the shared-memory-atomic spreader for every channel count.
 // More than 8 channels (four images with their first-order lattice channels: 12) take one
 // tensor-core launch of 8 and one of 4; the points' kernel values are then formed twice,
-// which still leaves the atomics of the other spreader far behind.
-static bool use_tensor_core_spread() {
+// which still leaves the atomics of the other spreader far behind (1024^2 px, 16 x 512^2
+// points: 40.5 ms). Below a tolerance of 1e-5 the FP16 hi/lo operands show beside the
+// transform's own error (2 % of it at 1e-6, 0.02 % at 1e-5), so those keep FP32 sums.
+static bool use_tensor_core_spread(int nch, double eps) {
   const char* e = std::getenv("BIPP_B200_SPREAD");
-  return !(e && std::string(e) == "warp");
+  if (e && std::string(e) == "warp") return false;
+  return nch <= kTcMaxChan || eps >= 1e-5;
 }
 
 
@@ -468,7 +474,7 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
   // the tensor-core spreader writes every tile it spreads in one part; the other tiles of a
   // slab (empty, or split into parts that accumulate with atomics) are cleared first from
   // a compact list; the warp spreader works on a cleared slab
-  const bool tc = use_tensor_core_spread();
+  const bool tc = use_tensor_core_spread(nch_, eps_);
   const bool prunedFft = fftPlansOk_ && tuned("nufft.fft") == 1;
   const int tb = std::min(8192, (ntiles + 255) / 256);
   clearFlag_.ensure(ctx_, (size_t)ntiles * sizeof(int));
