@@ -11,6 +11,7 @@
 #include "rank_mlp.cuh"
 #include "tune.hpp"
 #include "eig_kernels.cuh"
+#include "chol_kernels.cuh"
 #include "gemm_tc.cuh"
 
 namespace bippb200 {
@@ -222,32 +223,22 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
   if (L.gram) {
     mark(1);
     if (realG) {
-      auto k = cholesky_kernel<double>;
-      smem_optin(k, chol_smem<double>());
-      count_launch();
-      k<<<nb, kCholThreads, chol_smem<double>(), st>>>(reinterpret_cast<double*>(G), nred, Nmax,
-                                                        L.status + L.batchOffset, sizeOrder);
+      chol_inverse<R>(st, reinterpret_cast<double*>(G), reinterpret_cast<double*>(W64), reinterpret_cast<R*>(Linv), nred,
+                      nb, L.nBeam, Nmax, L.status + L.batchOffset);
+      mark(2);
     } else {
       auto k = cholesky_kernel<double2>;
       smem_optin(k, kCholSmem);
       count_launch();
       k<<<nb, kCholThreads, kCholSmem, st>>>(G, nred, Nmax, L.status + L.batchOffset, sizeOrder);
-    }
-    B2_CHECK_LAUNCH();
-    mark(2);
-    if (realG) {
-      auto k = trinv_kernel<double, R>;
-      smem_optin(k, trinv_smem<double>());
+      B2_CHECK_LAUNCH();
+      mark(2);
+      auto ki = trinv_kernel<double2, C>;
+      smem_optin(ki, kTrinvSmem);
       count_launch();
-      k<<<nb, 256, trinv_smem<double>(), st>>>(reinterpret_cast<const double*>(G), reinterpret_cast<double*>(W64),
-                                               reinterpret_cast<R*>(Linv), nred, Nmax, sizeOrder);
-    } else {
-      auto k = trinv_kernel<double2, C>;
-      smem_optin(k, kTrinvSmem);
-      count_launch();
-      k<<<nb, 256, kTrinvSmem, st>>>(G, W64, Linv, nred, Nmax, sizeOrder);
+      ki<<<nb, 256, kTrinvSmem, st>>>(G, W64, Linv, nred, Nmax, sizeOrder);
+      B2_CHECK_LAUNCH();
     }
-    B2_CHECK_LAUNCH();
     // T1 = Linv * A (Linv real for W = I)
     mark(3);
     GemmArgs<C> g1{};

@@ -115,3 +115,53 @@ def test_direct_sum_out_of_range(ctx, bad):
         x[5] = bad
         out = bipp.nuft_sum(np.float32(1.0), val, *base, x, pix[1], pix[2], ctx=ctx)
         assert np.isnan(out[5]) and np.isfinite(np.delete(out, 5)).all()
+
+
+def _steps(rng, b, n, dtype):
+    """b Hermitian visibility matrices of n antennas (sources plus noise) and positions with
+    every pair at least half a wavelength apart."""
+    side = int(math.ceil(math.sqrt(n)))
+    grid = np.stack(np.meshgrid(np.arange(side), np.arange(side)), -1).reshape(-1, 2)[:n] * 3.0
+    xyz = np.zeros((b, n, 3))
+    xyz[:, :, :2] = grid + rng.uniform(-0.9, 0.9, (b, n, 2))
+    q = 8
+    dirs = rng.standard_normal((b, q, 3)) * 0.1
+    a = np.exp(1j * np.pi * np.einsum("bqc,bnc->bnq", dirs, xyz))
+    noise = rng.standard_normal((b, n, n)) + 1j * rng.standard_normal((b, n, n))
+    s = np.einsum("bnq,q,bmq->bnm", a, rng.uniform(1, 20, q), a.conj()) + 0.05 * (noise + noise.conj().transpose(0, 2, 1))
+    return s.astype(dtype), xyz
+
+
+@pytest.mark.parametrize("n,b", [(1, 3), (2, 1), (31, 2), (33, 5), (63, 1), (64, 2), (65, 2), (96, 1), (127, 3), (129, 1),
+                                 (200, 2), (257, 1), (321, 1), (513, 1), (40, 400), (130, 40)])
+@pytest.mark.parametrize("precision", ["single", "double"])
+def test_eigh_gram_sizes(ctx, n, b, precision):
+    """Sizes around the tiles and panels of the Cholesky factor, inverse, tridiagonalisation
+    and eigenpairs, alone and in batches. Eigenvalues against scipy's FP64 solver on the same
+    inputs, and G-orthonormal eigenvectors that reconstruct S: normwise 64 eps sqrt(n) for
+    FP64 and 32 eps sqrt(n) for FP32 (a backward stable solver stays below n eps)."""
+    import scipy.linalg
+
+    import bipp_b200 as bipp
+
+    rng = np.random.default_rng(1000 * n + b)
+    dbl = precision == "double"
+    s, xyz = _steps(rng, b, n, np.complex128 if dbl else np.complex64)
+    wl = np.full(b, 2.0)
+    v, d, nred, _ = bipp.eigh_gram_batched(wl, s, xyz, ctx=ctx, precision=precision)
+    assert (nred == n).all()
+    eps = np.finfo(np.float64 if dbl else np.float32).eps
+    tol = (64 if dbl else 32) * eps * math.sqrt(n)
+    for k in sorted(set([0, b // 2, b - 1])):
+        x = xyz[k] if dbl else xyz[k].astype(np.float32).astype(np.float64)
+        g = np.sinc(np.linalg.norm(x[:, None] - x[None], axis=2))
+        s64 = np.tril(s[k]).astype(np.complex128)
+        s64 = s64 + np.tril(s64, -1).conj().T
+        np.fill_diagonal(s64, s64.diagonal().real)
+        ref = scipy.linalg.eigh(s64, g, eigvals_only=True)
+        scale = np.abs(ref).max()
+        cond = np.linalg.cond(g)
+        assert np.abs(d[k] - ref).max() <= tol * scale * max(1.0, math.sqrt(cond)), k
+        vk = v[k].astype(np.complex128)
+        assert np.linalg.norm(vk.conj().T @ g @ vk - np.eye(n)) <= tol * n * cond, k
+        assert np.linalg.norm(g @ (vk * d[k]) @ vk.conj().T @ g - s64) <= tol * n * cond * scale, k
