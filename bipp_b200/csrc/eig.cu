@@ -13,6 +13,7 @@
 #include "eig_kernels.cuh"
 #include "chol_kernels.cuh"
 #include "gemm_tc.cuh"
+#include "tridiag_kernels.cuh"
 
 namespace bippb200 {
 
@@ -162,6 +163,7 @@ void EigWork<T>::reserve(bipp_ctx_s* ctx, int nBatch, int nmax) {
   e.alloc(ctx, (size_t)nmax * sizeof(double) * nBatch);
   tau.alloc(ctx, (size_t)nmax * sizeof(C) * nBatch);
   krange.alloc(ctx, (size_t)2 * sizeof(int) * nBatch);
+  range.alloc(ctx, (size_t)2 * sizeof(int) * nBatch);
   order.alloc(ctx, (size_t)sizeof(int) * nBatch);
 }
 
@@ -335,20 +337,45 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
   }
   // 4. tridiagonal eigenpairs (FP64); workspace aliases W64 (free after trinv)
   mark(5);
-  {
+  double* lam = L.lam + (long long)L.batchOffset * Nmax;
+  if (L.mlpModel) {
+    // the predicted partial solve, whose size and fallbacks depend on its own results, stays
+    // in one kernel per matrix
     const size_t smem = 4 * (size_t)Nmax * sizeof(double);
     auto k = tridiag_kernel<R>;
     smem_optin(k, smem);
     count_launch();
-    // threads per matrix (tunable): by default 128 when only the eigenpairs of a range are
-    // computed (one lane per eigenvalue leaves most of 256 idle, and 128-thread CTAs put
-    // twice the matrices on an SM), 256 for every eigenpair
-    const int tt = tuned("tridiag.threads");
-    const int triThreads = tt > 0 ? tt : (L.allValues ? kTriThreads : kTriThreads / 2);
-    k<<<nb, triThreads, smem, st>>>(w.d.template get<double>(), w.e.template get<double>(), nred, Nmax,
-                                     L.lam + (long long)L.batchOffset * Nmax, Z, reinterpret_cast<double*>(W64),
-                                     L.status + L.batchOffset, L.vecLo, L.vecHi, krange, L.allValues, sizeOrder,
-                                     L.mlpModel ? L.predK : nullptr, L.predMargin, L.resTol);
+    k<<<nb, kTriThreads / 2, smem, st>>>(w.d.template get<double>(), w.e.template get<double>(), nred, Nmax, lam, Z,
+                                         reinterpret_cast<double*>(W64), L.status + L.batchOffset, L.vecLo, L.vecHi,
+                                         krange, L.allValues, sizeOrder, L.predK, L.predMargin, L.resTol);
+    B2_CHECK_LAUNCH();
+  } else {
+    // lanes per eigenvalue: double them while the batch's lanes stay within 1024 per SM
+    // (tunable), beyond which more cuts per sweep only repeat work; a range of eigenvalues
+    // is taken as half of them
+    const int perSm = tuned("tridiag.threads");
+    const long long lanes = (long long)(perSm > 0 ? perSm : 1024) * ctx->smCount;
+    const long long values = (long long)nb * std::max(1, L.allValues ? Nmax : Nmax / 2);
+    int M = 1;
+    while (M < 32 && 2 * M * values <= lanes) M *= 2;
+    const size_t smem = (size_t)Nmax * sizeof(double2);
+    int* range = w.range.template get<int>();
+    smem_optin(tridiag_values_kernel, smem);
+    count_launch();
+    tridiag_values_kernel<<<dim3((Nmax * M + kTsThreads - 1) / kTsThreads, nb), kTsThreads, smem, st>>>(
+        w.d.template get<double>(), w.e.template get<double>(), nred, Nmax, L.vecLo, L.vecHi, L.allValues, M, lam, range,
+        sizeOrder);
+    B2_CHECK_LAUNCH();
+    auto k = tridiag_vectors_kernel<R>;
+    smem_optin(k, smem);
+    count_launch();
+    k<<<dim3((2 * Nmax + kTsThreads - 1) / kTsThreads, nb), kTsThreads, smem, st>>>(
+        w.d.template get<double>(), w.e.template get<double>(), nred, Nmax, lam, L.vecLo, L.vecHi, range, krange, Z,
+        reinterpret_cast<double*>(W64), sizeOrder);
+    B2_CHECK_LAUNCH();
+    count_launch();
+    tridiag_clusters_kernel<R><<<nb, 256, 0, st>>>(w.d.template get<double>(), w.e.template get<double>(), nred, Nmax,
+                                                   lam, krange, Z, L.status + L.batchOffset);
     B2_CHECK_LAUNCH();
   }
   // 5. back-transform Y = Q Z -> T1

@@ -1,0 +1,376 @@
+// Eigenpairs of a batch of real symmetric tridiagonal matrices in FP64: bisection for the
+// eigenvalues, twisted factorisations for the eigenvectors, in three launches over
+// (matrix, eigenvalue chunk) (sm_100a).
+//
+// The reference leaves this to LAPACK's ?hegv (src/host/lapack_api.hpp:112-158). Both the
+// Sturm counts and the factorisations are n-step recurrences, so the time of a matrix is
+// the latency of its serial chain, not arithmetic or bytes. One CTA per matrix with the
+// quotient form q_k = (d_k - x) - e_k^2 / q_{k-1} paid a dependent FP64 division per step
+// and 53 bisection steps (6.0 ms for one matrix of 550 rows, 13.5 ms for 2048 matrices of
+// 380-512 rows). Here
+//  - the recurrences run on p_k = (d_k - x) p_{k-1} - e_{k-1}^2 p_{k-2} (q_k = p_k / p_{k-1}),
+//    one dependent FMA per step; p is rescaled every 8 steps. Each step's rounding is a
+//    relative perturbation of d_k - x and e_{k-1}^2, as in the quotient form. The matrix is
+//    scaled by a power of two to a norm in [1/2, 1), so 8 steps stay far inside FP64 range;
+//  - a CTA first counts at 128 points across the whole interval in one sweep, which gives
+//    every eigenvalue its starting interval; then M lanes per eigenvalue cut it M + 1 ways
+//    per sweep. M (1..32) is chosen so that the lanes of the batch fill the GPU once:
+//    more lanes only repeat work when the batch fills it already;
+//  - the two factorisations of an eigenvector, from the top and from the bottom, run in two
+//    lanes at once, their quotients off the chain.
+#pragma once
+
+#include "common.cuh"
+
+namespace bippb200 {
+
+constexpr int kTsThreads = 128;
+
+// quotient replaced by -2^-100 (of the scaled matrix) when a pivot is exactly zero
+constexpr double kTsTiny = 7.888609052210118e-31;
+
+// p replaced when zero, so that p / prev = -2^-100
+__device__ __forceinline__ double ts_nonzero(double p, double prev) {
+  return (__double2hiint(p) & 0x7fffffff) == 0 ? -kTsTiny * prev : p;
+}
+
+// common power-of-two factor that brings the larger of |a|, |b| to [1, 2)
+__device__ __forceinline__ void ts_rescale(double& a, double& b) {
+  const int ha = __double2hiint(a) & 0x7ff00000, hb = __double2hiint(b) & 0x7ff00000;
+  const double s = __hiloint2double(0x7fe00000 - max(ha, hb), 0);
+  a *= s;
+  b *= s;
+}
+
+// eigenvalues of the scaled matrix below x; de[k] = (d_k, e_{k-1}^2), de[0].y unused
+__device__ __forceinline__ int ts_count(const double2* __restrict__ de, int n, double x) {
+  double p0 = 1.0, p1 = ts_nonzero(de[0].x - x, 1.0);
+  unsigned cnt = (unsigned)__double2hiint(p1) >> 31;
+  int k = 1;
+  auto step = [&](double2 v) {
+    const double p2 = ts_nonzero(fma(v.x - x, p1, -v.y * p0), p1);
+    cnt += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+    p0 = p1;
+    p1 = p2;
+  };
+  for (; k + 8 <= n; k += 8) {
+    ts_rescale(p0, p1);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) step(de[k + u]);
+  }
+  ts_rescale(p0, p1);
+  for (; k < n; ++k) step(de[k]);
+  return (int)cnt;
+}
+
+// Load a matrix scaled by `scale` = 2^-k (norm in [1/2, 1)) and its Gershgorin interval
+// [lo, hi] (scaled); red: 32 doubles. Returns with every thread synchronised.
+__device__ __forceinline__ void ts_load(const double* __restrict__ d, const double* __restrict__ e, int n,
+                                        double2* __restrict__ de, double* red, double& lo, double& hi, double& tnorm,
+                                        double& scale) {
+  double l = 1e300, h = -1e300;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    const double ek = k < n - 1 ? fabs(e[k]) : 0.0, em = k > 0 ? fabs(e[k - 1]) : 0.0;
+    l = fmin(l, d[k] - (ek + em));
+    h = fmax(h, d[k] + (ek + em));
+  }
+  l = block_min(l, red, 1e300);
+  __syncthreads();
+  h = block_max(h, red, -1e300);
+  const double t = fmax(fabs(l), fabs(h));
+  // exponent field of t, kept where both 2^-k and its square products are normal
+  const int ex = min(max((__double2hiint(t) >> 20) & 0x7ff, 200), 1800);
+  scale = __hiloint2double((2045 - ex) << 20, 0);   // 2^(1022 - ex): t scale in [1/2, 1)
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    const double em = k > 0 ? e[k - 1] * scale : 0.0;
+    de[k] = make_double2(d[k] * scale, em * em);
+  }
+  tnorm = t * scale;
+  const double slack = 4.0 * 2.220446049250313e-16 * tnorm + 1e-290;
+  lo = l * scale - slack;
+  hi = h * scale + slack;
+  __syncthreads();
+}
+
+// Eigenvalues: all of them, or (allValues == 0) those in [vecLo, vecHi], whose index range
+// two Sturm counts give; the others come out as zero. CTA (c, r): chunk c of
+// kTsThreads / M eigenvalues of the matrix of rank r in `order`. range[2b], range[2b+1]:
+// the index range. Dynamic shared memory: Nmax double2.
+__global__ void __launch_bounds__(kTsThreads)
+tridiag_values_kernel(const double* __restrict__ dIn, const double* __restrict__ eIn, const int* __restrict__ nred,
+                      int Nmax, double vecLo, double vecHi, int allValues, int M, double* __restrict__ lamOut,
+                      int* __restrict__ range, const int* __restrict__ order) {
+  const int b = order ? order[blockIdx.y] : blockIdx.y;
+  const int n = nred[b];
+  if (n <= 0) return;
+  extern __shared__ __align__(16) double2 ts_smem[];
+  double2* de = ts_smem;
+  __shared__ double red[32];
+  __shared__ int cA[kTsThreads], sRange[2];
+  const int tid = threadIdx.x;
+  double lo, hi, tnorm, scale;
+  ts_load(dIn + (long long)b * Nmax, eIn + (long long)b * Nmax, n, de, red, lo, hi, tnorm, scale);
+  if (allValues) {
+    if (tid < 2) sRange[tid] = tid ? n : 0;
+  } else if (tid < 2) {
+    const double x = (tid ? vecHi : vecLo) * scale;
+    // bounds beyond the interval keep every eigenvalue on that side
+    sRange[tid] = tid ? (x < hi ? ts_count(de, n, x) : n) : (x > lo ? ts_count(de, n, x) : 0);
+  }
+  __syncthreads();
+  const int vLo = sRange[0], vHi = max(sRange[0], sRange[1]);
+  double* lam = lamOut + (long long)b * Nmax;
+  if (blockIdx.x == 0) {
+    for (int i = tid; i < n; i += kTsThreads)
+      if (i < vLo || i >= vHi) lam[i] = 0.0;
+    if (tid == 0) {
+      range[2 * b] = vLo;
+      range[2 * b + 1] = vHi;
+    }
+  }
+  const int perCta = kTsThreads / M;
+  const int i0 = vLo + blockIdx.x * perCta;
+  if (i0 >= vHi) return;
+  const double eps = 2.220446049250313e-16;
+  if (!allValues) {
+    const double a = vecLo * scale, c = vecHi * scale;
+    if (a > lo) lo = a - (2.0 * eps * fabs(a) + 1e-290);
+    if (c < hi) hi = c + (2.0 * eps * fabs(c) + 1e-290);
+  }
+  const double w = (hi - lo) / (kTsThreads + 1);
+  cA[tid] = ts_count(de, n, lo + w * (tid + 1));
+  __syncthreads();
+  const int i = i0 + tid / M, j = tid % M;
+  const bool act = i < vHi;
+  double a = lo, c = hi;
+  {
+    int l = 0, h = kTsThreads;   // first point with more than i eigenvalues below it
+    while (l < h) {
+      const int m = (l + h) >> 1;
+      if (cA[m] > i) h = m; else l = m + 1;
+    }
+    if (l > 0) a = lo + w * l;
+    if (l < kTsThreads) c = lo + w * (l + 1);
+  }
+  const double f = 1.0 / (M + 1);
+  const unsigned group = (M == 32 ? 0xffffffffu : ((1u << M) - 1u)) << ((tid & 31) / M * M);
+  bool done = !act;
+  for (int it = 0; it < 64; ++it) {
+    done = done || c - a <= fmax(2.0 * eps * fmax(fabs(a), fabs(c)), eps * tnorm);
+    if (!__any_sync(0xffffffffu, !done)) break;
+    const double x = a + (c - a) * (f * (j + 1));
+    const bool above = done ? false : ts_count(de, n, x) > i;
+    const unsigned bal = __ballot_sync(0xffffffffu, above) & group;
+    if (!done) {
+      const int first = bal ? __ffs(bal) - 1 - (tid & 31) / M * M : M;   // first point above eigenvalue i
+      const double an = first > 0 ? a + (c - a) * (f * first) : a;
+      const double cn = first < M ? a + (c - a) * (f * (first + 1)) : c;
+      done = !(an > a || cn < c);
+      a = an;
+      c = cn;
+    }
+  }
+  if (act && j == 0) lam[i] = 0.5 * (a + c) / scale;
+}
+
+// 1 / x to a rounding or two by Newton's iteration from the hardware estimate; x is a
+// normal number within 2^+-600 here
+__device__ __forceinline__ double ts_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  y = fma(y, fma(-x, y, 1.0), y);
+  return y;
+}
+
+// Eigenvectors of the eigenvalues range[2b] .. range[2b+1]-1 of matrix b (trimmed to
+// [vecLo, vecHi] by value), by the twisted factorisation of T - lambda I at the index of
+// the smallest |gamma|. CTA (c, r): 64 eigenvectors, lanes of the first half of the CTA
+// factorise from the top (quotients L_k = e_k / D+_k), of the second from the bottom
+// (U_k = e_k / D-_{k+1}). krange receives the trimmed range (krange may not alias range).
+// work: 2 Nmax^2 doubles per matrix, rows of eigenvalue index so that lanes are coalesced.
+// Z: row-major Z[k Nmax + i], columns outside the range are not written.
+// Dynamic shared memory: Nmax double2.
+template <typename R>
+__global__ void __launch_bounds__(kTsThreads)
+tridiag_vectors_kernel(const double* __restrict__ dIn, const double* __restrict__ eIn, const int* __restrict__ nred,
+                       int Nmax, const double* __restrict__ lamIn, double vecLo, double vecHi,
+                       const int* __restrict__ range, int* __restrict__ krange, R* __restrict__ Z,
+                       double* __restrict__ work, const int* __restrict__ order) {
+  const int b = order ? order[blockIdx.y] : blockIdx.y;
+  const int n = nred[b];
+  if (n <= 0) return;
+  extern __shared__ __align__(16) double2 ts_smem[];
+  double2* de = ts_smem;   // (d_k, e_k), scaled
+  __shared__ double red[32], sBest[kTsThreads], sNrm[kTsThreads];
+  __shared__ int sArg[kTsThreads], sK[2];
+  const int tid = threadIdx.x;
+  const double* lam = lamIn + (long long)b * Nmax;
+  if (tid == 0) {
+    int a = range[2 * b], c = range[2 * b + 1];
+    while (a < c && lam[a] < vecLo) ++a;
+    while (c > a && lam[c - 1] > vecHi) --c;
+    sK[0] = a;
+    sK[1] = c;
+    if (blockIdx.x == 0) {
+      krange[2 * b] = a;
+      krange[2 * b + 1] = c;
+    }
+  }
+  __syncthreads();
+  constexpr int VPC = kTsThreads / 2;
+  const int kHi = sK[1];
+  if (sK[0] + (int)blockIdx.x * VPC >= kHi) return;
+  double lo, hi, tnorm, scale;
+  ts_load(dIn + (long long)b * Nmax, eIn + (long long)b * Nmax, n, de, red, lo, hi, tnorm, scale);
+  for (int k = tid; k < n; k += kTsThreads) de[k].y = k < n - 1 ? eIn[(long long)b * Nmax + k] * scale : 0.0;
+  __syncthreads();
+  const int v = tid % VPC, role = tid / VPC;
+  const int iv = sK[0] + blockIdx.x * VPC + v;
+  const bool act = iv < kHi;
+  const int i = act ? iv : kHi - 1;   // idle lanes repeat the last column without storing
+  const double l = lam[i] * scale;
+  double* Lp = work + (long long)b * 2 * Nmax * Nmax + i;
+  double* Um = Lp + (long long)Nmax * Nmax;
+  {
+    // role 0: k = 0 .. n-2 from the top; role 1: k = n-2 .. 0 from the bottom
+    double p0 = 1.0, p1 = (role ? de[n - 1].x : de[0].x) - l;
+    double* out = role ? Um + (long long)max(n - 2, 0) * Nmax : Lp;
+    const long long step = role ? -(long long)Nmax : Nmax;
+    auto one = [&](int t) {
+      const int k = role ? n - 2 - t : t;
+      const double ek = de[k].y, dn = de[role ? k : k + 1].x;
+      p1 = ts_nonzero(p1, p0);
+      if (act) *out = ek * p0 * ts_rcp(p1);
+      out += step;
+      const double p2 = fma(dn - l, p1, -(ek * ek) * p0);
+      p0 = p1;
+      p1 = p2;
+    };
+    int t = 0;
+    for (; t + 4 <= n - 1; t += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) one(t + u);
+      p1 = ts_nonzero(p1, p0);
+      ts_rescale(p0, p1);
+    }
+    for (; t < n - 1; ++t) one(t);
+  }
+  __syncthreads();
+  // twist index: smallest |gamma_k|, gamma_k = (d_k - l) - L_{k-1} e_{k-1} - U_k e_k; ties
+  // go to the larger k
+  {
+    const int kb = role ? n / 2 : 0, ke = role ? n : n / 2;
+    double best = 1e300;
+    int arg = kb;
+#pragma unroll 4
+    for (int k = kb; k < ke; ++k) {
+      const double lm = k > 0 ? Lp[(long long)(k - 1) * Nmax] * de[k - 1].y : 0.0;
+      const double um = k < n - 1 ? Um[(long long)k * Nmax] * de[k].y : 0.0;
+      const double g = fabs((de[k].x - l) - lm - um);
+      if (g <= best) {
+        best = g;
+        arg = k;
+      }
+    }
+    sBest[tid] = best;
+    sArg[tid] = arg;
+  }
+  __syncthreads();
+  int r = sArg[v];
+  if (n > 1 && sBest[VPC + v] <= sBest[v]) r = sArg[VPC + v];
+  if (n == 1) r = 0;
+  // z_r = 1; z_k = -L_k z_{k+1} upwards (role 0), z_{k+1} = -U_k z_k downwards (role 1); the
+  // values overwrite L and U, 8 quotients loaded ahead of the chain
+  {
+    double z1 = 1.0, z2 = 0.0, nrm = role ? 1.0 : 0.0;
+    double* q = role ? Um : Lp;
+    for (int t0 = 0; t0 < n - 1; t0 += 8) {
+      double c[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int t = t0 + u, k = role ? t : n - 2 - t;
+        c[u] = t < n - 1 ? q[(long long)k * Nmax] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int t = t0 + u, k = role ? t : n - 2 - t;
+        if (t < n - 1 && (role ? k >= r : k < r)) {
+          double z;
+          if (z1 != 0.0) z = -c[u] * z1;
+          else if (de[k].y == 0.0) z = 0.0;
+          else z = role ? -((k > 0 ? de[k - 1].y : 0.0) / de[k].y) * z2 : -(de[k + 1].y / de[k].y) * z2;
+          nrm = fma(z, z, nrm);
+          if (act) q[(long long)k * Nmax] = z;
+          z2 = z1;
+          z1 = z;
+        }
+      }
+    }
+    sNrm[tid] = nrm;
+  }
+  __syncthreads();
+  if (!act) return;
+  const double inv = 1.0 / sqrt(sNrm[v] + sNrm[VPC + v]);
+  R* Zb = Z + (long long)b * Nmax * Nmax + i;
+  const int kb = role ? n / 2 : 0, ke = role ? n : n / 2;
+#pragma unroll 8
+  for (int k = kb; k < ke; ++k) {
+    double z = 1.0;
+    if (k < r) z = Lp[(long long)k * Nmax];
+    else if (k > r) z = Um[(long long)(k - 1) * Nmax];
+    Zb[(long long)k * Nmax] = (R)(z * inv);
+  }
+}
+
+// Clusters (neighbours closer than 1e-10 of the norm): modified Gram-Schmidt inside each,
+// in eigenvalue order. One CTA per matrix, which returns at once when there is none.
+template <typename R>
+__global__ void __launch_bounds__(256)
+tridiag_clusters_kernel(const double* __restrict__ dIn, const double* __restrict__ eIn, const int* __restrict__ nred,
+                        int Nmax, const double* __restrict__ lamIn, const int* __restrict__ krange, R* __restrict__ Z,
+                        int* __restrict__ status) {
+  const int b = blockIdx.x;
+  const int n = nred[b];
+  if (n <= 0) return;
+  __shared__ double red[32];
+  const double* d = dIn + (long long)b * Nmax;
+  const double* e = eIn + (long long)b * Nmax;
+  const double* lam = lamIn + (long long)b * Nmax;
+  R* Zb = Z + (long long)b * Nmax * Nmax;
+  const int kLo = krange[2 * b], kHi = krange[2 * b + 1];
+  double t = 0.0;
+  for (int k = threadIdx.x; k < n; k += blockDim.x)
+    t = fmax(t, fabs(d[k]) + (k < n - 1 ? fabs(e[k]) : 0.0) + (k > 0 ? fabs(e[k - 1]) : 0.0));
+  const double ctol = 1e-10 * fmax(block_max(t, red, 0.0), 1e-300);
+  bool close = false;
+  for (int i = kLo + 1 + threadIdx.x; i < kHi; i += blockDim.x) close = close || lam[i] - lam[i - 1] < ctol;
+  if (!__syncthreads_or(close)) return;
+  if (threadIdx.x == 0) atomicOr(status + b, (int)kStatusClusterFix);
+  for (int i = kLo + 1; i < kHi; ++i) {
+    if (!(lam[i] - lam[i - 1] < ctol)) continue;
+    int j0 = i - 1;
+    while (j0 > kLo && lam[j0] - lam[j0 - 1] < ctol) --j0;
+    for (int j = j0; j < i; ++j) {
+      double part = 0.0;
+      for (int k = threadIdx.x; k < n; k += blockDim.x)
+        part += (double)Zb[(long long)k * Nmax + i] * (double)Zb[(long long)k * Nmax + j];
+      const double dot = block_sum(part, red);
+      for (int k = threadIdx.x; k < n; k += blockDim.x)
+        Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] - dot * (double)Zb[(long long)k * Nmax + j]);
+      __syncthreads();
+    }
+    double part = 0.0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+      const double zv = (double)Zb[(long long)k * Nmax + i];
+      part += zv * zv;
+    }
+    const double nr = sqrt(block_sum(part, red));
+    const double inv = nr > 0 ? 1.0 / nr : 0.0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x)
+      Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] * inv);
+    __syncthreads();
+  }
+}
+
+}  // namespace bippb200
