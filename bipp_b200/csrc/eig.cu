@@ -154,7 +154,9 @@ void EigWork<T>::reserve(bipp_ctx_s* ctx, int nBatch, int nmax) {
   capBatch = nBatch;
   Nmax = nmax;
   A.alloc(ctx, n2 * sizeof(C) * nBatch);
-  G.alloc(ctx, n2 * sizeof(double2) * nBatch);
+  // G's storage also holds the back-transform's T blocks, which need more than a matrix of a
+  // few rows
+  G.alloc(ctx, std::max(n2 * sizeof(double2), bt_t_elems(nmax) * sizeof(C)) * nBatch);
   W64.alloc(ctx, n2 * sizeof(double2) * nBatch);
   Linv.alloc(ctx, n2 * sizeof(C) * nBatch);
   T1.alloc(ctx, n2 * sizeof(C) * nBatch);
@@ -384,7 +386,7 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
     // blocked: T of each 16-reflector block into G's storage (free between the triangular
     // inverse and the final GEMM), then one pass over Y per 16-column slice
     C* Tblk = reinterpret_cast<C*>(G);
-    const long long tStride = n2 * (long long)(sizeof(double2) / sizeof(C));
+    const long long tStride = (long long)bt_t_elems(Nmax);
     const int nblk = (Nmax - 1 + kBtNB - 1) / kBtNB;
     count_launch();
     bt_larft_kernel<C, R><<<dim3(std::max(1, nblk), nb), 256, 0, st>>>(A, w.tau.template get<C>(), nred, Nmax, Tblk,

@@ -1601,6 +1601,8 @@ backtransform_kernel(const C* __restrict__ A, const C* __restrict__ taus, const 
 constexpr int kBtNB = 16;             // reflectors per block
 constexpr int kBtCB = 16;             // columns of Y per CTA
 constexpr int kBtMaxRows = 1024;      // Nmax limit of the register-resident kernel
+// elements of one matrix's T blocks
+constexpr size_t bt_t_elems(int nmax) { return (size_t)(nmax < 2 ? 1 : (nmax - 1 + kBtNB - 1) / kBtNB) * kBtNB * kBtNB; }
 
 // element r of reflector i (v(i+1) = 1, stored below the subdiagonal of column i)
 template <typename C, typename R>
