@@ -13,6 +13,7 @@
 #include "eig_kernels.cuh"
 #include "chol_kernels.cuh"
 #include "gemm_tc.cuh"
+#include "hetrd.hpp"
 #include "tridiag_kernels.cuh"
 
 namespace bippb200 {
@@ -316,8 +317,13 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
   }
   // 3. tridiagonalisation
   mark(4);
-  {
-    // single precision: blocked panels while the V/W panel fits in shared memory
+  const int trdThreads = tuned("hetrd.threads"), trdPct = tuned("hetrd.ctas_pct");
+  const int grid1 = trdPct > 0 ? std::max(1, std::min(nb, trdPct * ctx->smCount / 100)) : 0;
+  if (!hetrd_cluster<C, R>(st, ctx->smCount, (size_t)ctx->prop.l2CacheSize, ctx->maxSmemOptin, A, nred, Nmax, w.d.template get<double>(),
+                           w.e.template get<double>(), w.tau.template get<C>(), sizeOrder, nb, Nmax,
+                           trdThreads > 0 ? trdThreads / 256 : 8, grid1)) {
+    // larger matrices: one CTA each; in single precision blocked panels while the V/W panel
+    // fits in shared memory
     bool blocked = false;
     if constexpr (sizeof(C) == 8) blocked = hetrd_blk_smem_bytes(Nmax) <= ctx->maxSmemOptin;
     const size_t smem = blocked ? hetrd_blk_smem_bytes(Nmax) : hetrd_smem_bytes(Nmax, sizeof(C));
@@ -327,14 +333,8 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
     }
     smem_optin(k, smem);
     count_launch();
-    // threads per matrix: by size, unless the tuning table fixes them; the blocked kernel
-    // may run as fewer persistent CTAs (a percentage of the SM count)
-    const int tt = tuned("hetrd.threads");
-    const int pct = blocked ? tuned("hetrd.ctas_pct") : 0;
-    const int grid = pct > 0 ? std::max(1, std::min(nb, pct * ctx->smCount / 100)) : nb;
-    k<<<grid, tt > 0 ? tt : trd_threads(Nmax), smem, st>>>(A, nred, Nmax, w.d.template get<double>(),
-                                                          w.e.template get<double>(), w.tau.template get<C>(),
-                                                          sizeOrder, nb);
+    k<<<blocked && grid1 ? grid1 : nb, trdThreads > 0 ? trdThreads : trd_threads(Nmax), smem, st>>>(
+        A, nred, Nmax, w.d.template get<double>(), w.e.template get<double>(), w.tau.template get<C>(), sizeOrder, nb);
     B2_CHECK_LAUNCH();
   }
   // 4. tridiagonal eigenpairs (FP64); workspace aliases W64 (free after trinv)

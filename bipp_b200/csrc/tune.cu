@@ -52,7 +52,10 @@ std::vector<Param>& table() {
        0},
       {"spread.schedule", 1, {0, 1},
        "spreading work items: 0 round-robin over the persistent CTAs, 1 heaviest first from a work counter", 0},
-      {"hetrd.threads", 0, {0, 256, 512, 1024}, "threads per matrix in the tridiagonalisation (0: by matrix size)", 0},
+      {"hetrd.threads", 0, {0, 256, 512, 1024},
+       "largest share of the GPU for one matrix's tridiagonalisation, in units of 256: 256 one CTA, 512 a cluster of 2, "
+       "1024 of 4; above 1024 rows the threads of its CTA (0: by matrix size and batch)",
+       0},
       {"hetrd.ctas_pct", 0, {0, 50, 75, 100, 150},
        "persistent tridiagonalisation CTAs in percent of the SM count (0: one CTA per matrix)", 0},
       {"tridiag.threads", 0, {0, 128, 256},
