@@ -53,7 +53,27 @@ struct FftLines {
   long long planeStride;         // cells per plane
   long long lineStep;            // offset between consecutive lines (rows: nx; columns: 1)
   long long elemStep;            // offset between the values of a line (rows: 1; columns: nx)
+  // Which values of a line hold data; the others are zero and are not read, nor need to have
+  // been written. xBits[layer][tile row][xWords]: one bit per 16 cells of a row (its tiles that
+  // points reach); yBits[layer][yWords]: one bit per 8 rows (tile rows with such a tile).
+  const unsigned *xBits, *yBits;
+  int xWords, yWords, tileRows, firstLayer;
 };
+
+// Bit of value b + j Nr of a line (2^SHIFT values per bit, b < Nr): the words are loaded at
+// offsets known at compile time wherever a stage's stride is a whole number of bits
+template <int SHIFT, int Nr>
+__device__ __forceinline__ bool fft_bit(const unsigned* __restrict__ bits, int b, int j) {
+  constexpr int step = Nr >> SHIFT;
+  if constexpr (Nr % (1 << SHIFT) == 0 && step <= 32 && 32 % (step ? step : 1) == 0) {
+    return ((__ldg(bits + ((j * step) >> 5)) >> (b >> SHIFT)) >> ((j * step) & 31)) & 1u;
+  } else if constexpr (Nr % (1 << SHIFT) == 0 && step % 32 == 0) {
+    return (__ldg(bits + (b >> (SHIFT + 5)) + j * (step / 32)) >> ((b >> SHIFT) & 31)) & 1u;
+  } else {
+    const int t = (b + j * Nr) >> SHIFT;
+    return (__ldg(bits + (t >> 5)) >> (t & 31)) & 1u;
+  }
+}
 
 __host__ __device__ __forceinline__ int fft_pad(int i) { return i + (i >> 4); }
 
@@ -234,7 +254,9 @@ template <int N, int... Rs> struct FftBlockPad {
 // layout (FftBlockPad) when on, with its c.
 template <int R, int MODE, int N, int P, int ES, bool BP, int BPC>
 __device__ __forceinline__ void fft_stage(const FftLinePlan& pl, int t, bool active, float2* __restrict__ lp, int es,
-                                          float2* __restrict__ sl, const float2* __restrict__ tw) {
+                                          float2* __restrict__ sl, const float2* __restrict__ tw,
+                                          const unsigned* __restrict__ bits) {
+  constexpr int SHIFT = ES > 0 ? 4 : 3;   // cells per bit of a row, of a column
   constexpr bool first = MODE == 0, last = MODE == 2;
   constexpr int MB = kFftMaxValues / R;   // butterflies per thread (the plan's thread count ensures enough)
   constexpr int Nr = N / R, twStep = N / (P * R);
@@ -249,7 +271,10 @@ __device__ __forceinline__ void fft_stage(const FftLinePlan& pl, int t, bool act
 #pragma unroll
       for (int j = 0; j < R; ++j) {
         const int i = b + j * Nr;
-        if constexpr (first) v[q][j] = active ? lp[i * st] : mk(0.f, 0.f);
+        if constexpr (first) {
+          v[q][j] = mk(0.f, 0.f);
+          if (active && fft_bit<SHIFT, Nr>(bits, b, j)) v[q][j] = lp[i * st];
+        }
         else if constexpr (BP) v[q][j] = sl[b + j * (BPB + BPC)];   // Nr == B in stages 2 and 3
         else v[q][j] = sl[fft_pad(i)];
       }
@@ -297,10 +322,11 @@ __device__ __forceinline__ void fft_stage(const FftLinePlan& pl, int t, bool act
 
 template <int S, int N, int P, int ES, bool BP, int BPC, int R, int... Rest>
 __device__ __forceinline__ void fft_stages(const FftLinePlan& pl, int t, bool active, float2* __restrict__ lp, int es,
-                                           float2* __restrict__ sl, const float2* __restrict__ tw) {
-  fft_stage<R, S == 0 ? 0 : (sizeof...(Rest) == 0 ? 2 : 1), N, P, ES, BP, BPC>(pl, t, active, lp, es, sl, tw);
+                                           float2* __restrict__ sl, const float2* __restrict__ tw,
+                                           const unsigned* __restrict__ bits) {
+  fft_stage<R, S == 0 ? 0 : (sizeof...(Rest) == 0 ? 2 : 1), N, P, ES, BP, BPC>(pl, t, active, lp, es, sl, tw, bits);
   if constexpr (sizeof...(Rest) > 0)
-    fft_stages<S + 1, N, P * R, ES, BP, BPC, Rest...>(pl, t, active, lp, es, sl, tw);
+    fft_stages<S + 1, N, P * R, ES, BP, BPC, Rest...>(pl, t, active, lp, es, sl, tw, bits);
 }
 
 // The pass over lines of N = the product of the radices Rs (at least two stages).
@@ -310,7 +336,8 @@ __device__ __forceinline__ void fft_stages(const FftLinePlan& pl, int t, bool ac
 // tw[m] = exp(2 pi i m / N), m < N. Launch: lines x threads threads, lines x lineStride
 // float2 of dynamic shared memory, ceil(nLines / lines) CTAs.
 template <bool LINE_FAST, int... Rs>
-__global__ void __launch_bounds__(512, 2) fft_lines_kernel(FftLinePlan pl, FftLines L, const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(LINE_FAST ? 1024 : 512, LINE_FAST ? 1 : 2)
+fft_lines_kernel(FftLinePlan pl, FftLines L, const float2* __restrict__ tw) {
   static_assert(sizeof...(Rs) >= 2, "two stages at least");
   constexpr int N = (Rs * ...);
   extern __shared__ float2 fft_smem[];
@@ -319,18 +346,30 @@ __global__ void __launch_bounds__(512, 2) fft_lines_kernel(FftLinePlan pl, FftLi
   const int g = LINE_FAST ? tid % G : tid / T;
   const int t = LINE_FAST ? tid / G : tid % T;
   const long long line = (long long)blockIdx.x * G + g;
-  const bool active = line < L.nLines;
+  bool active = line < L.nLines;
   long long base = 0;
+  const unsigned* bits = L.xBits;
   if (active) {
     const long long o = line / L.linesPerPlane;
     const int li = (int)(line - o * L.linesPerPlane);
     const int c = (int)(o / L.planesUsed), pj = (int)(o - (long long)c * L.planesUsed);
     base = ((long long)c * L.slabPlanes + pj) * L.planeStride + (long long)li * L.lineStep;
+    const int layer = L.firstLayer + (pj >> 3);
+    bits = L.yBits + layer * L.yWords;
+    if constexpr (!LINE_FAST) {
+      // a row without any data is not transformed: the column pass knows it as zero
+      const int ty = li >> 3;
+      active = (__ldg(bits + (ty >> 5)) >> (ty & 31)) & 1u;
+      bits = L.xBits + ((long long)layer * L.tileRows + ty) * L.xWords;
+    }
+  }
+  if constexpr (!LINE_FAST) {
+    if (!__syncthreads_or(active)) return;
   }
   // rows: unit stride (compile time); columns: the row length
   using BPad = FftBlockPad<N, Rs...>;
   fft_stages<0, N, 1, LINE_FAST ? 0 : 1, BPad::on, BPad::c, Rs...>(pl, t, active, L.data + base, (int)L.elemStep,
-                                                                   fft_smem + (size_t)g * pl.lineStride, tw);
+                                                                   fft_smem + (size_t)g * pl.lineStride, tw, bits);
 }
 
 using FftLinesKernel = void (*)(FftLinePlan, FftLines, const float2*);

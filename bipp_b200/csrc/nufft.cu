@@ -144,7 +144,8 @@ NufftCore::~NufftCore() {
 // so the first stage's reads precede a barrier that the last stage's in-place writes
 // follow. Threads per line: the fewest warps with which no thread holds more than
 // kFftMaxValues values in any stage. Lines per CTA: 256 threads for the row pass; 4 lines
-// for the column pass (a warp reads 32-byte row segments).
+// for the column pass (a warp reads 32-byte row segments) while they fit 1024 threads and
+// shared memory.
 static bool make_fft_plan(int n, int nout, bool columnPass, FftLinePlan& pl, FftLinesKernel& kernel) {
   kernel = nullptr;
   pl = FftLinePlan{};
@@ -190,7 +191,7 @@ static bool make_fft_plan(int n, int nout, bool columnPass, FftLinePlan& pl, Fft
   for (int s = 0; s < pl.ns; ++s) pl.radix[s] = r[s];
   pl.threads = T;
   pl.lineStride = (fft_pad(n - 1) + 1 + 15) / 16 * 16 + 4;
-  int G = columnPass ? std::min(4, 512 / T) : std::max(1, 256 / T);
+  int G = columnPass ? std::min(4, 1024 / T) : std::max(1, 256 / T);
   while (G > 1 && (size_t)G * pl.lineStride * sizeof(float2) > (size_t)227 * 1024) --G;
   if ((size_t)G * pl.lineStride * sizeof(float2) > (size_t)227 * 1024) return false;
   pl.lines = G;
@@ -199,10 +200,16 @@ static bool make_fft_plan(int n, int nout, bool columnPass, FftLinePlan& pl, Fft
 }
 
 // batched inverse 2-D FFT of the (channel, plane) arrays of the slab
-void NufftCore::inverse_fft(int slabPlanes, int planesUsed, float2* slab, bool pruned) {
+void NufftCore::inverse_fft(int slabPlanes, int planesUsed, int firstLayer, float2* slab, bool pruned) {
   if (pruned) {
     FftLines L{};
     L.data = slab;
+    L.firstLayer = firstLayer;
+    L.tileRows = g_.nty;
+    L.xWords = (g_.ntx + 31) / 32;
+    L.yWords = (g_.nty + 31) / 32;
+    L.xBits = tileBits_.get<unsigned>();
+    L.yBits = L.xBits + (long long)g_.ntw * g_.nty * L.xWords;
     L.planesUsed = planesUsed;
     L.slabPlanes = slabPlanes;
     L.planeStride = (long long)g_.nx * g_.ny;
@@ -428,7 +435,7 @@ static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, co
 static bool use_tensor_core_spread(int nch, double eps) {
   const char* e = std::getenv("BIPP_B200_SPREAD");
   if (e && std::string(e) == "warp") return false;
-  return nch <= kTcMaxChan || eps >= 1e-5;
+  return nch <= kTcMaxChan || eps > 0.99e-5;   // 1e-5 given in single precision is a little less
 }
 
 
@@ -463,7 +470,6 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
   slabTiles_ = slabTiles;
   const int slabPlanes = slabTiles * kTW;
   grid_.ensure(ctx_, (size_t)nch_ * slabPlanes * planeBytes);
-  B2_CUDA(cudaMemsetAsync(acc_.get(), 0, (size_t)nch_ * P * sizeof(float2), ctx_->stream));
   // per-tile loads -> work items (non-empty tiles, heavy tiles split in parts), built on
   // the device: parts per tile, exclusive scan -> item offsets, fill; tiles are numbered
   // slab by slab, so a slab's items are one contiguous range
@@ -471,9 +477,10 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
   load_.ensure(ctx_, (size_t)ntiles * sizeof(int));
   parts_.ensure(ctx_, (size_t)ntiles * sizeof(int));
   itemOff_.ensure(ctx_, (size_t)(ntiles + 1) * sizeof(int));
-  // the tensor-core spreader writes every tile it spreads in one part; the other tiles of a
-  // slab (empty, or split into parts that accumulate with atomics) are cleared first from
-  // a compact list; the warp spreader works on a cleared slab
+  // the tensor-core spreader writes every tile it spreads in one part; tiles split into parts
+  // that accumulate with atomics are cleared first from a compact list, and so are the empty
+  // ones unless the pruned FFT, which reads by the tiles' bits, leaves them out; the warp
+  // spreader works on a cleared slab
   const bool tc = use_tensor_core_spread(nch_, eps_);
   const bool prunedFft = fftPlansOk_ && tuned("nufft.fft") == 1;
   const int tb = std::min(8192, (ntiles + 255) / 256);
@@ -488,9 +495,20 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
   // points per spreading work item (tunable): heavier tiles are split so that no CTA
   // serialises the dense core of the uv plane (short baselines)
   const int spreadCap = tuned("spread.items_cap");
-  tile_parts_kernel<<<tb, 256, 0, ctx_->stream>>>(ntiles, load_.get<int>(), spreadCap, parts_.get<int>(),
-                                                  clearFlag_.get<int>(), splitCount_.get<int>());
+  tile_parts_kernel<<<tb, 256, 0, ctx_->stream>>>(ntiles, load_.get<int>(), spreadCap, prunedFft ? 0 : 1,
+                                                  parts_.get<int>(), clearFlag_.get<int>(), splitCount_.get<int>());
   B2_CHECK_LAUNCH();
+  if (prunedFft) {
+    const int xWords = (g_.ntx + 31) / 32, yWords = (g_.nty + 31) / 32;
+    const long long xAll = (long long)g_.ntw * g_.nty * xWords, yAll = (long long)g_.ntw * yWords;
+    tileBits_.ensure(ctx_, (size_t)(xAll + yAll) * sizeof(unsigned));
+    unsigned* xBits = tileBits_.get<unsigned>();
+    B2_CUDA(cudaMemsetAsync(xBits + xAll, 0, (size_t)yAll * sizeof(unsigned), ctx_->stream));
+    count_launch();
+    tile_bits_kernel<<<std::min(4096, (g_.ntw * g_.nty + 7) / 8), 256, 0, ctx_->stream>>>(g_, load_.get<int>(), xWords,
+                                                                                        yWords, xBits, xBits + xAll);
+    B2_CHECK_LAUNCH();
+  }
   exclusive_scan(parts_.get<int>(), itemOff_.get<int>(), ntiles);
   if (tc) {
     exclusive_scan(clearFlag_.get<int>(), clearOff_.get<int>(), ntiles);
@@ -619,13 +637,13 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
     }
     if (stageMs) B2_CUDA(cudaEventRecord(ev[1], ctx_->stream));
     const int planesUsed = std::min(tiles * kTW, planes_ - tw0 * kTW);
-    inverse_fft(slabPlanes, planesUsed, grid_.get<float2>(), prunedFft);
+    inverse_fft(slabPlanes, planesUsed, tw0, grid_.get<float2>(), prunedFft);
     if (stageMs) B2_CUDA(cudaEventRecord(ev[2], ctx_->stream));
     const int blocks = (int)std::min<long long>((P + 255) / 256, 65535);
     count_launch();
-    auto wk = nch_ <= 4 ? wsum_kernel<4> : wsum_kernel<kMaxChan>;
+    auto wk = nch_ <= 4 ? wsum_kernel<4> : nch_ <= 8 ? wsum_kernel<8> : wsum_kernel<kMaxChan>;
     wk<<<blocks, 256, 0, ctx_->stream>>>(g_, grid_.get<float2>(), nch_, slabPlanes, tw0 * kTW, planesUsed,
-                                         nTilde_.get<double>(), acc_.get<float2>(), P, prunedFft ? 1 : 0);
+                                         nTilde_.get<double>(), acc_.get<float2>(), P, prunedFft ? 1 : 0, sl == 0 ? 1 : 0);
     B2_CHECK_LAUNCH();
     if (stageMs) {
       B2_CUDA(cudaEventRecord(ev[3], ctx_->stream));

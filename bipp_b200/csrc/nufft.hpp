@@ -92,9 +92,11 @@ private:
   DevBuf fftTw_;
   int slabTiles_ = 1;
   int planes_ = 0;    // w-planes that supports of the current transform reach
-  // inverse 2-D FFT of the first planesUsed planes of every channel of the slab: pruned
-  // (cell (a, b) of a plane then holds pixel (a, b)'s output) or in full by cuFFT
-  void inverse_fft(int slabPlanes, int planesUsed, float2* slab, bool pruned);
+  DevBuf tileBits_;   // tiles that points reach, then tile rows with any (tile_bits_kernel)
+  // inverse 2-D FFT of the first planesUsed planes of every channel of the slab, whose first
+  // tile layer is firstLayer: pruned (by the tiles' bits; cell (a, b) of a plane then holds
+  // pixel (a, b)'s output) or in full by cuFFT
+  void inverse_fft(int slabPlanes, int planesUsed, int firstLayer, float2* slab, bool pruned);
   void exclusive_scan(const int* in, int* out, long long n);
 
 public:

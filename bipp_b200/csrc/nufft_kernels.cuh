@@ -465,14 +465,36 @@ static __global__ void tile_load_kernel(NufftGeom g, const int* __restrict__ off
 }
 
 // spreading parts of each tile (ceil(load / cap), 0 when empty) and whether the tile has
-// to be cleared before spreading (empty, or spread in several parts that accumulate)
-static __global__ void tile_parts_kernel(int ntiles, const int* __restrict__ load, int cap, int* __restrict__ parts,
-                                         int* __restrict__ clearFlag, int* __restrict__ splitTiles) {
+// to be cleared before spreading: spread in several parts that accumulate, or empty and read
+// all the same (clearEmpty)
+static __global__ void tile_parts_kernel(int ntiles, const int* __restrict__ load, int cap, int clearEmpty,
+                                         int* __restrict__ parts, int* __restrict__ clearFlag,
+                                         int* __restrict__ splitTiles) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
     const int np = (load[t] + cap - 1) / cap;
     parts[t] = np;
-    clearFlag[t] = (np != 1) ? 1 : 0;
+    clearFlag[t] = (np > 1 || (np == 0 && clearEmpty)) ? 1 : 0;
     if (np > 1) atomicAdd(splitTiles, 1);
+  }
+}
+
+// Bits of the tiles that points reach, for the pruned FFT: xBits[tile row (tw, ty)][word of 32
+// tx], one warp per tile row, and yBits[tw][word of 32 ty] of the tile rows that have any
+// (zeroed before)
+static __global__ void tile_bits_kernel(NufftGeom g, const int* __restrict__ load, int xWords, int yWords,
+                                        unsigned* __restrict__ xBits, unsigned* __restrict__ yBits) {
+  const int lane = threadIdx.x & 31;
+  const int rows = g.nty * g.ntw;
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += (gridDim.x * blockDim.x) >> 5) {
+    unsigned any = 0;
+    for (int w = 0; w < xWords; ++w) {
+      const int tx = 32 * w + lane;
+      const unsigned m = __ballot_sync(0xffffffffu, tx < g.ntx && load[(long long)row * g.ntx + tx] > 0);
+      if (lane == 0) xBits[(long long)row * xWords + w] = m;
+      any |= m;
+    }
+    const int ty = row % g.nty, tw = row / g.nty;
+    if (lane == 0 && any) atomicOr(yBits + tw * yWords + (ty >> 5), 1u << (ty & 31));
   }
 }
 
@@ -614,15 +636,15 @@ spread_warp_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __
 // ---------------------------------------------------------------------------------------
 // w-sum: acc[ch][p] += sum_{planes j of slab} F[ch][j][a'][b'] exp(i n~_p t_j)
 // ---------------------------------------------------------------------------------------
-// CH: channels held in registers (4, or kMaxChan for more); with 4 channels the planes are
-// read 4 at a time (their 16 loads issued together), with more one at a time (registers),
-// while the FP64 phase recurrence runs in order
-template <int CH, int kWsumUnroll = (CH <= 4 ? 4 : 1)>
+// CH: channels held in registers (4, 8 or kMaxChan); with 4 channels the planes are read 4 at a
+// time, with 8 two at a time (16 loads issued together), with more one at a time (registers),
+// while the FP64 phase recurrence runs in order. The first slab starts the sums (`start`).
+template <int CH, int kWsumUnroll = (CH <= 4 ? 4 : CH <= 8 ? 2 : 1)>
 static __global__ void __launch_bounds__(256) wsum_kernel(NufftGeom g, const float2* __restrict__ F, int nch,
                                                            int slabPlanes, int jFirst, int planesUsed,
                                                            const double* __restrict__ nTilde /*[P]*/,
                                                            float2* __restrict__ acc, long long accStride,
-                                                           int pruned) {
+                                                           int pruned, int start) {
   const long long P = (long long)g.Na * g.Nb;
   const long long planeStride = (long long)g.ny * g.nx;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
@@ -669,7 +691,7 @@ static __global__ void __launch_bounds__(256) wsum_kernel(NufftGeom g, const flo
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if (c < nch) {
-        float2 o = acc[(long long)c * accStride + p];
+        float2 o = start ? make_float2(0.f, 0.f) : acc[(long long)c * accStride + p];
         o.x += sum[c].x;
         o.y += sum[c].y;
         acc[(long long)c * accStride + p] = o;
