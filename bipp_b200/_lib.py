@@ -64,6 +64,8 @@ SIGNATURES = {
     "bipp_eigh_d": [_p, _d, _sz, _sz, _p, _sz, _p, _sz, _p, _p, _sz, _psz, _pd],
     "bipp_eigh_gram_batched_s": [_p, _sz, _sz, _p, _p, _p, _p, _p, _p, _p],
     "bipp_eigh_gram_batched_d": [_p, _sz, _sz, _p, _p, _p, _p, _p, _p, _p],
+    "bipp_eigh_gram_batched_rows_s": [_p, _sz, _sz, _p, _p, _p, _p, _p, _p, _p],
+    "bipp_eigh_gram_batched_rows_d": [_p, _sz, _sz, _p, _p, _p, _p, _p, _p, _p],
     "bipp_eigh_gram_batched_ranked_s": [_p, _sz, _sz, _p, _p, _p, _d, _i, _p, _i, _d, _p, _p, _p, _p, _p, _p, _p],
     "bipp_rank_features_s": [_p, _sz, _sz, _p, _p, _p, _d, _p, _p],
     "bipp_rank_mlp_num_params": [],

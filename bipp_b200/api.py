@@ -206,24 +206,22 @@ def eigh(wl, s, w, ctx: Optional[Context] = None, precision: Optional[str] = Non
 def eigh_gram_batched(wl, s, xyz, ctx: Optional[Context] = None, precision: str = "single"):
     """Batched eigh_gram with W = I over steps: wl [B], s [B, N, N] (s[b] is the step's
     matrix; its lower triangle in column-major order is used), xyz [B, N, 3]. Single
-    precision (complex64, bipp_eigh_gram_batched_s) or "double" (complex128,
-    bipp_eigh_gram_batched_d). Returns (v [B, N, N] (v[b][:, c] eigenvector c), d [B, N],
+    precision (complex64, bipp_eigh_gram_batched_rows_s) or "double" (complex128,
+    bipp_eigh_gram_batched_rows_d). Returns (v [B, N, N] (v[b][:, c] eigenvector c), d [B, N],
     nReduced [B], scale [B])."""
     ctx = ctx or default_context()
     dbl = precision == "double"
     rt, ct = (np.float64, np.complex128) if dbl else (np.float32, np.complex64)
     wl = np.ascontiguousarray(wl, dtype=rt)
-    s = np.asarray(s, dtype=ct)
+    s = np.ascontiguousarray(s, dtype=ct)   # row-major per matrix, turned on the GPU
     B, N = s.shape[0], s.shape[1]
-    # column-major per matrix: store transposed so that memory order matches F layout
-    sF = np.ascontiguousarray(np.transpose(s, (0, 2, 1)))
     xyzF = np.ascontiguousarray(np.transpose(np.asarray(xyz, dtype=rt), (0, 2, 1)))
     d = np.zeros((B, N), dtype=rt)
-    vF = np.zeros((B, N, N), dtype=ct)
+    vF = np.empty((B, N, N), dtype=ct)
     nred = np.zeros(B, dtype=np.uint64)
     scale = np.zeros(B, dtype=rt)
-    fn = ctx._lib.bipp_eigh_gram_batched_d if dbl else ctx._lib.bipp_eigh_gram_batched_s
-    check(fn(ctx.handle, B, N, _ptr(wl), _ptr(sF), _ptr(xyzF), _ptr(d), _ptr(vF), _ptr(nred), _ptr(scale)))
+    fn = ctx._lib.bipp_eigh_gram_batched_rows_d if dbl else ctx._lib.bipp_eigh_gram_batched_rows_s
+    check(fn(ctx.handle, B, N, _ptr(wl), _ptr(s), _ptr(xyzF), _ptr(d), _ptr(vF), _ptr(nred), _ptr(scale)))
     v = np.transpose(vF, (0, 2, 1))
     return v, d, nred.astype(np.int64), scale
 

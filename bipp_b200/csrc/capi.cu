@@ -381,9 +381,8 @@ BippError bipp_image_synthesis(bipp_ctx_t ctx, const bipp_nufft_options* opt, co
       const float scale = ds->scale(ds->user, id);
       ds->uvw(ds->user, id, uvw, nB);
       ds->eig_vec(ds->user, id, v, nAnt);
-      // uvw scaled in single precision as the reference's float path
+      // uvw scaled in single precision as the reference's float path, on the device
       const float uvwScale = twoPi / wl;   // float division (src/nufft_synthesis.cpp:150-154)
-      for (size_t i = 0; i < nB * 3; ++i) uvw[i] *= uvwScale;
       for (size_t im = 0; im < nImages; ++im) {
         const float* d = eigvals[im * nSamples + order[im][k]];
         for (size_t c = 0; c < nBeam; ++c) ks[im * nBeam + c] = scale * d[c];
@@ -395,6 +394,7 @@ BippError bipp_image_synthesis(bipp_ctx_t ctx, const bipp_nufft_options* opt, co
         const long long ld = nufft_stage_ld(pl);
         float* su = nufft_stage_uvw(pl);
         for (int c = 0; c < 3; ++c) h2d(ctx, su + c * ld, uvw + c * nB, nB * sizeof(float));
+        nufft_scale_staged_uvw(pl, uvwScale);
         if (g0 + 4 >= nImages) host.record(slot, ctx->stream);   // last reader of the slot
         // VV of the group's images in one launch: "matrix" b = image g0 + b, the same
         // eigenvectors, its own column scales, output into the image's staging slot
@@ -414,14 +414,8 @@ BippError bipp_image_synthesis(bipp_ctx_t ctx, const bipp_nufft_options* opt, co
       }
     }
     sync(ctx);
-    for (size_t im = 0; im < nImages; ++im) {
-      const BippError e = bipp_nufft_get_image(plans[im / 4], im % 4, images + im * nPixel);
-      if (e != BIPP_SUCCESS) throw Error(e, bipp_last_error());
-    }
-    if (opt->normalizeImage) {
-      const float s = 1.f / float(nSamples);
-      for (size_t i = 0; i < nImages * nPixel; ++i) images[i] *= s;
-    }
+    const float s = opt->normalizeImage ? 1.f / float(nSamples) : 1.f;
+    for (size_t im = 0; im < nImages; im += 4) nufft_take_images(plans[im / 4], s, images + im * nPixel);
   });
 }
 

@@ -104,6 +104,43 @@ __global__ void unbeam_kernel(int nAnt, int nBeam, int nred, const C* __restrict
   }
 }
 
+// W = I, every matrix of a batch: rows idx[r] of out (nAnt x nAnt per matrix) = X[r, :] over the
+// columns [kLo, kHi) of krange (null: all kept ones), zero elsewhere. One CTA row per matrix;
+// the inverse of idx in shared memory (nAnt ints).
+template <typename C>
+__global__ void __launch_bounds__(256) expand_rows_kernel(int nAnt, const int* __restrict__ nred, const C* __restrict__ X,
+                                                          int Nmax, const int* __restrict__ idx,
+                                                          const int* __restrict__ krange, C* __restrict__ out) {
+  using R = decltype(C{}.x);
+  extern __shared__ int ex_row[];
+  const int b = blockIdx.y, n = nred[b];
+  for (int a = threadIdx.x; a < nAnt; a += blockDim.x) ex_row[a] = -1;
+  __syncthreads();
+  for (int r = threadIdx.x; r < n; r += blockDim.x) ex_row[idx[(long long)b * Nmax + r]] = r;
+  __syncthreads();
+  const int kLo = krange ? krange[2 * b] : 0, kHi = krange ? min(n, krange[2 * b + 1]) : n;
+  const C* Xb = X + (long long)b * Nmax * Nmax;
+  C* o = out + (long long)b * nAnt * nAnt;
+  for (int c = blockIdx.x; c < nAnt; c += gridDim.x)
+    for (int a = threadIdx.x; a < nAnt; a += blockDim.x) {
+      const int r = ex_row[a];
+      o[a + (long long)c * nAnt] = (r >= 0 && c >= kLo && c < kHi) ? Xb[r + (long long)c * Nmax] : mk(R(0), R(0));
+    }
+}
+
+// out[b](i, j) = in[b](j, i) of n x n matrices, 32 x 32 tiles
+template <typename C>
+__global__ void __launch_bounds__(256) transpose_kernel(int n, const C* __restrict__ in, C* __restrict__ out) {
+  __shared__ C t[32][33];
+  const long long off = (long long)blockIdx.z * n * n;
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int k = y; k < 32; k += 8)
+    if (r0 + x < n && c0 + k < n) t[k][x] = in[off + r0 + x + (long long)(c0 + k) * n];
+  __syncthreads();
+  for (int k = y; k < 32; k += 8)
+    if (c0 + x < n && r0 + k < n) out[off + c0 + x + (long long)(r0 + k) * n] = t[x][k];
+}
+
 __global__ void pad_eigenvalues_kernel(int nBatch, int nBeam, const int* __restrict__ nred, const double* __restrict__ lam,
                                        int Nmax, double* __restrict__ out) {
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)nBatch * nBeam;
@@ -504,28 +541,24 @@ static void eigh_host(bipp_ctx_s* ctx, bool gram, T wl, size_t nAntenna, size_t 
       if (val != CS(r == c ? 1 : 0, 0)) { identity = false; break; }
     }
   const int Nmax = (int)nBeam;
-  std::vector<CS> sh(nBeam * nBeam);
-  for (size_t c = 0; c < nBeam; ++c)
-    for (size_t r = 0; r < nBeam; ++r) sh[r + c * nBeam] = sp[r + c * lds];
   std::vector<double> xyzh(gram ? nAntenna * 3 : 0);
   for (size_t c = 0; gram && c < 3; ++c)
     for (size_t r = 0; r < nAntenna; ++r) xyzh[r + c * nAntenna] = (double)xyz[r + c * ldxyz];
   double wld = (double)wl;
 
-  DevBuf dS(ctx, sh.size() * sizeof(C)), dX(ctx, xyzh.size() * sizeof(double) + 8), dWl(ctx, sizeof(double));
+  DevBuf dS(ctx, nBeam * nBeam * sizeof(C)), dX(ctx, xyzh.size() * sizeof(double) + 8), dWl(ctx, sizeof(double));
   DevBuf dIdx(ctx, Nmax * sizeof(int)), dNred(ctx, sizeof(int)), dNvis(ctx, sizeof(long long)), dStatus(ctx, sizeof(int));
   DevBuf dLam(ctx, Nmax * sizeof(double));
   DevBuf dW;
-  h2d(ctx, dS.get(), sh.data(), sh.size() * sizeof(C));
+  B2_CUDA(cudaMemcpy2DAsync(dS.get(), nBeam * sizeof(C), sp, lds * sizeof(C), nBeam * sizeof(C), nBeam,
+                            cudaMemcpyHostToDevice, ctx->stream));
   if (gram) h2d(ctx, dX.get(), xyzh.data(), xyzh.size() * sizeof(double));
   h2d(ctx, dWl.get(), &wld, sizeof(double));
   dStatus.zero();
   if (!identity || (v && !identity)) {
-    std::vector<CS> wh(nAntenna * nBeam);
-    for (size_t c = 0; c < nBeam; ++c)
-      for (size_t r = 0; r < nAntenna; ++r) wh[r + c * nAntenna] = wp[r + c * ldw];
-    dW.alloc(ctx, wh.size() * sizeof(C));
-    h2d(ctx, dW.get(), wh.data(), wh.size() * sizeof(C));
+    dW.alloc(ctx, nAntenna * nBeam * sizeof(C));
+    B2_CUDA(cudaMemcpy2DAsync(dW.get(), nAntenna * sizeof(C), wp, ldw * sizeof(C), nAntenna * sizeof(C), nBeam,
+                              cudaMemcpyHostToDevice, ctx->stream));
   }
   EigWork<T> work;
   work.reserve(ctx, 1, Nmax);
@@ -600,23 +633,12 @@ static void eigh_host(bipp_ctx_s* ctx, bool gram, T wl, size_t nAntenna, size_t 
   *scale = nvis ? T(1) / T(nvis) : T(0);
 }
 
-// columns of v (nAnt x nAnt) outside the computed eigenvector range [kLo, kHi) of the
-// matrix (the ranked solves compute part of the eigenpairs) set to zero
-__global__ void zero_outside_range_kernel(int nAnt, const int* __restrict__ krange, float2* __restrict__ v) {
-  const int kLo = krange[0], kHi = krange[1];
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)nAnt * nAnt;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e / nAnt);
-    if (c < kLo || c >= kHi) v[e] = make_float2(0.f, 0.f);
-  }
-}
-
-// batched eigh_gram, W = I; with `ro` (single precision) the ranked forms: the full solve,
+// batched eigh_gram, W = I; rowMajor: the matrices of s hold element (i, j) at i nAnt + j; with `ro` (single precision) the ranked forms: the full solve,
 // the exact range above a threshold (Sturm counts) or the predicted partial solve
 template <typename T>
 static void eigh_gram_batched_host(bipp_ctx_s* ctx, size_t nBatch, size_t nAnt, const T* wl, const void* s,
                                    const T* xyz, T* d, void* v, size_t* nBeamReduced, T* scale,
-                                   const RankOpts* ro = nullptr) {
+                                   const RankOpts* ro = nullptr, bool rowMajor = false) {
   using C = typename Cplx<T>::type;
   require(nBatch > 0 && nAnt > 0, "empty problem");
   require(s && xyz && wl && d && nBeamReduced && scale, "null pointer", BIPP_INVALID_POINTER_ERROR);
@@ -638,6 +660,7 @@ static void eigh_gram_batched_host(bipp_ctx_s* ctx, size_t nBatch, size_t nAnt, 
   DevBuf dS(ctx, chunk * n2 * sizeof(C)), dX(ctx, xyzh.size() * sizeof(double)), dWl(ctx, nBatch * sizeof(double));
   DevBuf dIdx(ctx, nBatch * Nmax * sizeof(int)), dNred(ctx, nBatch * sizeof(int)), dNvis(ctx, nBatch * sizeof(long long));
   DevBuf dStatus(ctx, nBatch * sizeof(int)), dLam(ctx, nBatch * Nmax * sizeof(double)), dLamPad(ctx, chunk * nAnt * sizeof(double));
+  // eigenvectors; before the solve, the matrices as they arrive when they are row-major
   DevBuf dV(ctx, chunk * n2 * sizeof(C));
   h2d(ctx, dX.get(), xyzh.data(), xyzh.size() * sizeof(double));
   h2d(ctx, dWl.get(), wlh.data(), nBatch * sizeof(double));
@@ -670,7 +693,13 @@ static void eigh_gram_batched_host(bipp_ctx_s* ctx, size_t nBatch, size_t nAnt, 
   std::vector<double> lamh(chunk * nAnt);
   for (size_t b0 = 0; b0 < nBatch; b0 += chunk) {
     const size_t nb = std::min(chunk, nBatch - b0);
-    h2d(ctx, dS.get(), static_cast<const char*>(s) + b0 * n2 * sizeof(C), nb * n2 * sizeof(C));
+    h2d(ctx, rowMajor ? dV.get() : dS.get(), static_cast<const char*>(s) + b0 * n2 * sizeof(C), nb * n2 * sizeof(C));
+    if (rowMajor) {
+      const int tiles = (Nmax + 31) / 32;
+      count_launch();
+      transpose_kernel<C><<<dim3(tiles, tiles, (unsigned)nb), 256, 0, ctx->stream>>>(Nmax, dV.get<C>(), dS.get<C>());
+      B2_CHECK_LAUNCH();
+    }
     EigLaunch<T> L{};
     L.nBatch = (int)nb; L.nBeam = (int)nAnt; L.nAnt = (int)nAnt; L.Nmax = Nmax;
     L.S = dS.get<C>(); L.sStride = (long long)n2; L.lds = (int)nAnt;
@@ -711,25 +740,18 @@ static void eigh_gram_batched_host(bipp_ctx_s* ctx, size_t nBatch, size_t nAnt, 
       if (ro->features) d2h(ctx, ro->features + b0 * kRankFeatures, dFeat.get(), nb * kRankFeatures * sizeof(float));
       d2h(ctx, kr.data(), work.krange.get(), 2 * nb * sizeof(int));
     }
-    // outputs for this chunk: scatter each matrix's eigenvectors to its kept antenna rows
+    // outputs for this chunk: every matrix's eigenvectors to their kept antenna rows
     std::vector<int> nr(nb);
     d2h(ctx, nr.data(), dNred.get<int>() + b0, nb * sizeof(int));
-    sync(ctx);
-    for (size_t b = 0; b < nb; ++b) {
+    if (v) {
+      auto k = expand_rows_kernel<C>;
+      const size_t smem = nAnt * sizeof(int);
       count_launch();
-      unbeam_kernel<C><<<128, 256, 0, ctx->stream>>>((int)nAnt, (int)nAnt, nr[b],
-                                                     work.X(true) + (long long)b * Nmax * Nmax, Nmax,
-                                                     dIdx.get<int>() + (b0 + b) * Nmax, nullptr, 0, 1,
-                                                     dV.get<C>() + b * n2);
-      if constexpr (sizeof(T) == 4) {
-        if (ro && ro->mode >= 1) {
-          count_launch();
-          zero_outside_range_kernel<<<128, 256, 0, ctx->stream>>>((int)nAnt, work.krange.template get<int>() + 2 * b,
-                                                                  dV.get<float2>() + b * n2);
-        }
-      }
+      k<<<dim3((unsigned)std::min<size_t>(nAnt, 64), (unsigned)nb), 256, smem, ctx->stream>>>(
+          (int)nAnt, dNred.get<int>() + b0, work.X(true), Nmax, dIdx.get<int>() + b0 * Nmax,
+          ro && ro->mode >= 1 ? work.krange.template get<int>() : nullptr, dV.get<C>());
+      B2_CHECK_LAUNCH();
     }
-    B2_CHECK_LAUNCH();
     count_launch();
     pad_eigenvalues_kernel<<<64, 256, 0, ctx->stream>>>((int)nb, (int)nAnt, dNred.get<int>() + b0,
                                                         dLam.get<double>() + b0 * Nmax, Nmax, dLamPad.get<double>());
@@ -881,6 +903,20 @@ BippError bipp_eigh_gram_batched_d(bipp_ctx_t ctx, size_t nBatch, size_t nAntenn
   return guard([&] {
     require(ctx != nullptr, "null context", BIPP_INVALID_HANDLE_ERROR);
     eigh_gram_batched_host<double>(ctx, nBatch, nAntenna, wl, s, xyz, d, v, nBeamReduced, scale);
+  });
+}
+BippError bipp_eigh_gram_batched_rows_s(bipp_ctx_t ctx, size_t nBatch, size_t nAntenna, const float* wl, const void* s,
+                                        const float* xyz, float* d, void* v, size_t* nBeamReduced, float* scale) {
+  return guard([&] {
+    require(ctx != nullptr, "null context", BIPP_INVALID_HANDLE_ERROR);
+    eigh_gram_batched_host<float>(ctx, nBatch, nAntenna, wl, s, xyz, d, v, nBeamReduced, scale, nullptr, true);
+  });
+}
+BippError bipp_eigh_gram_batched_rows_d(bipp_ctx_t ctx, size_t nBatch, size_t nAntenna, const double* wl, const void* s,
+                                        const double* xyz, double* d, void* v, size_t* nBeamReduced, double* scale) {
+  return guard([&] {
+    require(ctx != nullptr, "null context", BIPP_INVALID_HANDLE_ERROR);
+    eigh_gram_batched_host<double>(ctx, nBatch, nAntenna, wl, s, xyz, d, v, nBeamReduced, scale, nullptr, true);
   });
 }
 BippError bipp_eigh_gram_batched_ranked_s(bipp_ctx_t ctx, size_t nBatch, size_t nAntenna, const float* wl,

@@ -89,45 +89,100 @@ static int next_smooth(int n) {
   }
 }
 
-Lattice fit_lattice(const std::vector<double>& l, const std::vector<double>& m) {
-  Lattice L;
-  const size_t P = l.size();
-  if (P < 4) return L;
-  // candidate Nb: first index where the b-direction step changes, else try sqrt(P) and divisors
+// Distance of pixel p = a nb + b from the lattice, as the host forms it (no contraction)
+__device__ __forceinline__ double lattice_resid(double x, double x0, double A, double B, int a, int b) {
+  return __dsub_rn(x, __dadd_rn(__dadd_rn(x0, __dmul_rn((double)a, A)), __dmul_rn((double)b, B)));
+}
+
+// max |residual| of l and m over all pixels, as the bits of non-negative doubles
+__global__ void __launch_bounds__(256) lattice_check_kernel(Lattice L, const float* __restrict__ l,
+                                                            const float* __restrict__ m,
+                                                            unsigned long long* __restrict__ out) {
+  __shared__ double red[32];
+  double rl = 0.0, rm = 0.0;
+  const long long P = (long long)L.Na * L.Nb;
+  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
+    const int a = (int)(p / L.Nb), b = (int)(p % L.Nb);
+    const double el = fabs(lattice_resid((double)l[p], L.l0, L.Al, L.Bl, a, b));
+    const double em = fabs(lattice_resid((double)m[p], L.m0, L.Am, L.Bm, a, b));
+    rl = fmax(rl, el);
+    rm = fmax(rm, em);
+  }
+  rl = block_max(rl, red, 0.0);
+  __syncthreads();
+  rm = block_max(rm, red, 0.0);
+  if (threadIdx.x == 0) {
+    atomicMax(out, (unsigned long long)__double_as_longlong(rl));
+    atomicMax(out + 1, (unsigned long long)__double_as_longlong(rm));
+  }
+}
+
+// residuals of every pixel and n - nc
+__global__ void __launch_bounds__(256) lattice_pixels_kernel(Lattice L, const float* __restrict__ l,
+                                                             const float* __restrict__ m, const float* __restrict__ n,
+                                                             double nc, double* __restrict__ dl,
+                                                             double* __restrict__ dm, double* __restrict__ nTilde) {
+  const long long P = (long long)L.Na * L.Nb;
+  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
+    const int a = (int)(p / L.Nb), b = (int)(p % L.Nb);
+    dl[p] = lattice_resid((double)l[p], L.l0, L.Al, L.Bl, a, b);
+    dm[p] = lattice_resid((double)m[p], L.m0, L.Am, L.Bm, a, b);
+    nTilde[p] = __dsub_rn((double)n[p], nc);
+  }
+}
+
+// Lattice of FP32 pixel coordinates (host l, m; the same on the device at lDev, mDev): the
+// candidate row lengths are tried on the corners and a few thousand pixels here, and the
+// one that passes on all of them there.
+static Lattice fit_lattice(bipp_ctx_s* ctx, size_t P, const float* l, const float* m, const float* lDev,
+                           const float* mDev) {
+  if (P < 4) return Lattice{};
+  // candidate Nb: try sqrt(P), then the divisors
   std::vector<int> cands;
   const int sq = (int)std::llround(std::sqrt((double)P));
   if ((size_t)sq * sq == P) cands.push_back(sq);
   for (int nb = 2; nb <= (int)P / 2 && cands.size() < 64; ++nb)
     if (P % nb == 0 && nb != sq) cands.push_back(nb);
+  DevBuf out(ctx, 2 * sizeof(unsigned long long));
   for (int nb : cands) {
     const int na = (int)(P / nb);
     if (na < 2) continue;
-    const double Bl = (l[nb - 1] - l[0]) / (nb - 1), Bm = (m[nb - 1] - m[0]) / (nb - 1);
-    const double Al = (l[(size_t)(na - 1) * nb] - l[0]) / (na - 1), Am = (m[(size_t)(na - 1) * nb] - m[0]) / (na - 1);
-    const double step = std::max(std::hypot(Bl, Bm), std::hypot(Al, Am));
+    Lattice L;
+    L.Na = na;
+    L.Nb = nb;
+    L.l0 = l[0];
+    L.m0 = m[0];
+    L.Bl = ((double)l[nb - 1] - L.l0) / (nb - 1);
+    L.Bm = ((double)m[nb - 1] - L.m0) / (nb - 1);
+    L.Al = ((double)l[(size_t)(na - 1) * nb] - L.l0) / (na - 1);
+    L.Am = ((double)m[(size_t)(na - 1) * nb] - L.m0) / (na - 1);
+    const double step = std::max(std::hypot(L.Bl, L.Bm), std::hypot(L.Al, L.Am));
     if (!(step > 0)) continue;
-    double rl = 0, rm = 0;
+    const size_t stride = std::max<size_t>(1, P / 4099);
     bool ok = true;
-    for (int a = 0; a < na && ok; ++a)
-      for (int b = 0; b < nb; ++b) {
-        const size_t p = (size_t)a * nb + b;
-        const double el = std::fabs(l[p] - (l[0] + a * Al + b * Bl));
-        const double em = std::fabs(m[p] - (m[0] + a * Am + b * Bm));
-        rl = std::max(rl, el);
-        rm = std::max(rm, em);
-        if (el > 1e-3 * step || em > 1e-3 * step) { ok = false; break; }
-      }
-    if (!ok) continue;
+    for (size_t q = 0; q < P && ok; q += stride) {
+      const int a = (int)(q / nb), b = (int)(q % nb);
+      ok = !(std::fabs(l[q] - (L.l0 + a * L.Al + b * L.Bl)) > 1e-3 * step) &&
+           !(std::fabs(m[q] - (L.m0 + a * L.Am + b * L.Bm)) > 1e-3 * step);
+    }
     // non-degenerate lattice
-    const double det = Al * Bm - Am * Bl;
-    if (std::fabs(det) < 1e-12 * step * step) continue;
+    const double det = L.Al * L.Bm - L.Am * L.Bl;
+    if (!ok || std::fabs(det) < 1e-12 * step * step) continue;
+    out.zero();
+    count_launch();
+    lattice_check_kernel<<<(int)std::min<size_t>(1024, (P + 255) / 256), 256, 0, ctx->stream>>>(
+        L, lDev, mDev, out.get<unsigned long long>());
+    B2_CHECK_LAUNCH();
+    double r[2];
+    d2h(ctx, r, out.get(), sizeof(r));
+    sync(ctx);
+    if (!(r[0] <= 1e-3 * step && r[1] <= 1e-3 * step)) continue;
     L.ok = true;
-    L.Na = na; L.Nb = nb;
-    L.l0 = l[0]; L.m0 = m[0]; L.Al = Al; L.Bl = Bl; L.Am = Am; L.Bm = Bm;
-    L.maxResidL = rl; L.maxResidM = rm;
+    L.maxResidL = r[0];
+    L.maxResidM = r[1];
     return L;
   }
-  return L;
+  return Lattice{};
 }
 
 // ---------------------------------------------------------------------------------------
@@ -250,16 +305,36 @@ void NufftCore::inverse_fft(int slabPlanes, int planesUsed, int firstLayer, floa
                         CUFFT_INVERSE));
 }
 
-void NufftCore::setup(bipp_ctx_s* ctx, const Lattice& lat, const std::vector<double>& n, double eps, int nch,
-                      const std::vector<double>* dl, const std::vector<double>* dm, double su, double sv,
-                      int levels) {
+void NufftCore::setup(bipp_ctx_s* ctx, const Lattice& lat, const std::vector<double>& n, double eps, int nch) {
+  require((long long)n.size() == (long long)lat.Na * lat.Nb, "pixel n size mismatch");
+  setup_grid(ctx, lat, *std::min_element(n.begin(), n.end()), *std::max_element(n.begin(), n.end()), eps, nch, false);
+  std::vector<double> nt(n.size());
+  for (size_t p = 0; p < n.size(); ++p) nt[p] = n[p] - g_.nc;
+  h2d(ctx, nTilde_.get(), nt.data(), nt.size() * sizeof(double));
+  setup_decon();
+  sync(ctx);
+}
+
+void NufftCore::setup(bipp_ctx_s* ctx, const Lattice& lat, const float* l, const float* m, const float* n, double nmin,
+                      double nmax, double eps, int nch) {
+  setup_grid(ctx, lat, nmin, nmax, eps, nch, true);
+  const long long P = num_pixels();
+  count_launch();
+  lattice_pixels_kernel<<<(int)std::min<long long>(4096, (P + 255) / 256), 256, 0, ctx->stream>>>(
+      lat, l, m, n, g_.nc, dl_.get<double>(), dm_.get<double>(), nTilde_.get<double>());
+  B2_CHECK_LAUNCH();
+  setup_decon();
+  sync(ctx);
+}
+
+void NufftCore::setup_grid(bipp_ctx_s* ctx, const Lattice& lat, double nmin, double nmax, double eps, int nch,
+                           bool corr) {
   ctx_ = ctx;
   require(lat.ok, "pixel coordinates are not on a lattice");
-  corrCapable_ = (dl != nullptr);
+  corrCapable_ = corr;
   require(nch >= 1 && nch * (corrCapable_ ? 3 : 1) <= kMaxChan, "too many NUFFT channels");
   nch_ = nch;
   levels_ = nch;
-  (void)levels;
   eps_ = eps;
   g_ = NufftGeom{};
   g_.l0 = lat.l0; g_.m0 = lat.m0; g_.Al = lat.Al; g_.Bl = lat.Bl; g_.Am = lat.Am; g_.Bm = lat.Bm;
@@ -297,42 +372,39 @@ void NufftCore::setup(bipp_ctx_s* ctx, const Lattice& lat, const std::vector<dou
     h2d(ctx, fftTw_.get(), tw.data(), tw.size() * sizeof(float2));
   }
   const long long P = (long long)g_.Na * g_.Nb;
-  require((long long)n.size() == P, "pixel n size mismatch");
-  double nmin = *std::min_element(n.begin(), n.end()), nmax = *std::max_element(n.begin(), n.end());
   g_.nc = 0.5 * (nmin + nmax);
   Sn_ = std::max(0.5 * (nmax - nmin), 1e-12);
   g_.hw = M_PI / (sigma * Sn_);
   g_.ihx = 1.0 / g_.hx;
   g_.ihy = 1.0 / g_.hy;
   g_.ihw = 1.0 / g_.hw;
-  std::vector<double> nt(P);
-  for (long long p = 0; p < P; ++p) nt[p] = n[p] - g_.nc;
   nTilde_.alloc(ctx, P * sizeof(double));
-  h2d(ctx, nTilde_.get(), nt.data(), P * sizeof(double));
   corrTerms_ = false;
-  su_ = su;
-  sv_ = sv;
+  su_ = sv_ = 1.0;
   if (corrCapable_) {
     dl_.alloc(ctx, P * sizeof(double));
     dm_.alloc(ctx, P * sizeof(double));
-    h2d(ctx, dl_.get(), dl->data(), P * sizeof(double));
-    h2d(ctx, dm_.get(), dm->data(), P * sizeof(double));
   }
-  // deconvolution factors (independent of the points)
+  decon_.alloc(ctx, P * sizeof(double));
+  acc_.alloc(ctx, (size_t)levels_ * (corrCapable_ ? 3 : 1) * P * sizeof(float2));
+  zeroAcc_.alloc(ctx, kMaxChan * sizeof(double));
+}
+
+// deconvolution factors (independent of the points), from nTilde_; the caller synchronises
+void NufftCore::setup_decon() {
+  bipp_ctx_s* ctx = ctx_;
+  const long long P = num_pixels();
   std::vector<double> qx, qwt;
   gauss_legendre(2 * g_.W + 16, qx, qwt);
   qz_.alloc(ctx, qx.size() * sizeof(double));
   qw_.alloc(ctx, qwt.size() * sizeof(double));
   h2d(ctx, qz_.get(), qx.data(), qx.size() * sizeof(double));
   h2d(ctx, qw_.get(), qwt.data(), qwt.size() * sizeof(double));
-  decon_.alloc(ctx, P * sizeof(double));
   count_launch();
   decon_kernel<<<std::min<long long>(4096, (P + 255) / 256), 256, 0, ctx->stream>>>(
       g_, nTilde_.get<double>(), qz_.get<double>(), qw_.get<double>(), (int)qx.size(), decon_.get<double>());
   B2_CHECK_LAUNCH();
-  acc_.alloc(ctx, (size_t)levels_ * (corrCapable_ ? 3 : 1) * P * sizeof(float2));
-  zeroAcc_.alloc(ctx, kMaxChan * sizeof(double));
-  sync(ctx);
+  sync(ctx);   // qx, qwt leave scope
 }
 
 void NufftCore::set_corr(bool on, double su, double sv) {
@@ -791,8 +863,6 @@ static void nufft_transform_lattice(bipp_nufft_s* p, long long n, long long ld) 
   // residual phase could exceed a tenth of the tolerance
   const double bound = p->residL * su + p->residM * sv;
   p->core.set_corr(bound > 0.1 * p->opt.tolerance, su, sv);
-  const size_t groups = p->nImages;
-  (void)groups;
   BaselinePoints bp{};
   bp.n = n;
   bp.uvw = p->uvw.get<float>();
@@ -832,6 +902,43 @@ float2* nufft_stage_values(bipp_nufft_t p, size_t im) {
   return p->values.get<float2>() + im * (long long)p->batch * p->nBaselines + p->count * p->nBaselines;
 }
 long long nufft_stage_ld(bipp_nufft_t p) { return (long long)p->batch * p->nBaselines; }
+__global__ void scale_stage_kernel(float* __restrict__ u, long long ld, long long n, float s) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 3 * n; i += (long long)gridDim.x * blockDim.x)
+    u[(i / n) * ld + i % n] *= s;
+}
+void nufft_scale_staged_uvw(bipp_nufft_t p, float s) {
+  count_launch();
+  scale_stage_kernel<<<(int)std::min<size_t>(1024, (3 * p->nBaselines + 255) / 256), 256, 0, p->ctx->stream>>>(
+      nufft_stage_uvw(p), nufft_stage_ld(p), (long long)p->nBaselines, s);
+  B2_CHECK_LAUNCH();
+}
+static void nufft_fold(bipp_nufft_s* p);
+__global__ void scale_floats_kernel(float* __restrict__ x, long long n, float s) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    x[i] *= s;
+}
+void nufft_take_images(bipp_nufft_t p, float s, float* images) {
+  nufft_transform(p);
+  nufft_fold(p);
+  const size_t n = p->nImages * p->nPixel;
+  if (s != 1.f) {
+    count_launch();
+    scale_floats_kernel<<<(int)std::min<size_t>(2048, (n + 255) / 256), 256, 0, p->ctx->stream>>>(p->images.get<float>(),
+                                                                                                (long long)n, s);
+    B2_CHECK_LAUNCH();
+  }
+  d2h(p->ctx, images, p->images.get(), n * sizeof(float));
+  sync(p->ctx);
+}
+// fold the FP64 direct-sum accumulator of pixels off a lattice into the float images
+static void nufft_fold(bipp_nufft_s* p) {
+  if (p->lattice) return;
+  count_launch();
+  add_double_to_float_kernel<<<256, 256, 0, p->ctx->stream>>>(p->imagesD.get<double>(),
+                                                             (long long)(p->nImages * p->nPixel), p->images.get<float>());
+  B2_CHECK_LAUNCH();
+  p->imagesD.zero();
+}
 void nufft_commit(bipp_nufft_t p) {
   ++p->count;
   if (p->count >= p->batch) nufft_transform(p);
@@ -856,34 +963,27 @@ BippError bipp_nufft_create(bipp_ctx_t ctx, const bipp_nufft_options* opt, size_
     size_t batch = opt->sampleBatchSize;
     if (batch == 0) batch = std::max<size_t>(1, (size_t)2000000000ull / (20 * nBaselines));
     p->batch = batch;
-    std::vector<double> l(nPixel), m(nPixel), nn(nPixel);
-    for (size_t i = 0; i < nPixel; ++i) {
-      l[i] = lmn[i];
-      m[i] = lmn[i + ldlmn];
-      nn[i] = lmn[i + 2 * ldlmn];
-    }
-    Lattice lat = fit_lattice(l, m);
+    const float *l = lmn, *m = lmn + ldlmn, *n = lmn + 2 * ldlmn;
+    DevBuf lmnF(ctx, 3 * nPixel * sizeof(float));
+    float* dev = lmnF.get<float>();
+    for (int c = 0; c < 3; ++c) h2d(ctx, dev + c * nPixel, lmn + c * ldlmn, nPixel * sizeof(float));
+    Lattice lat = fit_lattice(ctx, nPixel, l, m, dev, dev + nPixel);
     p->lattice = lat.ok;
     if (lat.ok) {
-      std::vector<double> dl(nPixel), dm(nPixel);
-      for (int a = 0; a < lat.Na; ++a)
-        for (int b = 0; b < lat.Nb; ++b) {
-          const size_t q = (size_t)a * lat.Nb + b;
-          dl[q] = l[q] - (lat.l0 + a * lat.Al + b * lat.Bl);
-          dm[q] = m[q] - (lat.m0 + a * lat.Am + b * lat.Bm);
-        }
       p->residL = lat.maxResidL;
       p->residM = lat.maxResidM;
-      p->core.setup(ctx, lat, nn, std::max<double>(opt->tolerance, 1e-12), (int)nImages, &dl, &dm);
-    } else {
-      std::vector<double> h(3 * nPixel);
-      for (size_t i = 0; i < nPixel; ++i) {
-        h[i] = l[i];
-        h[i + nPixel] = m[i];
-        h[i + 2 * nPixel] = nn[i];
+      float lo = n[0], hi = n[0];
+      for (size_t i = 1; i < nPixel; ++i) {
+        lo = std::min(lo, n[i]);
+        hi = std::max(hi, n[i]);
       }
-      p->lmnDev.alloc(ctx, h.size() * sizeof(double));
-      h2d(ctx, p->lmnDev.get(), h.data(), h.size() * sizeof(double));
+      p->core.setup(ctx, lat, dev, dev + nPixel, dev + 2 * nPixel, lo, hi, std::max<double>(opt->tolerance, 1e-12),
+                    (int)nImages);
+    } else {
+      p->lmnDev.alloc(ctx, 3 * nPixel * sizeof(double));
+      count_launch();
+      f2d_kernel<<<256, 256, 0, ctx->stream>>>(dev, (long long)(3 * nPixel), p->lmnDev.get<double>());
+      B2_CHECK_LAUNCH();
       p->imagesD.alloc(ctx, nImages * nPixel * sizeof(double));
       p->imagesD.zero();
     }
@@ -949,14 +1049,7 @@ BippError bipp_nufft_get_image(bipp_nufft_t plan, size_t imgIdx, float* image) {
     require(imgIdx < p->nImages, "image index out of range");
     nufft_transform(p);
     bipp_ctx_s* ctx = p->ctx;
-    if (!p->lattice) {
-      // fold the FP64 direct-sum accumulator into the float images
-      count_launch();
-      add_double_to_float_kernel<<<256, 256, 0, ctx->stream>>>(p->imagesD.get<double>(), (long long)(p->nImages * p->nPixel),
-                                                              p->images.get<float>());
-      B2_CHECK_LAUNCH();
-      p->imagesD.zero();
-    }
+    nufft_fold(p);
     d2h(ctx, image, p->images.get<float>() + imgIdx * p->nPixel, p->nPixel * sizeof(float));
     sync(ctx);
   });

@@ -22,8 +22,6 @@ struct Lattice {
   double maxResidL = 0, maxResidM = 0;  // max |l - lattice|, |m - lattice|
 };
 
-Lattice fit_lattice(const std::vector<double>& l, const std::vector<double>& m);
-
 // ES kernel width and shape for a tolerance at upsampling factor 2 (as used by type-1/3
 // NUFFTs with the "exponential of semicircle" kernel).
 // fine-grid oversampling in x, y and w: the tuning table's nufft.grid_per_1024 / 1024
@@ -33,9 +31,11 @@ void es_params(double eps, double sigma, int& W, float& beta);
 class NufftCore {
 public:
   // Pixel side: lattice + per-pixel n (FP64). nch = channels per transform.
-  void setup(bipp_ctx_s* ctx, const Lattice& lat, const std::vector<double>& n, double eps, int nch,
-             const std::vector<double>* dl = nullptr, const std::vector<double>* dm = nullptr, double su = 1.0,
-             double sv = 1.0, int levels = 0);
+  void setup(bipp_ctx_s* ctx, const Lattice& lat, const std::vector<double>& n, double eps, int nch);
+  // The same from FP32 pixel coordinates on the device (n between nmin and nmax), with their
+  // residuals from the lattice kept for the first-order channels (set_corr).
+  void setup(bipp_ctx_s* ctx, const Lattice& lat, const float* l, const float* m, const float* n, double nmin,
+             double nmax, double eps, int nch);
 
   // Per transform: w-range of the points (already scaled to phase units).
   void begin(double wmin, double wmax);
@@ -98,6 +98,8 @@ private:
   // pixel (a, b)'s output) or in full by cuFFT
   void inverse_fft(int slabPlanes, int planesUsed, int firstLayer, float2* slab, bool pruned);
   void exclusive_scan(const int* in, int* out, long long n);
+  void setup_grid(bipp_ctx_s* ctx, const Lattice& lat, double nmin, double nmax, double eps, int nch, bool corr);
+  void setup_decon();
 
 public:
   ~NufftCore();
@@ -113,6 +115,11 @@ float* nufft_stage_uvw(bipp_nufft_t p);
 float2* nufft_stage_values(bipp_nufft_t p, size_t im);
 long long nufft_stage_ld(bipp_nufft_t p);
 void nufft_commit(bipp_nufft_t p);
+// multiply the staged uvw of the current sample by s (single precision)
+void nufft_scale_staged_uvw(bipp_nufft_t p, float s);
+// transform what is collected and return all images ([nImages][nPixel], host) times s; the
+// collector's own images are scaled with them, so this ends its use
+void nufft_take_images(bipp_nufft_t p, float s, float* images);
 
 // Gauss-Legendre nodes/weights on [-1, 1]
 void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w);

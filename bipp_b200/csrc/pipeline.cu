@@ -110,9 +110,9 @@ __global__ void levels_kernel(int nSteps, int Nmax, int nLevels, const double* _
   }
 }
 
-__global__ void scale_images_kernel(float* __restrict__ img, long long n, float s) {
+__global__ void scale_images_kernel(const float* __restrict__ img, long long n, float s, float* __restrict__ out) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    img[i] *= s;
+    out[i] = img[i] * s;
 }
 
 }  // namespace bippb200
@@ -584,22 +584,20 @@ BippError bipp_pipeline_images(bipp_pipeline_t pl, float* images, int normalize,
     require(pl && images, "null pointer", BIPP_INVALID_POINTER_ERROR);
     bipp_ctx_s* ctx = pl->ctx;
     const long long n = (long long)pl->nLevels * pl->P;
-    const cudaMemcpyKind kind = onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    B2_CUDA(cudaMemcpyAsync(images, pl->images.get(), n * sizeof(float), kind, ctx->stream));
     if (normalize && pl->stepsDone > 0) {
-      const float s = 1.0f / (float)pl->stepsDone;
-      if (onDevice) {
-        count_launch();
-        scale_images_kernel<<<1024, 256, 0, ctx->stream>>>(images, n, s);
-        B2_CHECK_LAUNCH();
-        sync(ctx);
-      } else {
-        sync(ctx);
-        for (long long i = 0; i < n; ++i) images[i] *= s;
-      }
+      // one pass from the accumulated images to the caller's, or to a buffer that is copied out
+      DevBuf host;
+      if (!onDevice) host.alloc(ctx, n * sizeof(float));
+      float* out = onDevice ? images : host.get<float>();
+      count_launch();
+      scale_images_kernel<<<2048, 256, 0, ctx->stream>>>(pl->images.get<float>(), n, 1.0f / (float)pl->stepsDone, out);
+      B2_CHECK_LAUNCH();
+      if (!onDevice) d2h(ctx, images, out, n * sizeof(float));
     } else {
-      sync(ctx);
+      B2_CUDA(cudaMemcpyAsync(images, pl->images.get(), n * sizeof(float),
+                              onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream));
     }
+    sync(ctx);
   });
 }
 

@@ -114,6 +114,15 @@ BIPP_B200_EXPORT BippError bipp_eigh_gram_batched_d(bipp_ctx_t ctx, size_t nBatc
                                                     const double* wl, const void* s, const double* xyz, double* d,
                                                     void* v, size_t* nBeamReduced, double* scale);
 
+/* The batched forms with s in row-major order (element (i, j) of a step at i nAntenna + j),
+ * turned on the device; everything else as above. */
+BIPP_B200_EXPORT BippError bipp_eigh_gram_batched_rows_s(bipp_ctx_t ctx, size_t nBatch, size_t nAntenna,
+                                                         const float* wl, const void* s, const float* xyz, float* d,
+                                                         void* v, size_t* nBeamReduced, float* scale);
+BIPP_B200_EXPORT BippError bipp_eigh_gram_batched_rows_d(bipp_ctx_t ctx, size_t nBatch, size_t nAntenna,
+                                                         const double* wl, const void* s, const double* xyz, double* d,
+                                                         void* v, size_t* nBeamReduced, double* scale);
+
 /* ---- learned rank predictor --------------------------------------------------------- */
 /* No counterpart in the reference, which computes every eigenpair (LAPACK ?hegv,
  * src/eigensolver.cpp:188-216) and keeps those inside the energy levels afterwards.
