@@ -229,15 +229,23 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
 
   // 1. flags (optional) + compaction (+ Gram for W = I)
   mark(0);
-  {
+  if (L.doFlag) {
     const size_t smem = 2 * (size_t)Nmax * sizeof(int);
     auto k = prep_kernel<T>;
     smem_optin(k, smem);
     count_launch();
-    // W = I: the Gram matrix is real symmetric, stored as FP64 reals (withGram 2)
     k<<<nb, kPrepThreads, smem, st>>>(L.nBeam, L.S, L.sStride, L.lds, L.xyz, L.xyzStride, L.ldxyz, L.wl, L.mode,
-                                      L.eps, (L.gram && L.identityW) ? 2 : 0, Nmax, L.idx, L.nred, L.nvis, A, G,
-                                      L.status, L.doFlag, 1, L.batchOffset);
+                                      L.eps, 0, Nmax, L.idx, L.nred, L.nvis, nullptr, nullptr, L.status, 1, 0,
+                                      L.batchOffset);
+    B2_CHECK_LAUNCH();
+  }
+  {
+    // W = I: the Gram matrix is real symmetric, stored as FP64 reals
+    const int t = (Nmax + 31) / 32;
+    count_launch();
+    compact_kernel<T><<<dim3(t * (t + 1) / 2, nb), 256, 0, st>>>(L.S, L.sStride, L.lds, L.xyz, L.xyzStride, L.ldxyz, L.wl,
+                                                               (L.gram && L.identityW) ? 2 : 0, Nmax, L.idx, L.nred, A,
+                                                               G, L.batchOffset);
     B2_CHECK_LAUNCH();
   }
   if (L.gram && !L.identityW) {
