@@ -173,14 +173,15 @@ tridiag_values_kernel(const double* __restrict__ dIn, const double* __restrict__
   if (act && j == 0) lam[i] = 0.5 * (a + c) / scale;
 }
 
-// 1 / x to a rounding or two by Newton's iteration from the hardware estimate; x is a
-// normal number within 2^+-600 here
-__device__ __forceinline__ double ts_rcp(double x) {
+// a / x to about a rounding: reciprocal by Newton's iteration from the hardware estimate, the
+// quotient corrected by its residual; a and x are normal numbers within 2^+-600 here
+__device__ __forceinline__ double ts_div(double a, double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   y = fma(y, fma(-x, y, 1.0), y);
   y = fma(y, fma(-x, y, 1.0), y);
-  return y;
+  const double q = a * y;
+  return fma(fma(-x, q, a), y, q);
 }
 
 // Eigenvectors of the eigenvalues range[2b] .. range[2b+1]-1 of matrix b (trimmed to
@@ -241,7 +242,7 @@ tridiag_vectors_kernel(const double* __restrict__ dIn, const double* __restrict_
       const int k = role ? n - 2 - t : t;
       const double ek = de[k].y, dn = de[role ? k : k + 1].x;
       p1 = ts_nonzero(p1, p0);
-      if (act) *out = ek * p0 * ts_rcp(p1);
+      if (act) *out = ts_div(ek * p0, p1);
       out += step;
       const double p2 = fma(dn - l, p1, -(ek * ek) * p0);
       p0 = p1;
