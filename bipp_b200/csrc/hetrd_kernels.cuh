@@ -117,8 +117,8 @@ template <int NB> struct HtPanel<double2, NB> {   // pieces 2 q = V_q, 2 q + 1 =
 
 // One strip of SC columns from c0, rows [rBeg, rEnd) (multiples of 32): row sums a x_c into
 // yw[r], column sums conj(a) x_r into yw[c], for the trailing block of rows and columns
-// s0 .. n-1. Columns outside it carry x = 0 and are dropped; x is zero from row n on. On the
-// diagonal the column sum takes the element and the row sum leaves it out.
+// s0 .. n-1. x is zero outside it, and the column sums of columns outside it are dropped. On
+// the diagonal the column sum takes the element and the row sum leaves it out.
 template <typename C, typename R, int SC>
 __device__ __forceinline__ void ht_strip(const C* __restrict__ A, int ld, int n, int s0, int c0, int rBeg, int rEnd,
                                          const C* __restrict__ x, C* __restrict__ yw) {
@@ -126,7 +126,7 @@ __device__ __forceinline__ void ht_strip(const C* __restrict__ A, int ld, int n,
   const C zero = mk(R(0), R(0));
   C xc[SC];
 #pragma unroll
-  for (int u = 0; u < SC; ++u) xc[u] = (c0 + u >= s0 && c0 + u < n) ? x[c0 + u] : zero;
+  for (int u = 0; u < SC; ++u) xc[u] = x[c0 + u];
   C cs[SC];
 #pragma unroll
   for (int u = 0; u < SC; ++u) cs[u] = zero;
@@ -162,20 +162,20 @@ __device__ __forceinline__ void ht_strip(const C* __restrict__ A, int ld, int n,
   };
   C a[SC], b[SC];
   if (r0 == diag) {
-    // columns first .. r of this row are stored; the diagonal is real, enters the column sum
+    // columns up to r of this row are stored; the diagonal is real, enters the column sum
     // and leaves the row sum
-    const int r = r0 + lane, first = r < n ? max(s0, c0) : n;
+    const int r = r0 + lane, cols = r < n ? r - c0 : -1;   // columns c0 .. c0 + cols
     C dg = zero;
 #pragma unroll
     for (int u = 0; u < SC; ++u) {
       a[u] = zero;
-      if (c0 + u >= first && c0 + u <= r) a[u] = get(u);
+      if (u <= cols) a[u] = get(u);
     }
     p += 32;
     if (r0 + 32 < end) load(b, r0 + 32);
 #pragma unroll
     for (int u = 0; u < SC; ++u)
-      if (c0 + u == r) dg = cscale(xc[u], -a[u].x), a[u].y = R(0);
+      if (u == cols) dg = cscale(xc[u], -a[u].x), a[u].y = R(0);
     use(a, r);
     yw[r] = yw[r] + dg;
     r0 += 32;
@@ -225,31 +225,39 @@ __device__ __forceinline__ void ht_rank2k(C* __restrict__ A, int ld, int n, int 
 #pragma unroll
       for (int q = 0; q < NB; ++q) P.get(P.row(r), q, rv[i][q], rw[i][q]);
     }
+    auto column = [&](int c, C* p, bool whole) {
+      C a[ROWS];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        a[i] = mk(R(0), R(0));
+        if (whole || (row[i] >= c && row[i] < n)) a[i] = __ldcg(p + row[i]);
+      }
+      const uint32_t pc = P.row(c);
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        C v, w;
+        P.get(pc, q, v, w);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+          a[i].x = fma(-rv[i][q].x, w.x, a[i].x); a[i].x = fma(-rv[i][q].y, w.y, a[i].x);
+          a[i].y = fma(-rv[i][q].y, w.x, a[i].y); a[i].y = fma(rv[i][q].x, w.y, a[i].y);
+          a[i].x = fma(-rw[i][q].x, v.x, a[i].x); a[i].x = fma(-rw[i][q].y, v.y, a[i].x);
+          a[i].y = fma(-rw[i][q].y, v.x, a[i].y); a[i].y = fma(rw[i][q].x, v.y, a[i].y);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+        if (whole || (row[i] >= c && row[i] < n)) p[row[i]] = a[i];
+    };
     for (; u < nJ; u += nw) {
       const int cb = s0 + 16 * u, ce = min(cb + 16, last);
       C* p = A + (long long)cb * ld;
+      if (ce == cb + 16 && ce <= R0 && R0 + 32 * ROWS <= n) {
+        // no entry on or above the diagonal or past the matrix
 #pragma unroll 2
-      for (int c = cb; c < ce; ++c, p += ld) {
-        C a[ROWS];
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i)
-          a[i] = (row[i] >= c && row[i] < n) ? __ldcg(p + row[i]) : mk(R(0), R(0));
-        const uint32_t pc = P.row(c);
-#pragma unroll
-        for (int q = 0; q < NB; ++q) {
-          C v, w;
-          P.get(pc, q, v, w);
-#pragma unroll
-          for (int i = 0; i < ROWS; ++i) {
-            a[i].x = fma(-rv[i][q].x, w.x, a[i].x); a[i].x = fma(-rv[i][q].y, w.y, a[i].x);
-            a[i].y = fma(-rv[i][q].y, w.x, a[i].y); a[i].y = fma(rv[i][q].x, w.y, a[i].y);
-            a[i].x = fma(-rw[i][q].x, v.x, a[i].x); a[i].x = fma(-rw[i][q].y, v.y, a[i].x);
-            a[i].y = fma(-rw[i][q].y, v.x, a[i].y); a[i].y = fma(rw[i][q].x, v.y, a[i].y);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i)
-          if (row[i] >= c && row[i] < n) p[row[i]] = a[i];
+        for (int c = cb; c < cb + 16; ++c, p += ld) column(c, p, true);
+      } else {
+        for (int c = cb; c < ce; ++c, p += ld) column(c, p, false);
       }
     }
     u -= nJ;
@@ -333,6 +341,7 @@ __device__ __forceinline__ void ht_matrix(C* __restrict__ A, int n, int ld, doub
       for (int i = 0; i < RPT; ++i) {
         const int r = tid + kHtThreads * i;
         v[i] = zero;
+        if (r == c) x[r] = zero;   // leaves the trailing block
         if (r > c && r < n) {
           v[i] = r == c + 1 ? mk(R(1), R(0)) : cmul(col[i], sc);
           x[r] = v[i];
