@@ -59,6 +59,16 @@ __device__ __forceinline__ float es_kernel(float z, float beta) {
   return t > 0.0f ? __expf(beta * (r - 1.0f)) : 0.0f;
 }
 
+// The same with beta log2(e) folded, for any z (zero for |z| >= 1): one instruction each for
+// the root and the power, whose subnormal ranges do not matter here
+__device__ __forceinline__ float es_kernel_fast(float z, float betaLog2) {
+  const float t = fmaf(-z, z, 1.0f);
+  float r, e;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(fmaf(betaLog2, r, -betaLog2)));
+  return t > 0.0f ? e : 0.0f;
+}
+
 __device__ __forceinline__ double wrap_pi(double x) {
   // to [-pi, pi)
   const double twopi = 6.283185307179586476925286766559;

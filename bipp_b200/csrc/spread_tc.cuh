@@ -31,13 +31,10 @@ constexpr int kTcMaxChan = 8;                 // channels of one launch of the t
 constexpr int kTcAStep = kTcM * 8 * 4;
 // per-visit kernel values at every tile position (zero outside the support) and the
 // channel values, stored position-major, 16 visits per row, so that the operand builders
-// read 4 visits with one 16-byte load. Rows read by 8 different threads of a quarter warp
-// (x positions, channel values) have their 16-byte chunks permuted by the row (tab_sw):
-// conflict-free for those loads and for the writes of a thread per visit.
-constexpr int kTcVS = kTcVisits;
-__device__ __forceinline__ int tab_sw(int row, int v) {
-  return row * kTcVS + ((((v >> 2) ^ (row >> 1)) & 3) << 2) + (v & 3);
-}
+// read 4 visits with one 16-byte load. Rows are 80 bytes apart: 8 different rows of a quarter
+// warp, and the rows 4 apart that a warp's two roles write, fall in distinct banks, and every
+// address is a per-thread base plus a constant.
+constexpr int kTcVS = kTcVisits + 4;
 static_assert(kTX == 16 && kTY == 8 && kTW == 8 && kTcVisits == 16, "prep mapping assumes 16 x 8 x 8 tiles, 16 visits");
 
 // Shape of the kernel for CH channels (4 or 8), STAGES operand stages (1, or 2 so that a
@@ -70,7 +67,7 @@ struct TcShape {
   static constexpr int OffEw = OffEy + kTY * kTcVS * 4;    // float [8 w][kTcVS]
   static constexpr int OffVal = OffEw + kTW * kTcVS * 4;   // float [2 CH (channel, re/im)][kTcVS]
   static constexpr int Smem = OffVal + 2 * CH * kTcVS * 4;
-  static constexpr int BySmem = 233472 / (Smem + 512 + 1024);
+  static constexpr int BySmem = 233472 / (Smem + 256 + 1024);
   static constexpr int MinBlocks = (512 / Cols) < BySmem ? (512 / Cols) : BySmem;   // CTAs per SM
   // instruction descriptor: D f32, A/B tf32 (2) or f16 (0), both K-major, N, M = 128
   static constexpr uint32_t Idesc = (1u << 4) | ((F16 ? 0u : 2u) << 7) | ((F16 ? 0u : 2u) << 10) |
@@ -80,8 +77,8 @@ struct TcShape {
   static_assert(N % 16 == 0 && N <= 256, "MMA N for M = 128");
   static_assert(OffEx % 1024 == 0, "operand blocks 1 KB aligned");
   static_assert(STAGES == 1 || STAGES == 2, "one or two operand stages");
-  static_assert(MinBlocks >= 1 && MinBlocks * (Smem + 512 + 1024) <= 233472,
-                "shared memory (dynamic + static <= 512 B + 1 KB reserved) for MinBlocks CTAs per SM");
+  static_assert(MinBlocks >= 1 && MinBlocks * (Smem + 256 + 1024) <= 233472,
+                "shared memory (dynamic + static <= 256 B + 1 KB reserved) for MinBlocks CTAs per SM");
 };
 
 // FP16 hi + lo of two values, each pair packed in one 32-bit word (low half = first):
@@ -159,7 +156,7 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
   const uint32_t tmem = tmemSlot;
   const uint32_t tmemWarp = tmem + ((uint32_t)(warp * 32) << 16);
   const float invHalf = 2.0f / (float)g.W;
-  const int W = g.W;
+  const float betaLog2 = g.beta * 1.4426950408889634f;
   const int xm = tid % kTX, ym = tid / kTX;   // cell of accumulator row tid
   const int lane = tid & 31;
   const int myPair = (lane < 27) ? tc_range_pair(lane) : -1;
@@ -274,9 +271,9 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
       // per-visit tables from the prefetched point data (the tensor cores read only the
       // operand blocks, so the tables are rebuilt while the previous phase's MMAs run)
       {
-        float* tab = (pa < 4) ? ex : (pa < 6) ? ey : ew;
-        const bool swz = pa < 4;
         const int first = 4 * ((pa < 4) ? pa : (pa < 6) ? pa - 4 : pa - 6);   // first table row of this role
+        float* tab = ((pa < 4) ? ex : (pa < 6) ? ey : ew) + first * kTcVS + pv;
+        float* vtab = val + 2 * CPR * (pa >= 6 ? pa - 6 : 0) * kTcVS + pv;
         if (pv < nk) {
           int l = pfL;
           // periodic offset of the support start from the tile, in (-n/2, n/2]: the start
@@ -291,27 +288,25 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
           } else {
             l -= w0;
           }
+          // support index j = first + i - l of tile position first + i; outside the support
+          // |j - d| >= W / 2, where the kernel is zero
+          const float z0 = ((float)(first - l) - pfD) * invHalf;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int j = first + i - l;   // support index of tile position first + i
-            tab[swz ? tab_sw(first + i, pv) : (first + i) * kTcVS + pv] =
-                ((unsigned)j < (unsigned)W) ? es_kernel(((float)j - pfD) * invHalf, g.beta) : 0.f;
-          }
+          for (int i = 0; i < 4; ++i) tab[i * kTcVS] = es_kernel_fast(fmaf((float)i, invHalf, z0), betaLog2);
           if (pa >= 6) {
 #pragma unroll
             for (int cc = 0; cc < CPR; ++cc) {
-              const int c = CPR * (pa - 6) + cc;
-              val[tab_sw(2 * c, pv)] = pfX[cc].x * invS[cc];
-              val[tab_sw(2 * c + 1, pv)] = pfX[cc].y * invS[cc];
+              vtab[2 * cc * kTcVS] = pfX[cc].x * invS[cc];
+              vtab[(2 * cc + 1) * kTcVS] = pfX[cc].y * invS[cc];
             }
           }
         } else if (pv < kpad) {
           // padding visits of the last K-step contribute nothing (values too: 0 x stale
           // shared memory could be 0 x NaN)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) tab[swz ? tab_sw(first + i, pv) : (first + i) * kTcVS + pv] = 0.f;
+          for (int i = 0; i < 4; ++i) tab[i * kTcVS] = 0.f;
           if (pa >= 6)
-            for (int c = 2 * CPR * (pa - 6); c < 2 * CPR * (pa - 5); ++c) val[tab_sw(c, pv)] = 0.f;
+            for (int c = 0; c < 2 * CPR; ++c) vtab[c * kTcVS] = 0.f;
         }
       }
       // the operands of this stage's previous phase must have been consumed before they
@@ -328,7 +323,7 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
         uint32_t h[8], l[8];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float4 xq = *reinterpret_cast<const float4*>(ex + tab_sw(xm, 4 * q));
+          const float4 xq = *reinterpret_cast<const float4*>(ex + xm * kTcVS + 4 * q);
           const float4 yq = *reinterpret_cast<const float4*>(ey + ym * kTcVS + 4 * q);
           split_f16x2(__fmul2_rn(make_float2(xq.x, xq.y), make_float2(yq.x, yq.y)), h[2 * q], l[2 * q]);
           split_f16x2(__fmul2_rn(make_float2(xq.z, xq.w), make_float2(yq.z, yq.w)), h[2 * q + 1], l[2 * q + 1]);
@@ -342,8 +337,8 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
       for (int s = 0; s < (F16 ? 0 : steps); ++s) {
         float h[8], l[8];
         {
-          const float4 x0 = *reinterpret_cast<const float4*>(ex + tab_sw(xm, 8 * s));
-          const float4 x1 = *reinterpret_cast<const float4*>(ex + tab_sw(xm, 8 * s + 4));
+          const float4 x0 = *reinterpret_cast<const float4*>(ex + xm * kTcVS + 8 * s);
+          const float4 x1 = *reinterpret_cast<const float4*>(ex + xm * kTcVS + 8 * s + 4);
           const float4 y0 = *reinterpret_cast<const float4*>(ey + ym * kTcVS + 8 * s);
           const float4 y1 = *reinterpret_cast<const float4*>(ey + ym * kTcVS + 8 * s + 4);
           // products and splits two at a time (packed FP32x2)
@@ -385,8 +380,8 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
           const int v = kh * VPT + 8 * q;   // first visit of this 16-byte chunk
           const float4 e0 = *reinterpret_cast<const float4*>(ew + plane * kTcVS + v);
           const float4 e1 = *reinterpret_cast<const float4*>(ew + plane * kTcVS + v + 4);
-          const float4 c0 = *reinterpret_cast<const float4*>(val + tab_sw(cc, v));
-          const float4 c1 = *reinterpret_cast<const float4*>(val + tab_sw(cc, v + 4));
+          const float4 c0 = *reinterpret_cast<const float4*>(val + cc * kTcVS + v);
+          const float4 c1 = *reinterpret_cast<const float4*>(val + cc * kTcVS + v + 4);
           uint32_t h[4], l[4];
           split_f16x2(__fmul2_rn(make_float2(e0.x, e0.y), make_float2(c0.x, c0.y)), h[0], l[0]);
           split_f16x2(__fmul2_rn(make_float2(e0.z, e0.w), make_float2(c0.z, c0.w)), h[1], l[1]);
@@ -408,7 +403,7 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
             {
               const int v = s * 8 + k0;
               const float4 e4 = *reinterpret_cast<const float4*>(ew + plane * kTcVS + v);
-              const float4 c4 = *reinterpret_cast<const float4*>(val + tab_sw(cc, v));
+              const float4 c4 = *reinterpret_cast<const float4*>(val + cc * kTcVS + v);
               const float2 p0 = __fmul2_rn(make_float2(e4.x, e4.y), make_float2(c4.x, c4.y));
               const float2 p1 = __fmul2_rn(make_float2(e4.z, e4.w), make_float2(c4.z, c4.w));
               float2 h0, l0, h1, l1;
