@@ -503,6 +503,114 @@ hetrd_cluster_kernel(C* __restrict__ A, const int* __restrict__ nred, int ld, do
   }
 }
 
+// Matrices of at most 4 NK rows, one CTA of 16 NK threads each, unblocked, the whole matrix in
+// registers: thread (row i = tid / 4, part p = tid % 4) holds the elements of columns p + 4 k
+// of both triangles. Such a matrix is all latency: with panels in shared memory and the triangle
+// in L2 a column took 3.3 us (0.20 ms for 60 rows) for a few hundred multiply-adds. Here a
+// column is four barriers and no global load: the rank-2 update hands the next column and its
+// norm on, v and w are read as broadcasts.
+template <typename C, typename R, int NK>
+__global__ void __launch_bounds__(16 * NK)
+hetrd_small_kernel(C* __restrict__ A, const int* __restrict__ nred, int ld, double* __restrict__ dOut,
+                   double* __restrict__ eOut, C* __restrict__ tauOut, const int* __restrict__ order) {
+  constexpr int NMAX = 4 * NK, NW = NK / 2;
+  const int b = order[blockIdx.x], n = nred[b];
+  if (n <= 0) return;
+  __shared__ __align__(16) C vs[NMAX], ws[NMAX], col[NMAX];
+  __shared__ R sNorm[NW], sDot[2 * NW];
+  C* Ab = A + (long long)b * ld * ld;
+  double *d = dOut + (long long)b * ld, *e = eOut + (long long)b * ld;
+  C* taus = tauOut + (long long)b * ld;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, i = tid >> 2, p = tid & 3;
+  const C zero = mk(R(0), R(0));
+  C a[NK];
+  R part = 0;
+  // element (i, c) of the next column c: the diagonal to d, the rest to col and the norm of
+  // the rows below c + 1
+  auto hand_on = [&](int c, C x) {
+    if (i == c) d[c] = (double)x.x;
+    if (i > c) col[i] = x;
+    if (i > c + 1) part = cabs2(x);
+  };
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    const int j = p + 4 * k;
+    a[k] = zero;
+    if (i < n && j <= i) a[k] = Ab[i + (long long)j * ld];
+    else if (j < n && i < j) a[k] = cconj(Ab[j + (long long)i * ld]);
+    if (j == i) a[k].y = R(0);
+    if (j == 0) hand_on(0, a[k]);
+  }
+  for (int c = 0; c + 1 < n; ++c) {
+    part = warp_sum(part);
+    if (lane == 0) sNorm[warp] = part;
+    __syncthreads();
+    R xnorm2 = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) xnorm2 += sNorm[w];
+    const C alpha = col[c + 1];
+    C tau = zero, sc = zero;
+    R beta = alpha.x;
+    if (!(xnorm2 == R(0) && alpha.y == R(0))) {
+      const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2);
+      beta = (alpha.x >= R(0)) ? -nrm : nrm;
+      tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
+      const C am = mk(alpha.x - beta, alpha.y);
+      const R den = am.x * am.x + am.y * am.y;
+      sc = mk(am.x / den, -am.y / den);
+    }
+    const bool in = i > c && i < n;
+    const C v = in ? (i == c + 1 ? mk(R(1), R(0)) : cmul(col[i], sc)) : zero;
+    if (p == 0) {
+      vs[i] = v;
+      if (in) Ab[i + (long long)c * ld] = i == c + 1 ? mk(beta, R(0)) : v;
+    }
+    if (tid == 0) {
+      e[c] = (double)beta;
+      taus[c] = tau;
+    }
+    __syncthreads();
+    // y = A v over the trailing block (v is zero outside it)
+    C y = zero;
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (4 * k + 3 > c) cfma(y, a[k], vs[p + 4 * k]);
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      y.x += __shfl_xor_sync(0xffffffffu, y.x, o);
+      y.y += __shfl_xor_sync(0xffffffffu, y.y, o);
+    }
+    // w = tau y - 1/2 tau ((tau y)^H v) v
+    y = cmul(tau, y);
+    C dot = p == 0 ? cconjmul(y, v) : zero;
+    dot.x = warp_sum(dot.x);
+    dot.y = warp_sum(dot.y);
+    if (lane == 0) {
+      sDot[2 * warp] = dot.x;
+      sDot[2 * warp + 1] = dot.y;
+    }
+    __syncthreads();
+    dot = zero;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) dot = dot + mk(sDot[2 * w], sDot[2 * w + 1]);
+    const C wv = in ? y + cmul(cscale(cmul(tau, dot), R(-0.5)), v) : zero;
+    if (p == 0) ws[i] = wv;
+    __syncthreads();
+    // A -= v w^H + w v^H
+    part = 0;
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      if (4 * k + 3 > c) {
+        const int j = p + 4 * k;
+        const C vj = vs[j], wj = ws[j];
+        a[k].x -= v.x * wj.x + v.y * wj.y + wv.x * vj.x + wv.y * vj.y;
+        a[k].y -= v.y * wj.x - v.x * wj.y + wv.y * vj.x - wv.x * vj.y;
+        if (j == c + 1) hand_on(c + 1, a[k]);
+      }
+    }
+  }
+}
+
 template <typename C, typename R, int NB, int T, int RPT, int CS>
 inline void ht_launch_cs(cudaStream_t st, int grid, size_t smem, C* A, const int* nred, int ld, double* d, double* e,
                          C* tau, const int* order, int nb, int nmax) {
@@ -548,18 +656,25 @@ inline void ht_launch(cudaStream_t st, int smCount, size_t l2Bytes, C* A, const 
 
 // hetrd.hpp; at most 1024 rows, and the panel has to fit shared memory.
 // FP32: panels of 8 up to 512 rows, of 4 above (shared memory holds a row of partial sums per
-// warp). 512 threads; 256, two CTAs per SM, for matrices that leave most of 512 idle: up to 64
-// rows, and up to 256 rows when the batch has several per SM (1024 of 256 rows: 8.8 ms
-// against 11.3; 64 of them 1.9 against 1.56). FP64: 256 threads (registers), panels of 8 up to
+// warp). 512 threads; 256, two CTAs per SM, up to 256 rows when the batch has several matrices
+// per SM (1024 of 256 rows: 8.8 ms against 11.3; 64 of them 1.9 against 1.56). FP64: 256 threads (registers), panels of 8 up to
 // 512 rows, of 4 while they fit.
 template <typename C, typename R>
 bool hetrd_cluster(cudaStream_t st, int smCount, size_t l2Bytes, size_t maxSmem, C* A, const int* nred, int ld,
                           double* d, double* e, C* tau, const int* order, int nb, int nmax, int most, int grid1) {
+  // in registers up to 96 rows (16 bytes of FP64 complex: 24 elements a thread are 96 registers)
+  if (nmax <= 96) {
+    count_launch();
+    if (nmax <= 64) hetrd_small_kernel<C, R, 16><<<nb, 256, 0, st>>>(A, nred, ld, d, e, tau, order);
+    else hetrd_small_kernel<C, R, 24><<<nb, 384, 0, st>>>(A, nred, ld, d, e, tau, order);
+    B2_CHECK_LAUNCH();
+    return true;
+  }
   if constexpr (sizeof(C) == 8) {
     if (nmax > 1024) return false;
-    const auto k = nmax <= 64 || (nmax <= 256 && nb > smCount) ? ht_launch<C, R, 8, 256, 1>
-                   : nmax <= 512                               ? ht_launch<C, R, 8, 512, 1>
-                                                               : ht_launch<C, R, 4, 512, 2>;
+    const auto k = nmax <= 256 && nb > smCount ? ht_launch<C, R, 8, 256, 1>
+                   : nmax <= 512               ? ht_launch<C, R, 8, 512, 1>
+                                               : ht_launch<C, R, 4, 512, 2>;
     k(st, smCount, l2Bytes, A, nred, ld, d, e, tau, order, nb, nmax, most, grid1);
   } else {
     if (nmax > 1024 || (nmax > 512 && ht_smem<C, 4, 256>(nmax, true) > maxSmem)) return false;
