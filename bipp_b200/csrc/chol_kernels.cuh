@@ -82,6 +82,48 @@ __device__ __forceinline__ void ct_each(double (&acc)[2][4][2], F f) {
       for (int u = 0; u < 2; ++u) f(rw + 8 * i + g, cw + 8 * j + 2 * t + u, acc[i][j][u]);
 }
 
+// Factor the 64 x 64 lower block D in place and form its inverse X (both [col][row], stride
+// kCtS; on entry synchronised, X the identity, rows and columns past the matrix an identity
+// too): 64 elimination steps on [D | X], each a pivot column scaled by every thread for itself
+// and one update of the entries to its right and of X, thread = row tid % 64, columns tid / 64
+// + 4 k. Bound by the chain of pivots (root, two barriers, update); for real blocks the
+// register form below is twice as fast. False when a pivot was not positive.
+template <typename E>
+__device__ __forceinline__ bool ct_eliminate(E* __restrict__ D, E* __restrict__ X, E* __restrict__ lcol) {
+  const int r = threadIdx.x % kCtB, g = threadIdx.x / kCtB;
+  constexpr int G = kCtThreads / kCtB;
+  bool ok = true;
+  for (int j = 0; j < kCtB; ++j) {
+    double p = e_re(D[j * kCtS + j]);
+    if (!(p > 0.0)) {
+      ok = false;
+      p = 1e-300;
+    }
+    const double inv = rsqrt(p);
+    const E l = r == j ? e_real(e_zero<E>(), p * inv) : e_scale(D[j * kCtS + r], inv);
+    if (g == 0 && r >= j) lcol[r] = l;
+    // row j of X is final; column j of D is taken, and rewritten below
+    const int cx = threadIdx.x;
+    if (cx <= j) X[cx * kCtS + j] = e_scale(X[cx * kCtS + j], inv);
+    __syncthreads();
+    if (r >= j && g == 0) D[j * kCtS + r] = l;
+    if (r > j) {
+      for (int c = j + 1 + g; c <= r; c += G) {
+        E t = D[c * kCtS + r];
+        e_sub_mulc(t, l, lcol[c]);
+        D[c * kCtS + r] = t;
+      }
+      for (int c = g; c <= j; c += G) {
+        E t = X[c * kCtS + r];
+        e_sub_mul(t, l, X[c * kCtS + j]);
+        X[c * kCtS + r] = t;
+      }
+    }
+    __syncthreads();
+  }
+  return ok;
+}
+
 // One warp: factor of the 32 x 32 lower block at D (D[col][row], stride kCtS), lane = row;
 // invd[j] = 1 / L_jj. False when a pivot was not positive.
 __device__ __forceinline__ bool ct_factor32(double* __restrict__ D, double* __restrict__ invd) {
@@ -183,24 +225,27 @@ __device__ __forceinline__ bool ct_diag(double* __restrict__ D, double* __restri
 }
 
 // Factor the pivot block at k0 held in D, write L, and its inverse to W64 and LinvOut
-template <typename O>
-__device__ __forceinline__ void ct_pivot(double* D, double* X, double* invd, double* __restrict__ Gb,
-                                         double* __restrict__ Wb, O* __restrict__ Ob, int n, int k0, int ld,
-                                         int* __restrict__ status) {
+template <typename E, typename O>
+__device__ __forceinline__ void ct_pivot(E* D, E* X, E* lcol /* 64 */, E* __restrict__ Gb, E* __restrict__ Wb,
+                                         O* __restrict__ Ob, int n, int k0, int ld, int* __restrict__ status) {
   const int kb = min(kCtB, n - k0);
+  const E zero = e_zero<E>();
   for (int e = threadIdx.x; e < kCtB * kCtB; e += kCtThreads) {
     const int r = e % kCtB, c = e / kCtB;
-    if (r >= kb || c >= kb) D[c * kCtS + r] = r == c ? 1.0 : 0.0;
-    X[c * kCtS + r] = 0.0;
+    const E id = e_real(zero, r == c ? 1.0 : 0.0);
+    if (r >= kb || c >= kb) D[c * kCtS + r] = id;
+    X[c * kCtS + r] = sizeof(E) == 8 ? zero : id;   // the elimination starts from the identity
   }
   __syncthreads();
-  const bool ok = ct_diag(D, X, invd);
+  bool ok;
+  if constexpr (sizeof(E) == 8) ok = ct_diag(D, X, lcol);
+  else ok = ct_eliminate(D, X, lcol);
   for (int e = threadIdx.x; e < kCtB * kCtB; e += kCtThreads) {
     const int r = e % kCtB, c = e / kCtB;
     if (r < kb && c < kb) {
       const long long at = (k0 + r) + (long long)(k0 + c) * ld;
       if (r >= c) Gb[at] = D[c * kCtS + r];
-      Wb[at] = X[c * kCtS + r];
+      if (Wb) Wb[at] = X[c * kCtS + r];
       store_conv(Ob + at, X[c * kCtS + r]);
     }
   }
@@ -214,10 +259,30 @@ chol_diag_kernel(double* __restrict__ G, double* __restrict__ W64, O* __restrict
   const int b = blockIdx.x, n = nred[b];
   if (n <= 0) return;
   extern __shared__ __align__(16) double ct_smem[];
-  __shared__ double invd[32];
+  __shared__ double lcol[kCtB];
   const long long off = (long long)b * ld * ld;
   ct_load(ct_smem, G + off, ld, 0, 0, n, n);
-  ct_pivot<O>(ct_smem, ct_smem + kCtB * kCtS, invd, G + off, W64 + off, Linv + off, n, 0, ld, status + b);
+  ct_pivot<double, O>(ct_smem, ct_smem + kCtB * kCtS, lcol, G + off, W64 + off, Linv + off, n, 0, ld, status + b);
+}
+
+// Complex Hermitian matrices of at most 64 rows (beamformed Gram matrices): factor and inverse
+// in one launch
+constexpr size_t kCtSmemC = 2 * (size_t)kCtB * kCtS * sizeof(double2);
+template <typename O>
+__global__ void __launch_bounds__(kCtThreads, 1)
+chol_small_kernel(double2* __restrict__ G, O* __restrict__ Linv, const int* __restrict__ nred, int ld,
+                  int* __restrict__ status) {
+  const int b = blockIdx.x, n = nred[b];
+  if (n <= 0) return;
+  extern __shared__ __align__(16) double2 ct_smem_c[];
+  __shared__ double2 lcol[kCtB];
+  const long long off = (long long)b * ld * ld;
+  for (int e = threadIdx.x; e < kCtB * kCtB; e += kCtThreads) {
+    const int r = e % kCtB, c = e / kCtB;
+    if (c <= r && r < n) ct_smem_c[c * kCtS + r] = G[off + r + (long long)c * ld];
+  }
+  ct_pivot<double2, O>(ct_smem_c, ct_smem_c + kCtB * kCtS, lcol, G + off, (double2*)nullptr, Linv + off, n, 0, ld,
+                       status + b);
 }
 
 // rows below pivot block k0: A <- A X^T, and the zero block of the inverse's upper triangle
@@ -257,7 +322,7 @@ chol_trail_kernel(double* __restrict__ G, double* __restrict__ W64, O* __restric
   const int i0 = k0 + kCtB * (1 + ti), j0 = k0 + kCtB * (1 + tj);
   if (i0 >= n) return;
   extern __shared__ __align__(16) double ct_smem[];
-  __shared__ double invd[32];
+  __shared__ double lcol[kCtB];
   double *Pi = ct_smem, *Pj = ct_smem + kCtB * kCtS;
   const long long off = (long long)b * ld * ld;
   ct_load(Pi, G + off, ld, i0, k0, n, n);
@@ -276,7 +341,7 @@ chol_trail_kernel(double* __restrict__ G, double* __restrict__ W64, O* __restric
     Pi[c * kCtS + r] = (i0 + r < n && c <= r) ? G[off + (i0 + r) + (long long)(i0 + c) * ld] - v : 0.0;
   });
   __syncthreads();
-  ct_pivot<O>(Pi, Pj, invd, G + off, W64 + off, Linv + off, n, i0, ld, status + b);
+  ct_pivot<double, O>(Pi, Pj, lcol, G + off, W64 + off, Linv + off, n, i0, ld, status + b);
 }
 
 // One half of a doubling level of the inverse, diagonal blocks of size B already inverted

@@ -276,6 +276,13 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
       chol_inverse<R>(st, reinterpret_cast<double*>(G), reinterpret_cast<double*>(W64), reinterpret_cast<R*>(Linv), nred,
                       nb, L.nBeam, Nmax, L.status + L.batchOffset);
       mark(2);
+    } else if (L.nBeam <= kCtB) {
+      auto k = chol_small_kernel<C>;
+      smem_optin(k, kCtSmemC);
+      count_launch();
+      k<<<nb, kCtThreads, kCtSmemC, st>>>(G, Linv, nred, Nmax, L.status + L.batchOffset);
+      B2_CHECK_LAUNCH();
+      mark(2);
     } else {
       auto k = cholesky_kernel<double2>;
       smem_optin(k, kCholSmem);
