@@ -30,7 +30,7 @@
 
 namespace bippb200 {
 
-constexpr int kFftMaxStages = 4;
+constexpr int kFftMaxStages = 6;
 constexpr int kFftMaxValues = 16;   // complex values a thread holds in a stage
 
 // One batched 1-D pass: the transform of length n, its stages and the launch shape.
@@ -155,7 +155,43 @@ __device__ __forceinline__ void fft_dft_odd(float2 (&x)[R], const float (&cs)[R]
 }
 
 template <int R> __device__ __forceinline__ void fft_dft(float2 (&x)[R]) {
-  if constexpr (R == 2) {
+  if constexpr (R == 9 || R == 15) {
+    // R = R1 x 3 as the even composites below
+    constexpr int R1 = R / 3;
+    const float c9[9] = {1.0f, 0.766044443118978f, 0.1736481776669304f, -0.4999999999999998f, -0.9396926207859083f,
+                         -0.9396926207859084f, -0.5000000000000004f, 0.17364817766693f, 0.7660444431189778f};
+    const float s9[9] = {0.0f, 0.6427876096865393f, 0.984807753012208f, 0.8660254037844387f, 0.3420201433256689f,
+                         -0.3420201433256687f, -0.8660254037844384f, -0.9848077530122081f, -0.6427876096865396f};
+    const float c15[15] = {1.0f, 0.9135454576426009f, 0.6691306063588582f, 0.3090169943749475f,
+                           -0.1045284632676533f, -0.4999999999999998f, -0.8090169943749473f, -0.9781476007338057f,
+                           -0.9781476007338057f, -0.8090169943749476f, -0.5000000000000004f, -0.1045284632676542f,
+                           0.3090169943749472f, 0.6691306063588585f, 0.913545457642601f};
+    const float s15[15] = {0.0f, 0.4067366430758002f, 0.7431448254773941f, 0.9510565162951535f,
+                           0.9945218953682734f, 0.8660254037844387f, 0.5877852522924732f, 0.2079116908177593f,
+                           -0.2079116908177591f, -0.587785252292473f, -0.8660254037844384f, -0.9945218953682733f,
+                           -0.9510565162951536f, -0.743144825477394f, -0.4067366430758002f};
+    float2 Y[3][R1];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+      float2 y[R1];
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) y[n1] = x[3 * n1 + n2];
+      fft_dft<R1>(y);
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) {
+        const int m = n2 * k1;
+        Y[n2][k1] = m == 0 ? y[k1] : cmul(y[k1], R == 9 ? mk(c9[m % 9], s9[m % 9]) : mk(c15[m % 15], s15[m % 15]));
+      }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < R1; ++k1) {
+      float2 z[3] = {Y[0][k1], Y[1][k1], Y[2][k1]};
+      fft_dft<3>(z);
+      x[k1] = z[0];
+      x[k1 + R1] = z[1];
+      x[k1 + 2 * R1] = z[2];
+    }
+  } else if constexpr (R == 2) {
     fft_dft2(x[0], x[1]);
   } else if constexpr (R == 4) {
     fft_dft4(x[0], x[1], x[2], x[3]);
@@ -329,6 +365,26 @@ __device__ __forceinline__ void fft_stages(const FftLinePlan& pl, int t, bool ac
     fft_stages<S + 1, N, P * R, ES, BP, BPC, Rest...>(pl, t, active, lp, es, sl, tw, bits);
 }
 
+// Offset and bits of a line; false past the last one and for rows without any data, which are
+// not transformed (the column pass knows them as zero)
+template <bool LINE_FAST>
+__device__ __forceinline__ bool fft_line(const FftLines& L, long long line, long long& base, const unsigned*& bits) {
+  base = 0;
+  bits = L.xBits;
+  if (line >= L.nLines) return false;
+  const long long o = line / L.linesPerPlane;
+  const int li = (int)(line - o * L.linesPerPlane);
+  const int c = (int)(o / L.planesUsed), pj = (int)(o - (long long)c * L.planesUsed);
+  base = ((long long)c * L.slabPlanes + pj) * L.planeStride + (long long)li * L.lineStep;
+  const int layer = L.firstLayer + (pj >> 3);
+  bits = L.yBits + layer * L.yWords;
+  if constexpr (LINE_FAST) return true;
+  const int ty = li >> 3;
+  const bool any = (__ldg(bits + (ty >> 5)) >> (ty & 31)) & 1u;
+  bits = L.xBits + ((long long)layer * L.tileRows + ty) * L.xWords;
+  return any;
+}
+
 // The pass over lines of N = the product of the radices Rs (at least two stages).
 // LINE_FAST: consecutive threads take consecutive lines (the column pass: a warp reads
 // 32-byte row segments of 4 adjacent columns); otherwise consecutive threads take
@@ -345,24 +401,9 @@ fft_lines_kernel(FftLinePlan pl, FftLines L, const float2* __restrict__ tw) {
   const int tid = threadIdx.x;
   const int g = LINE_FAST ? tid % G : tid / T;
   const int t = LINE_FAST ? tid / G : tid % T;
-  const long long line = (long long)blockIdx.x * G + g;
-  bool active = line < L.nLines;
-  long long base = 0;
-  const unsigned* bits = L.xBits;
-  if (active) {
-    const long long o = line / L.linesPerPlane;
-    const int li = (int)(line - o * L.linesPerPlane);
-    const int c = (int)(o / L.planesUsed), pj = (int)(o - (long long)c * L.planesUsed);
-    base = ((long long)c * L.slabPlanes + pj) * L.planeStride + (long long)li * L.lineStep;
-    const int layer = L.firstLayer + (pj >> 3);
-    bits = L.yBits + layer * L.yWords;
-    if constexpr (!LINE_FAST) {
-      // a row without any data is not transformed: the column pass knows it as zero
-      const int ty = li >> 3;
-      active = (__ldg(bits + (ty >> 5)) >> (ty & 31)) & 1u;
-      bits = L.xBits + ((long long)layer * L.tileRows + ty) * L.xWords;
-    }
-  }
+  long long base;
+  const unsigned* bits;
+  const bool active = fft_line<LINE_FAST>(L, (long long)blockIdx.x * G + g, base, bits);
   if constexpr (!LINE_FAST) {
     if (!__syncthreads_or(active)) return;
   }
@@ -374,33 +415,35 @@ fft_lines_kernel(FftLinePlan pl, FftLines L, const float2* __restrict__ tw) {
 
 using FftLinesKernel = void (*)(FftLinePlan, FftLines, const float2*);
 
-// Compiled radix sequences: the power of two 2^a (a = 4..10) as 4 x 4, 8 x 4, 16 x 4,
-// 16 x 8, 16 x 16, 16 x 8 x 4, 16 x 16 x 4, or one odd radix 3, 5 or 7 followed by 16,
-// 8 x 4, 16 x 4, 16 x 8, 16 x 16, 16 x 8 x 4, 16 x 16 x 4. Null when the sequence has no compiled kernel (the caller
-// then transforms with cuFFT).
-inline FftLinesKernel fft_lines_kernel_for(const int* radix, int ns, bool lineFast) {
-  struct Entry {
-    int r[4];
-    FftLinesKernel rows, cols;
-  };
-#define B2_FFT_ENTRY(...) {{__VA_ARGS__}, fft_lines_kernel<false, __VA_ARGS__>, fft_lines_kernel<true, __VA_ARGS__>}
-#define B2_FFT_ODD(f)                                                                                          \
-  B2_FFT_ENTRY(f, 16), B2_FFT_ENTRY(f, 8, 4), B2_FFT_ENTRY(f, 16, 4), B2_FFT_ENTRY(f, 16, 8),                 \
-      B2_FFT_ENTRY(f, 16, 16), B2_FFT_ENTRY(f, 16, 8, 4), B2_FFT_ENTRY(f, 16, 16, 4)
-  static const Entry table[] = {B2_FFT_ENTRY(4, 4),  B2_FFT_ENTRY(8, 4),      B2_FFT_ENTRY(16, 4),
-                                B2_FFT_ENTRY(16, 8), B2_FFT_ENTRY(16, 16),    B2_FFT_ENTRY(16, 8, 4),
-                                B2_FFT_ENTRY(16, 16, 4),
-                                B2_FFT_ODD(3),       B2_FFT_ODD(5),           B2_FFT_ODD(7)};
-#undef B2_FFT_ODD
-#undef B2_FFT_ENTRY
-  for (const Entry& e : table) {
+// Compiled radix sequences. A power of two 2^a (a = 4..10) as 4 x 4, 8 x 4, 16 x 4, 16 x 8,
+// 16 x 16, 16 x 8 x 4, 16 x 16 x 4, alone (a lone 16 for the odd lines) or after one odd
+// radix 3, 5 or 7 (fft_seq_1.cu); after two or more odd factors, 15 = 3 x 5 and 9 = 3 x 3 taken
+// together, up to 3600 cells (images up to 2057 px; fft_seq_2.cu .. 5): two thirds of the
+// fine-grid sizes of arbitrary image widths, which cuFFT's full 2-D transform took before with
+// 2.4 times the bytes, empty tiles cleared and a plan made on the first call. (A kernel with
+// the radices at run time, 64 registers and spills, took 1.6 times cuFFT's time.) Null when
+// the sequence has no compiled kernel (the caller then transforms with cuFFT).
+struct FftSeq {
+  int r[kFftMaxStages];
+  FftLinesKernel rows, cols;
+};
+#define B2_FFT_SEQ(...) {{__VA_ARGS__}, fft_lines_kernel<false, __VA_ARGS__>, fft_lines_kernel<true, __VA_ARGS__>}
+// the entry of `table` for these radices, or null
+template <size_t K>
+inline FftLinesKernel fft_find(const FftSeq (&table)[K], const int* radix, int ns, bool lineFast) {
+  for (const FftSeq& e : table) {
     int m = 0;
-    while (m < 4 && e.r[m] != 0) ++m;
+    while (m < kFftMaxStages && e.r[m] != 0) ++m;
     bool same = m == ns;
     for (int s = 0; same && s < ns; ++s) same = e.r[s] == radix[s];
     if (same) return lineFast ? e.cols : e.rows;
   }
   return nullptr;
 }
+FftLinesKernel fft_seq_1(const int* radix, int ns, bool lineFast);
+FftLinesKernel fft_seq_2(const int* radix, int ns, bool lineFast);
+FftLinesKernel fft_seq_3(const int* radix, int ns, bool lineFast);
+FftLinesKernel fft_seq_4(const int* radix, int ns, bool lineFast);
+FftLinesKernel fft_seq_5(const int* radix, int ns, bool lineFast);
 
 }  // namespace bippb200

@@ -193,8 +193,7 @@ NufftCore::~NufftCore() {
 }
 
 // Plan of one pass of the pruned FFT over lines of n values keeping nout outputs, with its
-// compiled kernel (false when n has none: the caller uses cuFFT). Radices: the odd factor
-// first, then the power of two 2^a (a >= 4, as the grid sizes are multiples of 16) as 16s
+// compiled kernel (false when n has none: the caller uses cuFFT). Radices: the odd factors first, then the power of two 2^a (a >= 4, as the grid sizes are multiples of 16) as 16s
 // with a remainder of 8 x 4 (a = 5 left), 8, 4 or 2; a lone radix-16 stage becomes 4 x 4,
 // so the first stage's reads precede a barrier that the last stage's in-place writes
 // follow. Threads per line: the fewest warps with which no thread holds more than
@@ -207,12 +206,25 @@ static bool make_fft_plan(int n, int nout, bool columnPass, FftLinePlan& pl, Fft
   pl.n = n;
   pl.nout = nout;
   std::vector<int> r;
-  int m = n;
-  for (int f : {7, 5, 3})
+  int m = n, odd[8] = {};
+  for (int f : {3, 5, 7})
     while (m % f == 0) {
-      r.push_back(f);
+      ++odd[f];
       m /= f;
     }
+  const bool single = odd[3] + odd[5] + odd[7] <= 1;
+  // odd factors, larger composites first: 15 = 3 x 5, 9 = 3 x 3
+  while (odd[3] && odd[5] && !single) {
+    r.push_back(15);
+    --odd[3];
+    --odd[5];
+  }
+  while (odd[3] >= 2) {
+    r.push_back(9);
+    odd[3] -= 2;
+  }
+  for (int f : {7, 5, 3})
+    for (; odd[f]; --odd[f]) r.push_back(f);
   int a = 0;
   while (m % 2 == 0) {
     ++a;
@@ -250,7 +262,8 @@ static bool make_fft_plan(int n, int nout, bool columnPass, FftLinePlan& pl, Fft
   while (G > 1 && (size_t)G * pl.lineStride * sizeof(float2) > (size_t)227 * 1024) --G;
   if ((size_t)G * pl.lineStride * sizeof(float2) > (size_t)227 * 1024) return false;
   pl.lines = G;
-  kernel = fft_lines_kernel_for(pl.radix, pl.ns, columnPass);
+  for (auto f : {fft_seq_1, fft_seq_2, fft_seq_3, fft_seq_4, fft_seq_5})
+    if (!kernel) kernel = f(pl.radix, pl.ns, columnPass);
   return kernel != nullptr;
 }
 

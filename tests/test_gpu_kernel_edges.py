@@ -164,3 +164,20 @@ def test_eigh_gram_sizes(ctx, n, b, precision):
         assert np.abs(d[k] - ref).max() <= tol * scale * max(1.0, math.sqrt(cond)), k
         vk = v[k].astype(np.complex128)
         assert np.linalg.norm(g @ (vk * d[k]) @ vk.conj().T @ g - s64) <= tol * n * cond * scale, k
+
+
+@pytest.mark.parametrize("px", [11, 26, 41, 63, 114, 200, 274, 343, 514, 900, 1200])
+def test_fft_lines_with_several_odd_factors(ctx, px):
+    """Image widths whose fine grids have more than one odd factor (among them 48, 144, 240,
+    432, 1575 -> 1600, 2100 -> 2160 cells) or are small, along either axis of the image."""
+    rng = np.random.default_rng(24)
+    na = 20
+    a, b = np.meshgrid(np.arange(na), np.arange(px), indexing="ij")
+    for transposed in (False, True):
+        l = (b.reshape(-1) - px / 2 + 0.5) * (0.2 / px)
+        m = (a.reshape(-1) - na / 2 + 0.25) * (0.03 / na)
+        if transposed:
+            l, m = (l.reshape(na, px).T.reshape(-1), m.reshape(na, px).T.reshape(-1))
+        lmn = np.stack([l, m, np.sqrt(1 - l * l - m * m)], 1).astype(np.float32)
+        uvw, c = _points(rng, 500, 400.0, 20.0, 1)
+        _check_nufft(ctx, lmn, uvw, c, 1e-6, 2e-5)
