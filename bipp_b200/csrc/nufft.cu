@@ -830,7 +830,7 @@ static void nufft_transform(bipp_nufft_s* p) {
     }
     B2_CHECK_LAUNCH();
     const double* ud = u64.get<double>();
-    const dim3 blocks = direct_sum_grid((long long)p->nPixel, (long long)n, ctx->smCount, tuned("direct.ctas_per_sm"));
+    const dim3 blocks = direct_sum_grid((long long)p->nPixel, (long long)n, ctx->smCount, tuned("direct.ctas_per_sm"), 1, 1024);
     for (size_t im = 0; im < p->nImages; ++im) {
       count_launch();
       f2d_kernel<<<256, 256, 0, ctx->stream>>>(reinterpret_cast<const float*>(p->values.get<float2>() + im * ld), 2 * n,
@@ -1093,9 +1093,14 @@ BippError bipp_nuft_sum_s(bipp_ctx_t ctx, float alpha, size_t nIn, const void* i
     h2d(ctx, dX.get<float>() + nOut, y, nOut * sizeof(float));
     h2d(ctx, dX.get<float>() + 2 * nOut, z, nOut * sizeof(float));
     h2d(ctx, dO.get(), out, nOut * sizeof(float));
-    const dim3 blocks = direct_sum_grid((long long)nOut, (long long)nIn, ctx->smCount, tuned("direct.ctas_per_sm"));
+    // two outputs per thread where they and the slices still make three CTAs per SM
+    const int perSm = tuned("direct.ctas_per_sm");
+    dim3 blocks = direct_sum_grid((long long)nOut, (long long)nIn, ctx->smCount, perSm, 2, 4096);
+    const bool two = (long long)blocks.x * blocks.y >= 5ll * ctx->smCount / 2;
+    if (!two) blocks = direct_sum_grid((long long)nOut, (long long)nIn, ctx->smCount, perSm, 1, 4096);
     count_launch();
-    direct_sum_kernel<float, float2, float, 1><<<blocks, kDirectThreads, 0, ctx->stream>>>(
+    auto k = two ? direct_sum_kernel<float, float2, float, 1, 2> : direct_sum_kernel<float, float2, float, 1, 1>;
+    k<<<blocks, kDirectThreads, 0, ctx->stream>>>(
         (double)alpha, (long long)nIn, dIn.get<float2>(), (long long)nIn, dU.get<float>(), dU.get<float>() + nIn,
         dU.get<float>() + 2 * nIn, (long long)nOut, dX.get<float>(), dX.get<float>() + nOut, dX.get<float>() + 2 * nOut,
         dO.get<float>(), (long long)nOut, 1, 0);
@@ -1120,7 +1125,7 @@ BippError bipp_nuft_sum_d(bipp_ctx_t ctx, double alpha, size_t nIn, const void* 
     h2d(ctx, dX.get<double>() + nOut, y, nOut * sizeof(double));
     h2d(ctx, dX.get<double>() + 2 * nOut, z, nOut * sizeof(double));
     h2d(ctx, dO.get(), out, nOut * sizeof(double));
-    const dim3 blocks = direct_sum_grid((long long)nOut, (long long)nIn, ctx->smCount, tuned("direct.ctas_per_sm"));
+    const dim3 blocks = direct_sum_grid((long long)nOut, (long long)nIn, ctx->smCount, tuned("direct.ctas_per_sm"), 1, 1024);
     count_launch();
     direct_sum_kernel<double, double2, double, 1><<<blocks, kDirectThreads, 0, ctx->stream>>>(
         alpha, (long long)nIn, dIn.get<double2>(), (long long)nIn, dU.get<double>(), dU.get<double>() + nIn,
@@ -1140,7 +1145,7 @@ BippError bipp_nuft_sum_multi_device(bipp_ctx_t ctx, double alpha, size_t nIn, s
     require(ctx && values && u && v && w && x && y && z && out, "null pointer", BIPP_INVALID_POINTER_ERROR);
     require(nch >= 1 && ldIn >= nIn && ldOut >= nOut, "invalid sizes");
     if (!nOut) return;
-    const dim3 blocks = direct_sum_grid((long long)nOut, (long long)nIn, ctx->smCount, tuned("direct.ctas_per_sm"));
+    const dim3 blocks = direct_sum_grid((long long)nOut, (long long)nIn, ctx->smCount, tuned("direct.ctas_per_sm"), 1, 1024);
     for (size_t c0 = 0; c0 < nch; c0 += 4) {
       const int n = (int)std::min<size_t>(4, nch - c0);
       count_launch();

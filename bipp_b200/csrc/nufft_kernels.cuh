@@ -767,15 +767,16 @@ static __global__ void decon_kernel(NufftGeom g, const double* __restrict__ nTil
 //
 // Bound by the conversion/transcendental pipe: a first form spent 6 FP64 conversions and
 // roundings per pair there beside the two transcendentals (2.41 ms for 65,536 inputs x
-// 16,384 outputs in FP32). Here rounding is by adding 1.5 2^52, the reduced phase leaves
-// FP64 as the low word of r + 1.5 2^20 (its fraction in units of 2^-32 turns, finer than
-// FP32), FP32 sine and cosine enter the FP64 sum by rewriting their bits, and the values
-// are converted once per chunk. Inputs or pixels outside the range in which these hold
-// (non-finite, or phases that could reach 2^50 turns) take the plain form.
+// 16,384 outputs in FP32). Here the fraction of the phase leaves FP64 as the low word of
+// ph + 1.5 2^20 (in units of 2^-32 turns, finer than FP32), FP32 sine and cosine enter the
+// FP64 sum by rewriting their bits, and the values are converted once per chunk; OUT outputs
+// per thread share the loads of an input. Phases of up to 2^19 turns need no rounding first
+// (the sum's integer bits do not reach the low word); beyond them, and for non-finite inputs or
+// pixels, the plain form.
 // ---------------------------------------------------------------------------------------
 constexpr int kDirectThreads = 256;
 constexpr int kDirectChunk = 256;
-constexpr double kDirectMaxInput = 1e12, kDirectMaxPixel = 300.0;
+constexpr double kDirectMaxInput = 131072.0, kDirectMaxPixel = 1.25;   // 3 of their products stay below 2^19
 
 // the value of a finite FP32 number as FP64 by its bits (zero and FP32 subnormals come out
 // below 2^-126 in magnitude)
@@ -784,7 +785,7 @@ __device__ __forceinline__ double f2d_bits(float f) {
   return __hiloint2double(((b >> 3) & (int)0x8fffffff) + 0x38000000, b << 29);
 }
 
-template <typename TC, typename C, typename TO, int CH>
+template <typename TC, typename C, typename TO, int CH, int OUT = 1>
 __global__ void __launch_bounds__(kDirectThreads)
 direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long long ldIn,
                   const TC* __restrict__ u, const TC* __restrict__ v, const TC* __restrict__ w, long long nOut,
@@ -796,11 +797,18 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const bool active = p < nOut;
   constexpr double inv2pi = 0.15915494309189533576888376337251;
-  const double xp = active ? (double)x[p] * alpha * inv2pi : 0.0;
-  const double yp = active ? (double)y[p] * alpha * inv2pi : 0.0;
-  const double zp = active ? (double)z[p] * alpha * inv2pi : 0.0;
-  const bool pixelInRange = fabs(xp) < kDirectMaxPixel && fabs(yp) < kDirectMaxPixel && fabs(zp) < kDirectMaxPixel;
-  double acc[CH];
+  const long long p0 = blockIdx.x * (long long)(blockDim.x * OUT) + threadIdx.x;
+  double xp[OUT], yp[OUT], zp[OUT], acc[OUT][CH];
+  bool pixelInRange = true;
+#pragma unroll
+  for (int o = 0; o < OUT; ++o) {
+    const long long p = p0 + o * (long long)blockDim.x;
+    const bool there = p < nOut;
+    xp[o] = there ? (double)x[p] * alpha * inv2pi : 0.0;
+    yp[o] = there ? (double)y[p] * alpha * inv2pi : 0.0;
+    zp[o] = there ? (double)z[p] * alpha * inv2pi : 0.0;
+    pixelInRange = pixelInRange && fabs(xp[o]) < kDirectMaxPixel && fabs(yp[o]) < kDirectMaxPixel &&
+                   fabs(zp[o]) < kDirectMaxPixel;
 #pragma unroll
   for (int c = 0; c < CH; ++c) acc[c] = 0.0;
   // blockIdx.y takes one slice of the inputs (whole chunks); slices add their partial
@@ -839,33 +847,43 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
 #pragma unroll 4
       for (int i = 0; i < nk; ++i) {
         const double2 uv = suv[i];
-        const double ph = fma(xp, uv.x, fma(yp, uv.y, zp * sw[i]));
-        constexpr double m52 = 6755399441055744.0;   // 1.5 2^52
-        const double r = ph - __dadd_rn(__dadd_rn(ph, m52), -m52);
-        const int turns = __double2loint(r + 1572864.0);   // 1.5 2^20: r in units of 2^-32
-        float sf, cf;
-        __sincosf((float)turns * 1.4629180792671596e-9f, &sf, &cf);   // 2 pi 2^-32
-        add(i, f2d_bits(sf), f2d_bits(cf));
+        const double wi = sw[i];
+#pragma unroll
+        for (int o = 0; o < OUT; ++o) {
+          const double ph = fma(xp[o], uv.x, fma(yp[o], uv.y, zp[o] * wi));
+          const int turns = __double2loint(ph + 1572864.0);   // 1.5 2^20: fraction in units of 2^-32
+          float sf, cf;
+          __sincosf((float)turns * 1.4629180792671596e-9f, &sf, &cf);   // 2 pi 2^-32
+          add(o, i, f2d_bits(sf), f2d_bits(cf));
+        }
       }
     } else {
       for (int i = 0; i < nk; ++i) {
         const double2 uv = suv[i];
-        double ph = fma(xp, uv.x, fma(yp, uv.y, zp * sw[i]));
-        ph -= rint(ph);
-        double s, cs;
-        if (fp64Trig) {
-          sincospi(2.0 * ph, &s, &cs);
-        } else {
-          float sf, cf;
-          __sincosf((float)(ph * 6.283185307179586476925286766559), &sf, &cf);
-          s = sf;
-          cs = cf;
+        const double wi = sw[i];
+#pragma unroll
+        for (int o = 0; o < OUT; ++o) {
+          double ph = fma(xp[o], uv.x, fma(yp[o], uv.y, zp[o] * wi));
+          ph -= rint(ph);
+          double s, cs;
+          if (fp64Trig) {
+            sincospi(2.0 * ph, &s, &cs);
+          } else {
+            float sf, cf;
+            __sincosf((float)(ph * 6.283185307179586476925286766559), &sf, &cf);
+            s = sf;
+            cs = cf;
+          }
+          add(o, i, s, cs);
         }
         add(i, s, cs);
       }
     }
   }
-  if (active) {
+#pragma unroll
+  for (int o = 0; o < OUT; ++o) {
+    const long long p = p0 + o * (long long)blockDim.x;
+    if (p >= nOut) continue;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if (c < nch) {
@@ -878,16 +896,19 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
   }
 }
 
-// Grid of direct_sum_kernel: one thread per output; when the outputs fill fewer than
-// ctasPerSm CTAs per SM, the inputs are split over blockIdx.y (slices of at least 4096
-// inputs) so that few pixels over many baselines still fill the GPU.
-inline dim3 direct_sum_grid(long long nOut, long long nIn, int smCount, int ctasPerSm) {
-  const long long bx = (nOut + kDirectThreads - 1) / kDirectThreads;
+// Grid of direct_sum_kernel: one thread per `outs` outputs; when the outputs fill fewer than
+// ctasPerSm CTAs per SM, the inputs are split over blockIdx.y (slices of at least minSlice
+// inputs: 4096 where the slices' sums meet in FP32, 1024 in FP64) so that few pixels over many
+// baselines still fill the GPU. Of the slice counts down
+// to three quarters of that the one whose fullest SM has the least to do is taken (32 x 16
+// CTAs give some SMs 4 slices of 1/16, 32 x 13 none more than 3 of 1/13).
+inline dim3 direct_sum_grid(long long nOut, long long nIn, int smCount, int ctasPerSm, int outs, int minSlice) {
+  const long long bx = (nOut + kDirectThreads * outs - 1) / (kDirectThreads * outs);
   const long long target = (long long)ctasPerSm * (smCount > 0 ? smCount : 148);
   long long by = 1;
   if (bx < target) {
     by = (target + bx - 1) / bx;
-    const long long maxSlices = nIn / 4096 > 1 ? nIn / 4096 : 1;
+    const long long maxSlices = nIn / minSlice > 1 ? nIn / minSlice : 1;
     by = by < maxSlices ? by : maxSlices;
     by = by < 65535 ? by : 65535;
   }
@@ -923,3 +944,6 @@ static __global__ void value_scale_kernel(const int* __restrict__ total, const f
 }
 
 }  // namespace bippb200
+    const long long sms = smCount > 0 ? smCount : 148, most = by;
+    for (long long t = most - 1; 4 * t >= 3 * most && t >= 1; --t)
+      if ((bx * t + sms - 1) / sms * by < (bx * by + sms - 1) / sms * t) by = t;
