@@ -193,7 +193,8 @@ NufftCore::~NufftCore() {
 }
 
 // Plan of one pass of the pruned FFT over lines of n values keeping nout outputs, with its
-// compiled kernel (false when n has none: the caller uses cuFFT). Radices: the odd factors first, then the power of two 2^a (a >= 4, as the grid sizes are multiples of 16) as 16s
+// compiled kernel (false when n has none: the caller uses cuFFT). Radices: the odd factors
+// first, then the power of two 2^a (a >= 4, as the grid sizes are multiples of 16) as 16s
 // with a remainder of 8 x 4 (a = 5 left), 8, 4 or 2; a lone radix-16 stage becomes 4 x 4,
 // so the first stage's reads precede a barrier that the last stage's in-place writes
 // follow. Threads per line: the fewest warps with which no thread holds more than
@@ -453,17 +454,7 @@ void NufftCore::end_count(long long nPoints) {
   const long long n = nkeys_;
   offsets_.ensure(ctx_, (n + 1) * sizeof(int));
   cursor_.ensure(ctx_, (n + 1) * sizeof(int));
-  const long long per = (long long)kScanThreads * kScanItems;
-  const int nb = (int)((n + per - 1) / per);
-  blockSums_.ensure(ctx_, (nb + 1) * sizeof(int));
-  count_launch();
-  scan_partial_kernel<<<nb, kScanThreads, 0, ctx_->stream>>>(counts_.get<int>(), offsets_.get<int>(), n,
-                                                             blockSums_.get<int>());
-  count_launch();
-  scan_blocksums_kernel<<<1, 1024, 0, ctx_->stream>>>(blockSums_.get<int>(), nb, offsets_.get<int>() + n);
-  count_launch();
-  scan_add_kernel<<<nb, 1024, 0, ctx_->stream>>>(offsets_.get<int>(), n, blockSums_.get<int>(), cursor_.get<int>());
-  B2_CHECK_LAUNCH();
+  scan(counts_.get<int>(), offsets_.get<int>(), cursor_.get<int>(), n);
   valStride_ = std::max<long long>(nPoints, 1);
   rec_.ensure(ctx_, valStride_ * sizeof(PtRec));
   vals_.ensure(ctx_, (size_t)nch_ * valStride_ * sizeof(float2));
@@ -524,17 +515,23 @@ static bool use_tensor_core_spread(int nch, double eps) {
 }
 
 
-// exclusive scan of n ints on the stream; out[n] = total
-void NufftCore::exclusive_scan(const int* in, int* out, long long n) {
+// exclusive scan of n ints on the stream into out (and out2, if given); out[n] = total
+void NufftCore::scan(const int* in, int* out, int* out2, long long n) {
+  if (n <= kScanShort) {
+    count_launch();
+    scan_short_kernel<<<1, kScanThreads, 0, ctx_->stream>>>(in, n, out, out2, out + n);
+    B2_CHECK_LAUNCH();
+    return;
+  }
   const long long per = (long long)kScanThreads * kScanItems;
   const int nb = (int)((n + per - 1) / per);
-  itemSums_.ensure(ctx_, (nb + 1) * sizeof(int));
+  blockSums_.ensure(ctx_, (nb + 1) * sizeof(int));
   count_launch();
-  scan_partial_kernel<<<nb, kScanThreads, 0, ctx_->stream>>>(in, out, n, itemSums_.get<int>());
+  scan_partial_kernel<<<nb, kScanThreads, 0, ctx_->stream>>>(in, out, n, blockSums_.get<int>());
   count_launch();
-  scan_blocksums_kernel<<<1, 1024, 0, ctx_->stream>>>(itemSums_.get<int>(), nb, out + n);
+  scan_blocksums_kernel<<<1, 1024, 0, ctx_->stream>>>(blockSums_.get<int>(), nb, out + n);
   count_launch();
-  scan_add_kernel<<<nb, 1024, 0, ctx_->stream>>>(out, n, itemSums_.get<int>(), nullptr);
+  scan_add_kernel<<<nb, 1024, 0, ctx_->stream>>>(out, n, blockSums_.get<int>(), out2);
   B2_CHECK_LAUNCH();
 }
 
@@ -594,31 +591,41 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
                                                                                         yWords, xBits, xBits + xAll);
     B2_CHECK_LAUNCH();
   }
-  exclusive_scan(parts_.get<int>(), itemOff_.get<int>(), ntiles);
+  scan(parts_.get<int>(), itemOff_.get<int>(), nullptr, ntiles);
   if (tc) {
-    exclusive_scan(clearFlag_.get<int>(), clearOff_.get<int>(), ntiles);
+    scan(clearFlag_.get<int>(), clearOff_.get<int>(), nullptr, ntiles);
     count_launch();
     clear_list_kernel<<<tb, 256, 0, ctx_->stream>>>(ntiles, clearFlag_.get<int>(), clearOff_.get<int>(),
                                                     clearList_.get<int>());
     B2_CHECK_LAUNCH();
   }
   const int tilesPerPlaneSet = g_.ntx * g_.nty;
-  std::vector<int> slabBegin(nslab + 1, 0), clearBegin(nslab + 1, 0);
-  for (int sl = 0; sl <= nslab; ++sl) {
-    const int t = std::min(ntiles, sl * slabTiles * tilesPerPlaneSet);
-    d2h(ctx_, &slabBegin[sl], itemOff_.get<int>() + t, sizeof(int));
-    if (tc) d2h(ctx_, &clearBegin[sl], clearOff_.get<int>() + t, sizeof(int));
-  }
+  // one copy of everything the launches below depend on
+  std::vector<int> known(2 * (nslab + 1) + 2);
+  slabCounts_.ensure(ctx_, known.size() * sizeof(int));
+  count_launch();
+  slab_counts_kernel<<<1, 64, 0, ctx_->stream>>>(nslab, slabTiles * tilesPerPlaneSet, ntiles, itemOff_.get<int>(),
+                                                 tc ? clearOff_.get<int>() : nullptr, offsets_.get<int>() + nkeys_,
+                                                 splitCount_.get<int>(), slabCounts_.get<int>());
+  B2_CHECK_LAUNCH();
+  d2h(ctx_, known.data(), slabCounts_.get(), known.size() * sizeof(int));
   sync(ctx_);
+  const int *slabBegin = known.data(), *clearBegin = known.data() + nslab + 1;
   const int nItemsAll = slabBegin[nslab];
+  lastPoints = known[2 * (nslab + 1)];
+  lastSplitTiles = known[2 * (nslab + 1) + 1];
+  lastSlabs = nslab;
+  lastItems = nItemsAll;
+  lastGridBytes = (long long)g_.ntw * kTW * (long long)planeBytes * nch_;
   items_.ensure(ctx_, std::max<size_t>(1, (size_t)nItemsAll) * sizeof(SpreadItem));
   count_launch();
   item_fill_kernel<<<tb, 256, 0, ctx_->stream>>>(ntiles, load_.get<int>(), parts_.get<int>(), itemOff_.get<int>(),
                                                  items_.get<SpreadItem>());
   B2_CHECK_LAUNCH();
   // load-ordered dynamic schedule (tunable): the items of every slab sorted heaviest
-  // first, handed out by a work counter per slab launch
-  const bool dynamic = tc && tuned("spread.schedule") == 1 && nItemsAll > 0;
+  // first, handed out by a work counter per slab launch; a list of a few items per resident
+  // CTA (8 per SM) is not worth the sort's seven launches
+  const bool dynamic = tc && tuned("spread.schedule") == 1 && nItemsAll > 32 * ctx_->smCount;
   if (dynamic) {
     const int tilesPerSlab = slabTiles * g_.ntx * g_.nty;
     itemKeys_.ensure(ctx_, 2 * (size_t)nItemsAll * sizeof(unsigned));
@@ -643,17 +650,6 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
     const size_t counters = (size_t)std::max(1, nslab) * ((nch_ + kTcMaxChan - 1) / kTcMaxChan);
     workCounters_.ensure(ctx_, counters * sizeof(int));
     B2_CUDA(cudaMemsetAsync(workCounters_.get(), 0, counters * sizeof(int), ctx_->stream));
-  }
-  {
-    int total = 0, split = 0;
-    d2h(ctx_, &total, offsets_.get<int>() + nkeys_, sizeof(int));
-    d2h(ctx_, &split, splitCount_.get<int>(), sizeof(int));
-    sync(ctx_);
-    lastPoints = total;
-    lastSplitTiles = split;
-    lastSlabs = nslab;
-    lastItems = nItemsAll;
-    lastGridBytes = (long long)g_.ntw * kTW * (long long)planeBytes * nch_;
   }
   // spreader operands (tunable): 0 tf32 split with A in shared memory, 1 with A in tensor
   // memory, 2 FP16 hi/lo (values scaled per channel by their largest magnitude)

@@ -79,7 +79,7 @@ private:
   long long nkeys_ = 0, valStride_ = 0;
   DevBuf nTilde_, decon_, dl_, dm_, counts_, offsets_, cursor_, blockSums_, rec_, vals_, grid_, acc_;
   DevBuf itemKeys_, itemsAlt_, sortTmp_, workCounters_;
-  DevBuf qz_, qw_, zeroAcc_, load_, items_, errFlag_, splitCount_, parts_, itemOff_, itemSums_, clearFlag_, clearOff_, clearList_;
+  DevBuf qz_, qw_, zeroAcc_, load_, items_, errFlag_, splitCount_, parts_, itemOff_, slabCounts_, clearFlag_, clearOff_, clearList_;
   DevBuf valScale_;   // per-channel value scale of the FP16 spreader operands
   // batched 2-D cuFFT plans by batch size (channels x slab planes), for grid sizes without
   // a compiled pruned-FFT plan or nufft.fft = 0
@@ -97,7 +97,7 @@ private:
   // tile layer is firstLayer: pruned (by the tiles' bits; cell (a, b) of a plane then holds
   // pixel (a, b)'s output) or in full by cuFFT
   void inverse_fft(int slabPlanes, int planesUsed, int firstLayer, float2* slab, bool pruned);
-  void exclusive_scan(const int* in, int* out, long long n);
+  void scan(const int* in, int* out, int* out2, long long n);
   void setup_grid(bipp_ctx_s* ctx, const Lattice& lat, double nmin, double nmax, double eps, int nch, bool corr);
   void setup_decon();
 

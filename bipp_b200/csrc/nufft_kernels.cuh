@@ -378,6 +378,71 @@ static __global__ void scan_partial_kernel(const int* __restrict__ in, int* __re
   }
 }
 
+// exclusive scan of a short array by one CTA (out and, if given, out2; *total the sum), in
+// chunks of kScanThreads * kScanItems: three launches become one where they outweigh the work
+constexpr long long kScanShort = 8ll * kScanThreads * kScanItems;
+static __global__ void __launch_bounds__(kScanThreads) scan_short_kernel(const int* __restrict__ in, long long n,
+                                                                         int* __restrict__ out, int* __restrict__ out2,
+                                                                         int* __restrict__ total) {
+  __shared__ int warpSums[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int carry = 0;
+  for (long long base = 0; base < n; base += kScanThreads * kScanItems) {
+    int vals[kScanItems], tsum = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      const long long idx = base + (long long)threadIdx.x * kScanItems + i;
+      vals[i] = (idx < n) ? in[idx] : 0;
+      tsum += vals[i];
+    }
+    int incl = tsum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    __syncthreads();
+    if (lane == 31) warpSums[wid] = incl;
+    __syncthreads();
+    const int ws = warpSums[lane];
+    int wi = ws;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) wi += t;
+    }
+    int run = carry + __shfl_sync(0xffffffffu, wi - ws, wid) + incl - tsum;
+    carry += __shfl_sync(0xffffffffu, wi, 31);
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      const long long idx = base + (long long)threadIdx.x * kScanItems + i;
+      if (idx < n) {
+        out[idx] = run;
+        if (out2) out2[idx] = run;
+      }
+      run += vals[i];
+    }
+  }
+  if (threadIdx.x == 0) *total = carry;
+}
+
+// what the host needs to know before it launches the slabs: for sl = 0 .. nslab the first item
+// and (clearOff given) the first tile to clear of the slab, then the points and the split tiles
+static __global__ void slab_counts_kernel(int nslab, int tilesPerSlab, int ntiles, const int* __restrict__ itemOff,
+                                          const int* __restrict__ clearOff, const int* __restrict__ points,
+                                          const int* __restrict__ split, int* __restrict__ out) {
+  for (int sl = threadIdx.x; sl <= nslab; sl += blockDim.x) {
+    const long long at = (long long)sl * tilesPerSlab;
+    const int t = at < ntiles ? (int)at : ntiles;
+    out[sl] = itemOff[t];
+    out[nslab + 1 + sl] = clearOff ? clearOff[t] : 0;
+  }
+  if (threadIdx.x == 0) {
+    out[2 * (nslab + 1)] = *points;
+    out[2 * (nslab + 1) + 1] = *split;
+  }
+}
+
 static __global__ void scan_blocksums_kernel(int* __restrict__ blockSums, int nBlocks, int* __restrict__ total) {
   // single block, sequential chunks
   __shared__ int carry;
@@ -794,8 +859,6 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
   __shared__ double2 suv[kDirectChunk];
   __shared__ double sw[kDirectChunk];
   __shared__ double2 sval[CH][kDirectChunk];
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const bool active = p < nOut;
   constexpr double inv2pi = 0.15915494309189533576888376337251;
   const long long p0 = blockIdx.x * (long long)(blockDim.x * OUT) + threadIdx.x;
   double xp[OUT], yp[OUT], zp[OUT], acc[OUT][CH];
@@ -810,18 +873,20 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
     pixelInRange = pixelInRange && fabs(xp[o]) < kDirectMaxPixel && fabs(yp[o]) < kDirectMaxPixel &&
                    fabs(zp[o]) < kDirectMaxPixel;
 #pragma unroll
-  for (int c = 0; c < CH; ++c) acc[c] = 0.0;
+    for (int c = 0; c < CH; ++c) acc[o][c] = 0.0;
+  }
+  const bool active = p0 < nOut;
   // blockIdx.y takes one slice of the inputs (whole chunks); slices add their partial
   // sums atomically when the inputs are split
   const long long per = ((nIn + gridDim.y - 1) / gridDim.y + kDirectChunk - 1) / kDirectChunk * kDirectChunk;
   const long long kBegin = (long long)blockIdx.y * per;
   const long long kEnd = (kBegin + per < nIn) ? kBegin + per : nIn;
-  auto add = [&](int i, double s, double cs) {
+  auto add = [&](int o, int i, double s, double cs) {
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if (c < nch) {
         const double2 a = sval[c][i];
-        acc[c] = fma(a.x, cs, fma(-a.y, s, acc[c]));
+        acc[o][c] = fma(a.x, cs, fma(-a.y, s, acc[o][c]));
       }
     }
   };
@@ -844,7 +909,7 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
     inRange = __syncthreads_and(inRange) && pixelInRange;
     if (!active) continue;
     if (inRange && !fp64Trig) {
-#pragma unroll 4
+#pragma unroll 2
       for (int i = 0; i < nk; ++i) {
         const double2 uv = suv[i];
         const double wi = sw[i];
@@ -876,7 +941,6 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
           }
           add(o, i, s, cs);
         }
-        add(i, s, cs);
       }
     }
   }
@@ -888,9 +952,9 @@ direct_sum_kernel(double alpha, long long nIn, const C* __restrict__ input, long
     for (int c = 0; c < CH; ++c) {
       if (c < nch) {
         if (gridDim.y > 1)
-          atomicAdd(&out[(long long)c * ldOut + p], (TO)acc[c]);
+          atomicAdd(&out[(long long)c * ldOut + p], (TO)acc[o][c]);
         else
-          out[(long long)c * ldOut + p] += (TO)acc[c];
+          out[(long long)c * ldOut + p] += (TO)acc[o][c];
       }
     }
   }
@@ -911,6 +975,9 @@ inline dim3 direct_sum_grid(long long nOut, long long nIn, int smCount, int ctas
     const long long maxSlices = nIn / minSlice > 1 ? nIn / minSlice : 1;
     by = by < maxSlices ? by : maxSlices;
     by = by < 65535 ? by : 65535;
+    const long long sms = smCount > 0 ? smCount : 148, most = by;
+    for (long long t = most - 1; 4 * t >= 3 * most && t >= 1; --t)
+      if ((bx * t + sms - 1) / sms * by < (bx * by + sms - 1) / sms * t) by = t;
   }
   return dim3((unsigned)bx, (unsigned)by, 1);
 }
@@ -944,6 +1011,3 @@ static __global__ void value_scale_kernel(const int* __restrict__ total, const f
 }
 
 }  // namespace bippb200
-    const long long sms = smCount > 0 ? smCount : 148, most = by;
-    for (long long t = most - 1; 4 * t >= 3 * most && t >= 1; --t)
-      if ((bx * t + sms - 1) / sms * by < (bx * by + sms - 1) / sms * t) by = t;
