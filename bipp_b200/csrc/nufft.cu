@@ -455,28 +455,29 @@ void NufftCore::end_count(long long nPoints) {
   offsets_.ensure(ctx_, (n + 1) * sizeof(int));
   cursor_.ensure(ctx_, (n + 1) * sizeof(int));
   scan(counts_.get<int>(), offsets_.get<int>(), cursor_.get<int>(), n);
-  valStride_ = std::max<long long>(nPoints, 1);
-  rec_.ensure(ctx_, valStride_ * sizeof(PtRec));
-  vals_.ensure(ctx_, (size_t)nch_ * valStride_ * sizeof(float2));
+  ptCapacity_ = std::max<long long>(nPoints, 1);
+  pts_.ensure(ctx_, ptCapacity_ * pt_bytes(nch_));
+  valScale_.ensure(ctx_, kMaxChan * sizeof(unsigned));
+  B2_CUDA(cudaMemsetAsync(valScale_.get(), 0, kMaxChan * sizeof(unsigned), ctx_->stream));
 }
 
 template <int CH, int W>
 static void launch_spread_w(const NufftGeom& g, int nItems, size_t smem, cudaStream_t st, const int* offs,
-                            const PtRec* rec, const float2* vals, long long vs, int nch, const SpreadItem* items,
+                            const char* pts, int stride, int nch, const SpreadItem* items,
                             int tw0, int slabPlanes, float2* out) {
   auto k = spread_warp_kernel<CH, W>;
   smem_optin(k, smem);
   count_launch();
-  k<<<nItems, kSpreadThreads, smem, st>>>(g, offs, rec, vals, vs, nch, items, tw0, slabPlanes, out);
+  k<<<nItems, kSpreadThreads, smem, st>>>(g, offs, pts, stride, nch, items, tw0, slabPlanes, out);
 }
 
 template <int CH>
 static void launch_spread(const NufftGeom& g, int nItems, size_t smem, cudaStream_t st, const int* offs,
-                          const PtRec* rec, const float2* vals, long long vs, int nch, const SpreadItem* items, int tw0,
+                          const char* pts, int stride, int nch, const SpreadItem* items, int tw0,
                           int slabPlanes, float2* out) {
   switch (g.W) {
 #define B2_W(w) \
-  case w: launch_spread_w<CH, w>(g, nItems, smem, st, offs, rec, vals, vs, nch, items, tw0, slabPlanes, out); break;
+  case w: launch_spread_w<CH, w>(g, nItems, smem, st, offs, pts, stride, nch, items, tw0, slabPlanes, out); break;
     B2_W(2) B2_W(3) B2_W(4) B2_W(5) B2_W(6) B2_W(7) B2_W(8) B2_W(9)
 #undef B2_W
     default: throw Error(BIPP_INTERNAL_ERROR, "unsupported NUFFT kernel width");
@@ -486,9 +487,8 @@ static void launch_spread(const NufftGeom& g, int nItems, size_t smem, cudaStrea
 // tensor-core spreading (4 or 8 channels): persistent CTAs, as many per SM as tensor
 // memory allows
 template <int CH, int STAGES, bool AT, bool F16>
-static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, const int* offs, const PtRec* rec,
-                             const float2* vals, int chStride, int nch, const SpreadItem* items, int tw0,
-                             int slabPlanes, float2* out, int* errFlag, int* workCounter, const unsigned* valScale) {
+static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, const int* offs, const char* pts,
+                             int stride, int ch0, int nch, const SpreadItem* items, int tw0, int slabPlanes, float2* out, int* errFlag, int* workCounter, const unsigned* valScale) {
   using S = TcShape<CH, STAGES, AT, F16>;
   int dev = 0, sms = 148;
   B2_CUDA(cudaGetDevice(&dev));
@@ -499,7 +499,7 @@ static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, co
   const int grid = std::max(1, std::min(nItems, sms * std::min(S::MinBlocks, tuned("spread.ctas_per_sm"))));
   count_launch();
   spread_tc_kernel<CH, STAGES, AT, F16><<<grid, kTcThreads, S::Smem, st>>>(
-      g, offs, rec, vals, chStride, nch, items, nItems, tw0, slabPlanes, out, errFlag, workCounter, valScale);
+      g, offs, pts, stride, ch0, nch, items, nItems, tw0, slabPlanes, out, errFlag, workCounter, valScale);
 }
 
 // BIPP_B200_SPREAD=warp selects the shared-memory-atomic spreader for every channel count.
@@ -654,16 +654,6 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
   // spreader operands (tunable): 0 tf32 split with A in shared memory, 1 with A in tensor
   // memory, 2 FP16 hi/lo (values scaled per channel by their largest magnitude)
   const int operands = tc ? tuned("spread.operands") : 0;
-  valScale_.ensure(ctx_, kMaxChan * sizeof(unsigned));
-  if (operands == 2) {
-    B2_CUDA(cudaMemsetAsync(valScale_.get(), 0, kMaxChan * sizeof(unsigned), ctx_->stream));
-    if (lastPoints > 0) {
-      count_launch();
-      value_scale_kernel<<<std::min<long long>(4096, (lastPoints + 255) / 256), 256, 0, ctx_->stream>>>(
-          offsets_.get<int>() + nkeys_, vals_.get<float2>(), nch_, valScale_.get<unsigned>());
-      B2_CHECK_LAUNCH();
-    }
-  }
   const size_t smem = (size_t)nch_ * 2 * kTileCells * sizeof(float);
   errFlag_.ensure(ctx_, sizeof(int));
   B2_CUDA(cudaMemsetAsync(errFlag_.get(), 0, sizeof(int), ctx_->stream));
@@ -700,7 +690,7 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
       for (int c0 = 0, grp = 0; c0 < nch_; c0 += kTcMaxChan, ++grp) {
         const int nc = std::min(kTcMaxChan, nch_ - c0);
         const L launch = table[nc <= 4 ? 0 : 1][operands][two ? 1 : 0];
-        launch(g_, nItems, ctx_->stream, offsets_.get<int>(), rec_.get<PtRec>(), vals_.get<float2>() + c0, nch_, nc,
+        launch(g_, nItems, ctx_->stream, offsets_.get<int>(), pts_.get<char>(), pt_bytes(nch_), c0, nc,
                items_.get<SpreadItem>() + slabBegin[sl], tw0, slabPlanes,
                grid_.get<float2>() + slab_index(g_, nch_, slabPlanes, c0, 0, 0, 0), errFlag_.get<int>(),
                dynamic ? workCounters_.get<int>() + sl + grp * nslab : nullptr, valScale_.get<unsigned>() + c0);
@@ -709,11 +699,11 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
     } else if (nItems > 0) {
       const SpreadItem* it = items_.get<SpreadItem>() + slabBegin[sl];
       if (nch_ <= 4)
-        launch_spread<4>(g_, nItems, smem, ctx_->stream, offsets_.get<int>(), rec_.get<PtRec>(), vals_.get<float2>(),
-                         valStride_, nch_, it, tw0, slabPlanes, grid_.get<float2>());
+        launch_spread<4>(g_, nItems, smem, ctx_->stream, offsets_.get<int>(), pts_.get<char>(), pt_bytes(nch_),
+                         nch_, it, tw0, slabPlanes, grid_.get<float2>());
       else
-        launch_spread<kMaxChan>(g_, nItems, smem, ctx_->stream, offsets_.get<int>(), rec_.get<PtRec>(),
-                                vals_.get<float2>(), valStride_, nch_, it, tw0, slabPlanes, grid_.get<float2>());
+        launch_spread<kMaxChan>(g_, nItems, smem, ctx_->stream, offsets_.get<int>(), pts_.get<char>(),
+                                pt_bytes(nch_), nch_, it, tw0, slabPlanes, grid_.get<float2>());
       B2_CHECK_LAUNCH();
     }
     if (stageMs) B2_CUDA(cudaEventRecord(ev[1], ctx_->stream));
@@ -887,10 +877,10 @@ static void nufft_transform_lattice(bipp_nufft_s* p, long long n, long long ld) 
   B2_CHECK_LAUNCH();
   p->core.end_count(n);
   count_launch();
-  baseline_scatter_kernel<<<gb, 256, 0, ctx->stream>>>(g, bp, p->core.cursor(), p->core.records(), p->core.values(),
-                                                       p->core.value_stride(), p->core.sincos64() ? 1 : 0,
+  baseline_scatter_kernel<<<gb, 256, 0, ctx->stream>>>(g, bp, p->core.cursor(), p->core.points(), p->core.point_bytes(),
+                                                       p->core.point_capacity(), p->core.sincos64() ? 1 : 0,
                                                        p->core.corr_terms() ? 1 : 0, p->core.su(), p->core.sv(),
-                                                       p->core.zero_acc(), p->core.channels());
+                                                       p->core.zero_acc(), p->core.value_max());
   B2_CHECK_LAUNCH();
   p->core.execute(p->images.get<float>(), (long long)p->nPixel);
 }

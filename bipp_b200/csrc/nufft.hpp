@@ -46,11 +46,12 @@ public:
   // After the count kernels: scan -> offsets & cursor; allocate records for nPoints
   void end_count(long long nPoints);
   int* cursor() { return cursor_.get<int>(); }
-  PtRec* records() { return rec_.get<PtRec>(); }
-  // values of the sorted points, [point][channel] (channels() per point)
-  float2* values() { return vals_.get<float2>(); }
-  // capacity in points of records() / values() (the scatter kernels' bounds guard)
-  long long value_stride() const { return valStride_; }
+  // sorted points (PtRec and values, point_bytes() each) and their largest values per channel
+  char* points() { return pts_.get<char>(); }
+  int point_bytes() const { return pt_bytes(nch_); }
+  unsigned* value_max() { return valScale_.get<unsigned>(); }
+  // capacity of points() (the scatter kernels' bounds guard)
+  long long point_capacity() const { return ptCapacity_; }
   // per-channel accumulator of zero-baseline values (added to every pixel)
   double* zero_acc() { return zeroAcc_.get<double>(); }
   // spread/FFT/w-sum over all slabs and accumulate Re(...) into image[ch][P] (ld P)
@@ -62,7 +63,6 @@ public:
   // parts (more points than the spread.items_cap tunable; their parts accumulate with atomics)
   long long lastPoints = 0, lastSlabs = 0, lastGridBytes = 0, lastItems = 0, lastSplitTiles = 0;
   long long num_pixels() const { return (long long)g_.Na * g_.Nb; }
-  int channels() const { return nch_; }
   bool sincos64() const { return eps_ < 1e-6; }
   double su() const { return su_; }
   double sv() const { return sv_; }
@@ -76,8 +76,8 @@ private:
   double Sn_ = 0;
   bool corrTerms_ = false, corrCapable_ = false;
   double su_ = 1, sv_ = 1;
-  long long nkeys_ = 0, valStride_ = 0;
-  DevBuf nTilde_, decon_, dl_, dm_, counts_, offsets_, cursor_, blockSums_, rec_, vals_, grid_, acc_;
+  long long nkeys_ = 0, ptCapacity_ = 0;
+  DevBuf nTilde_, decon_, dl_, dm_, counts_, offsets_, cursor_, blockSums_, pts_, grid_, acc_;
   DevBuf itemKeys_, itemsAlt_, sortTmp_, workCounters_;
   DevBuf qz_, qw_, zeroAcc_, load_, items_, errFlag_, splitCount_, parts_, itemOff_, slabCounts_, clearFlag_, clearOff_, clearList_;
   DevBuf valScale_;   // per-channel value scale of the FP16 spreader operands

@@ -291,8 +291,8 @@ static void pipeline_chunk(bipp_pipeline_s* p, int s0, int nb, const std::vector
     const int gb = (int)std::min<long long>((total + 255) / 256, 16384);
     count_launch();
     pipeline_scatter_kernel<<<gb, 256, 0, ctx->stream>>>(p->core.geom(), pp, total, p->core.cursor(), relD.get<long long>(),
-                                                         p->core.records(), p->core.values(), p->core.value_stride(),
-                                                         p->core.sincos64() ? 1 : 0, p->core.channels());
+                                                         p->core.points(), p->core.point_bytes(), p->core.point_capacity(),
+                                                         p->core.sincos64() ? 1 : 0, p->core.value_max());
     B2_CHECK_LAUNCH();
   }
   if (ms) {

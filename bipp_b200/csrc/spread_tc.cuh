@@ -116,15 +116,15 @@ __device__ __forceinline__ int tc_range_pair(int j) {
   return -1;
 }
 
-// The nch <= CH channels of one launch are consecutive ones of chStride channels per point:
-// more than 8 channels are spread by several launches, vals, valScale and grid pointing at
+// The nch <= CH channels of one launch are consecutive ones of a point's, from ch0: more than
+// 8 channels are spread by several launches, valScale and grid pointing at
 // each launch's first channel.
 // Persistent: each CTA takes work items blockIdx.x, blockIdx.x + gridDim.x, ... or, with
 // a work counter, the next item of the (load-ordered) list whenever it is free
 template <int CH, int STAGES, bool AT = false, bool F16 = false>
 static __global__ void __launch_bounds__(kTcThreads, TcShape<CH, STAGES, AT, F16>::MinBlocks)
-spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __restrict__ rec,
-                 const float2* __restrict__ vals, int chStride, int nch, const SpreadItem* __restrict__ items,
+spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const char* __restrict__ pts, int stride, int ch0,
+                 int nch, const SpreadItem* __restrict__ items,
                  int nItems, int tw0, int slabPlanes, float2* __restrict__ grid, int* __restrict__ errFlag,
                  int* __restrict__ workCounter, const unsigned* __restrict__ valScale = nullptr) {
   using S = TcShape<CH, STAGES, AT, F16>;
@@ -241,21 +241,18 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const PtRec* __re
         const int q = lo + vb + pv;
         while (q >= rPre[ri + 1]) ++ri;
         const int p = rBeg[ri] + (q - rPre[ri]);
-        const PtRec* pr = rec + p;
-        if (pa < 4) {
-          pfL = __ldg(&pr->ix0);
-          pfD = __ldg(&pr->dx);
-        } else if (pa < 6) {
-          pfL = __ldg(&pr->iy0);
-          pfD = __ldg(&pr->dy);
-        } else {
-          pfL = __ldg(&pr->iw0);
-          pfD = __ldg(&pr->dw);
+        // the role's axis of the PtRec: its 8 bytes 0, 1 or 2
+        const float2 ld = __ldg(reinterpret_cast<const float2*>(pt_rec(pts, stride, p)) +
+                                (pa < 4 ? 0 : pa < 6 ? 1 : 2));
+        pfL = __float_as_int(ld.x);
+        pfD = ld.y;
+        if (pa >= 6) {
+          const float2* vals = pt_vals(pts, stride, p) + ch0;
           // values of a point are contiguous ([point][channel])
 #pragma unroll
           for (int cc = 0; cc < CPR; ++cc) {
             const int c = CPR * (pa - 6) + cc;
-            pfX[cc] = (c < nch) ? vals[(long long)p * chStride + c] : make_float2(0.f, 0.f);
+            pfX[cc] = (c < nch) ? vals[c] : make_float2(0.f, 0.f);
           }
         }
       }
