@@ -140,10 +140,7 @@ prep_kernel(int nBeam, const typename Cplx<T>::type* __restrict__ S, long long s
         const double x = 2.0 * sqrt(dx * dx + dy * dy + dz * dz) / w;
         g = (x != 0.0) ? sinpi(x) / (3.14159265358979323846 * x) : 1.0;
       }
-      if (withGram == 2)
-        reinterpret_cast<double*>(G)[(long long)b * Nmax * Nmax + r + (long long)c * Nmax] = g;
-      else
-        Gb[r + (long long)c * Nmax] = make_double2(g, 0.0);
+      Gb[r + (long long)c * Nmax] = make_double2(g, 0.0);
     }
   }
 }
@@ -268,10 +265,10 @@ __device__ __forceinline__ double2 e_div(double2 a, double2 d) {
 __device__ __forceinline__ double e_div(double a, double d) { return a / d; }
 
 // Panel rows below the diagonal block are X = A L_kk^-H with L_kk^-1 formed in shared
-// memory (as the triangular inverse does per block), a register-tiled product that keeps
-// the kernel at three CTAs per SM in the real case.
+// memory (as the triangular inverse does per block). For the Gram matrices of general
+// beamforming above 64 beams and the allocation-free entry point.
 template <typename E>
-__global__ void __launch_bounds__(kCholThreads, sizeof(E) == 8 ? 4 : 1)
+__global__ void __launch_bounds__(kCholThreads)
 cholesky_kernel(E* __restrict__ G, const int* __restrict__ nred, int Nmax, int* __restrict__ status,
                 const int* __restrict__ order = nullptr) {
   const int b = order ? order[blockIdx.x] : blockIdx.x;
@@ -436,14 +433,14 @@ __device__ __forceinline__ void store_conv(double* p, double v) { *p = v; }
 
 // Linv is computed block row by block row: Linv[I,I] = inv(L[I,I]);
 // Linv[I,J] = -Linv[I,I] sum_{K=J}^{I-1} L[I,K] Linv[K,J]. The FP64 inverse goes to W64
-// (read back for the later block rows) and, rounded, to LinvOut. E = double2 (complex)
-// or double (real symmetric G); O = the matching working-precision output element.
+// (read back for the later block rows) and, rounded, to LinvOut. O = the
+// working-precision output element.
 template <typename E>
 constexpr size_t trinv_smem() { return 3 * 32 * 33 * sizeof(E); }
 constexpr size_t kTrinvSmem = trinv_smem<double2>();
 
 template <typename E, typename O>
-__global__ void __launch_bounds__(256, sizeof(E) == 8 ? 8 : 1)
+__global__ void __launch_bounds__(256)
 trinv_kernel(const E* __restrict__ L, E* __restrict__ W64, O* __restrict__ LinvOut, const int* __restrict__ nred,
              int Nmax, const int* __restrict__ order = nullptr) {
   constexpr int NB = 32;
@@ -1826,6 +1823,7 @@ bt_apply_kernel(const C* __restrict__ A, const C* __restrict__ Tin, long long tS
       // sum over the row groups of the warp. 16 columns (8 row groups, lane bits 2..4): each
       // exchange halves what a lane keeps, and every lane ends with one of the 8 sums
       if constexpr (CGN == 4) {
+        static_assert(kBtJC * 4 == 8, "8 sums over 8 row groups");
         C* v = &w[0][0];
 #pragma unroll
         for (int half = 4; half >= 1; half >>= 1) {
@@ -1839,23 +1837,23 @@ bt_apply_kernel(const C* __restrict__ A, const C* __restrict__ Tin, long long tS
         }
         const int s = lane >> 2;   // sum s = reflector s / 4, column s % 4 of the group
         red[(warp * kBtNB + kBtJC * jc + (s >> 2)) * CB + 4 * cg + (s & 3)] = v[0];
-        continue;
-      }
-#pragma unroll
-      for (int a = 0; a < kBtJC; ++a)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-          for (int o = CGN; o < 32; o <<= 1) {
-            w[a][u].x += __shfl_xor_sync(0xffffffffu, w[a][u].x, o);
-            w[a][u].y += __shfl_xor_sync(0xffffffffu, w[a][u].y, o);
-          }
-        }
-      if (lane < CGN) {
+      } else {
 #pragma unroll
         for (int a = 0; a < kBtJC; ++a)
 #pragma unroll
-          for (int u = 0; u < 4; ++u) red[(warp * kBtNB + kBtJC * jc + a) * CB + 4 * cg + u] = w[a][u];
+          for (int u = 0; u < 4; ++u) {
+#pragma unroll
+            for (int o = CGN; o < 32; o <<= 1) {
+              w[a][u].x += __shfl_xor_sync(0xffffffffu, w[a][u].x, o);
+              w[a][u].y += __shfl_xor_sync(0xffffffffu, w[a][u].y, o);
+            }
+          }
+        if (lane < CGN) {
+#pragma unroll
+          for (int a = 0; a < kBtJC; ++a)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) red[(warp * kBtNB + kBtJC * jc + a) * CB + 4 * cg + u] = w[a][u];
+        }
       }
     }
     __syncthreads();

@@ -890,11 +890,6 @@ __global__ void add_double_to_float_kernel(const double* __restrict__ a, long lo
     b[i] += (float)a[i];
 }
 
-__global__ void d2f_kernel(const double* __restrict__ in, long long n, float* __restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = (float)in[i];
-}
-
 namespace bippb200 {
 float* nufft_stage_uvw(bipp_nufft_t p) { return p->uvw.get<float>() + p->count * p->nBaselines; }
 float2* nufft_stage_values(bipp_nufft_t p, size_t im) {
