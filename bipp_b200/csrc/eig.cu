@@ -373,8 +373,8 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
   const int grid1 = trdPct > 0 ? std::max(1, std::min(nb, trdPct * ctx->smCount / 100)) : 0;
   if (!hetrd_cluster<C, R>(st, ctx->smCount, (size_t)ctx->prop.l2CacheSize, ctx->maxSmemOptin, A, nred, Nmax, w.d.template get<double>(),
                            w.e.template get<double>(), w.tau.template get<C>(), sizeOrder, nb, Nmax,
-                           trdThreads > 0 ? trdThreads / 256 : 8, grid1)) {
-    // larger matrices: one CTA each; in single precision blocked panels while the V/W panel
+                           trdThreads / 256, grid1)) {
+    // larger matrices, or many large ones: one CTA each; in single precision blocked panels while the V/W panel
     // fits in shared memory
     bool blocked = false;
     if constexpr (sizeof(C) == 8) blocked = hetrd_blk_smem_bytes(Nmax) <= ctx->maxSmemOptin;

@@ -635,15 +635,18 @@ inline void ht_launch_cs(cudaStream_t st, int grid, size_t smem, C* A, const int
 // at most 90 % of the SMs (clusters do not pack every SM; 37 matrices of 333 rows: 2.54 ms at
 // 2, 2.91 at 4) and a matrix has 64 rows per CTA (below, the repeated work of a column and the
 // cluster barrier cost more than the shared product: 60 rows 0.20 ms at 1, 0.24 at 2); and
-// while the lower triangles in flight exceed 5/4 of L2 (64 matrices of 1024 rows: 34.0 ms at
-// 2, all 64 in flight, 28.1 at 4).
+// while the lower triangles in flight exceed 8/5 of L2 (64 matrices of 1024 rows: 34.0 ms at
+// 2, all 64 in flight, 28.1 at 4; 150 of 1000: 109 and 91; 300 of 768 75 at 2, 85 at 4), as
+// long as the batch is at most 3/2 matrices per SM: beyond, one CTA each has the highest rate
+// (1024 of 768 rows: 218 ms, 227 at 2, 275 at 4), and larger clusters only even out a last
+// wave.
 template <typename C, typename R, int NB, int T, int RPT>
 inline void ht_launch(cudaStream_t st, int smCount, size_t l2Bytes, C* A, const int* nred, int ld, double* d, double* e,
                       C* tau, const int* order, int nb, int nmax, int most, int grid1) {
   int cs = 1;
   while (cs < most && 128 * cs <= nmax) {
     const double inFlight = std::min<double>(nb, (double)smCount / cs) * 0.5 * nmax * nmax * sizeof(C);
-    if (10ll * nb * cs * 2 > 9ll * smCount && inFlight <= 1.25 * l2Bytes) break;
+    if (10ll * nb * cs * 2 > 9ll * smCount && (2 * nb > 3 * smCount || inFlight <= 1.6 * l2Bytes)) break;
     cs *= 2;
   }
   const size_t smem = ht_smem<C, NB, T>(nmax, cs > 1);
@@ -672,16 +675,20 @@ bool hetrd_cluster(cudaStream_t st, int smCount, size_t l2Bytes, size_t maxSmem,
   }
   if constexpr (sizeof(C) == 8) {
     if (nmax > 1024) return false;
+    // of many matrices above 896 rows hetrd_blk_kernel, whose panels hold 8 columns at these
+    // sizes too, is the faster one (310 of 1000 rows: 175 ms against 200 here, of 800 rows 91
+    // against 86; 200 of 1000 115 against 122, 150 of them 112 against 91)
+    if (most == 0 && nmax > 896 && 4 * nb > 5 * smCount) return false;
     const auto k = nmax <= 256 && nb > smCount ? ht_launch<C, R, 8, 256, 1>
                    : nmax <= 512               ? ht_launch<C, R, 8, 512, 1>
                                                : ht_launch<C, R, 4, 512, 2>;
-    k(st, smCount, l2Bytes, A, nred, ld, d, e, tau, order, nb, nmax, most, grid1);
+    k(st, smCount, l2Bytes, A, nred, ld, d, e, tau, order, nb, nmax, most ? most : 8, grid1);
   } else {
     if (nmax > 1024 || (nmax > 512 && ht_smem<C, 4, 256>(nmax, true) > maxSmem)) return false;
     const auto k = nmax <= 256   ? ht_launch<C, R, 8, 256, 1>
                    : nmax <= 512 ? ht_launch<C, R, 8, 256, 2>
                                  : ht_launch<C, R, 4, 256, 4>;
-    k(st, smCount, l2Bytes, A, nred, ld, d, e, tau, order, nb, nmax, most, grid1);
+    k(st, smCount, l2Bytes, A, nred, ld, d, e, tau, order, nb, nmax, most ? most : 8, grid1);
   }
   return true;
 }

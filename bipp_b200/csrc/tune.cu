@@ -3,7 +3,7 @@
 // The reference's only launch-shape logic is a fixed block-size ladder for its direct sum
 // (src/gpu/kernels/nuft_sum.cu:73-84); here the shapes that matter for the batched
 // pipeline are measured on the caller's own workload: the points per spreading work item
-// and the spreader's resident CTAs per SM, the threads of the per-matrix
+// and the spreader's resident CTAs per SM, the share of the GPU for one matrix's
 // tridiagonalisation, the persistent grid of the tensor-core virtual visibilities, and the
 // input split of the direct sum. The tuner walks the parameters one at a time (coordinate
 // descent), times each candidate with CUDA events around a full pipeline call on the

@@ -166,6 +166,39 @@ def test_eigh_gram_sizes(ctx, n, b, precision):
         assert np.linalg.norm(g @ (vk * d[k]) @ vk.conj().T @ g - s64) <= tol * n * cond * scale, k
 
 
+@pytest.mark.parametrize("n,b", [(896, 223), (897, 185), (897, 186)])
+def test_eigenvalues_of_many_large_matrices(ctx, n, b):
+    """Batches around the sizes from which a matrix takes one CTA of the panel kernel; most
+    antennas are flagged (zero rows). FP32 eigenvalues against scipy's FP64 solver, 32 eps
+    sqrt(kept) normwise as above."""
+    import scipy.linalg
+
+    import bipp_b200 as bipp
+
+    rng = np.random.default_rng(n + b)
+    kept = 45
+    s0, x0 = _steps(rng, 3, kept, np.complex64)
+    s = np.zeros((b, n, n), dtype=np.complex64)
+    xyz = np.zeros((b, n, 3))
+    xyz[:, :, 2] = 10.0 + np.arange(n)
+    at = np.sort(rng.choice(n, kept, replace=False))
+    for k in range(b):
+        s[k][np.ix_(at, at)] = s0[k % 3]
+        xyz[k, at] = x0[k % 3]
+    _, d, nred, _ = bipp.eigh_gram_batched(np.full(b, 2.0), s, xyz, ctx=ctx)
+    assert (nred == kept).all()
+    tol = 32 * np.finfo(np.float32).eps * math.sqrt(kept)
+    for k in (0, 1, b - 1):
+        x = x0[k % 3].astype(np.float32).astype(np.float64)
+        g = np.sinc(np.linalg.norm(x[:, None] - x[None], axis=2))
+        s64 = np.tril(s0[k % 3]).astype(np.complex128)
+        s64 = s64 + np.tril(s64, -1).conj().T
+        np.fill_diagonal(s64, s64.diagonal().real)
+        ref = scipy.linalg.eigh(s64, g, eigvals_only=True)
+        bound = tol * np.abs(ref).max() * max(1.0, math.sqrt(np.linalg.cond(g)))
+        assert np.abs(d[k][:kept] - ref).max() <= bound, k
+
+
 @pytest.mark.parametrize("px", [11, 26, 41, 63, 114, 200, 274, 343, 514, 900, 1200])
 def test_fft_lines_with_several_odd_factors(ctx, px):
     """Image widths whose fine grids have more than one odd factor (among them 48, 144, 240,
