@@ -1318,7 +1318,10 @@ tridiag_kernel(const double* __restrict__ dIn, const double* __restrict__ eIn, c
                const int* __restrict__ predK = nullptr, int predMargin = 16, double resTol = -1.0) {
   const int b = order ? order[blockIdx.x] : blockIdx.x;
   const int n = nred[b];
-  if (n <= 0) return;
+  if (n <= 0) {
+    if (krange && threadIdx.x < 2) krange[2 * b + threadIdx.x] = 0;
+    return;
+  }
   extern __shared__ double smem_d[];
   double* d = smem_d;            // [Nmax]
   double* e = d + Nmax;          // [Nmax]

@@ -102,7 +102,10 @@ tridiag_values_kernel(const double* __restrict__ dIn, const double* __restrict__
                       int* __restrict__ range, const int* __restrict__ order) {
   const int b = order ? order[blockIdx.y] : blockIdx.y;
   const int n = nred[b];
-  if (n <= 0) return;
+  if (n <= 0) {   // every row flagged: an empty range
+    if (blockIdx.x == 0 && threadIdx.x < 2) range[2 * b + threadIdx.x] = 0;
+    return;
+  }
   extern __shared__ __align__(16) double2 ts_smem[];
   double2* de = ts_smem;
   __shared__ double red[32];
@@ -200,7 +203,10 @@ tridiag_vectors_kernel(const double* __restrict__ dIn, const double* __restrict_
                        double* __restrict__ work, const int* __restrict__ order) {
   const int b = order ? order[blockIdx.y] : blockIdx.y;
   const int n = nred[b];
-  if (n <= 0) return;
+  if (n <= 0) {
+    if (blockIdx.x == 0 && threadIdx.x < 2) krange[2 * b + threadIdx.x] = 0;
+    return;
+  }
   extern __shared__ __align__(16) double2 ts_smem[];
   double2* de = ts_smem;   // (d_k, e_k), scaled
   __shared__ double red[32], sBest[kTsThreads], sNrm[kTsThreads];

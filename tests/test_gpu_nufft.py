@@ -464,3 +464,37 @@ def test_pipeline_filters_vs_fp64_oracle(ctx, filt):
     pl.close()
     for lv in range(intervals.shape[0]):
         assert _rel_l2(img[lv], ref_img[:, lv]) <= 1e-3, (lv, _rel_l2(img[lv], ref_img[:, lv]))
+
+
+@pytest.mark.parametrize("empty", [[0], [1, 3], [0, 1, 2, 3]])
+def test_pipeline_fully_flagged_steps(ctx, empty):
+    """Steps without any visibility count as steps and add nothing: the sum over the batch
+    equals that over the other steps, whatever the buffers held before (the batch's own
+    steps in another order first). Tolerance as for a repeated batch: rounding of the
+    FP32 sums, 1e-6."""
+    import bipp_b200 as bipp
+
+    cfg, obs, s, xyz = _pipeline_case(n_ant=40, n_steps=4, image=24)
+    intervals = np.array([[0.0, 1.0], [1.0, np.inf]])
+    wl = np.full(s.shape[0], cfg.wl)
+    pl = bipp.Pipeline(ctx, cfg.n_antenna, intervals, _lattice(obs, cfg.image_size), obs.lmn[:, 2], obs.basis,
+                       tolerance=1e-6)
+    cut = s.copy()
+    cut[empty] = 0
+    pl.process(cut, xyz, wl)
+    first = pl.images(normalize=False)
+    pl.reset()
+    pl.process(s, xyz, wl)
+    pl.reset()
+    pl.process(cut, xyz, wl)
+    again = pl.images(normalize=False)
+    assert np.array_equal(pl.images(), (again * np.float32(1.0 / len(s))))
+    pl.reset()
+    rest = [k for k in range(len(s)) if k not in empty]
+    if rest:
+        pl.process(s[rest], xyz[rest], wl[rest])
+        ref = pl.images(normalize=False).astype(np.float64)
+        assert _rel_l2(first, ref) <= 1e-6 and _rel_l2(again, ref) <= 1e-6
+    else:
+        assert not first.any() and not again.any()
+    pl.close()
