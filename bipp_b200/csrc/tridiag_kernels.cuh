@@ -9,9 +9,10 @@
 // and 53 bisection steps (6.0 ms for one matrix of 550 rows, 13.5 ms for 2048 matrices of
 // 380-512 rows). Here
 //  - the recurrences run on p_k = (d_k - x) p_{k-1} - e_{k-1}^2 p_{k-2} (q_k = p_k / p_{k-1}),
-//    one dependent FMA per step; p is rescaled every 8 steps. Each step's rounding is a
-//    relative perturbation of d_k - x and e_{k-1}^2, as in the quotient form. The matrix is
-//    scaled by a power of two to a norm in [1/2, 1), so 8 steps stay far inside FP64 range;
+//    one dependent FMA per step. Each step's rounding is a relative perturbation of d_k - x
+//    and e_{k-1}^2, as in the quotient form. The matrix is scaled by a power of two to a norm
+//    in [1/2, 1), p is rescaled every 8 steps (4 in the factorisations) and pivots are
+//    bounded below (ts_pivot), so that every p is a normal number;
 //  - a CTA first counts at 128 points across the whole interval in one sweep, which gives
 //    every eigenvalue its starting interval; then M lanes per eigenvalue cut it M + 1 ways
 //    per sweep. M (1..32) is chosen so that the lanes of the batch fill the GPU once:
@@ -26,29 +27,42 @@ namespace bippb200 {
 
 constexpr int kTsThreads = 128;
 
-// quotient replaced by -2^-100 (of the scaled matrix) when a pivot is exactly zero
+// Pivots q_k = p_k / p_{k-1} below 2^-100 in magnitude (of the scaled matrix) count as
+// -2^-100: a perturbation of d_k of that size, far below a rounding of the norm. It bounds
+// what a product of pivots can reach between two rescales, so that couplings and differences
+// down to the smallest numbers leave no p subnormal.
 constexpr double kTsTiny = 7.888609052210118e-31;
 
-// p replaced when zero, so that p / prev = -2^-100
-__device__ __forceinline__ double ts_nonzero(double p, double prev) {
-  return (__double2hiint(p) & 0x7fffffff) == 0 ? -kTsTiny * prev : p;
+// p with its pivot p / prev so bounded
+__device__ __forceinline__ double ts_pivot(double p, double prev) {
+  const int hp = __double2hiint(p) & 0x7ff00000, hq = __double2hiint(prev) & 0x7ff00000;
+  return hp < hq - (100 << 20) ? -kTsTiny * prev : p;
 }
 
-// common power-of-two factor that brings the larger of |a|, |b| to [1, 2)
+// The counts' form, one comparison with a constant: `steps` steps after a rescale p stays at
+// or above 2^-100 (steps + 1), by induction over prev
+__device__ __forceinline__ double ts_pivot(double p, double prev, int steps) {
+  return (__double2hiint(p) & 0x7fffffff) < ((1023 - 100 * (steps + 1)) << 20) ? -kTsTiny * prev : p;
+}
+
+// common power-of-two factor that brings the larger of |a|, |b| to [1, 2); b, of which the
+// next pivots are multiples, then at least 2^-100 in magnitude, with its sign
 __device__ __forceinline__ void ts_rescale(double& a, double& b) {
   const int ha = __double2hiint(a) & 0x7ff00000, hb = __double2hiint(b) & 0x7ff00000;
   const double s = __hiloint2double(0x7fe00000 - max(ha, hb), 0);
   a *= s;
   b *= s;
+  const int h = __double2hiint(b);
+  if ((h & 0x7fffffff) < (923 << 20)) b = __hiloint2double((h & (int)0x80000000) | (923 << 20), 0);
 }
 
 // eigenvalues of the scaled matrix below x; de[k] = (d_k, e_{k-1}^2), de[0].y unused
 __device__ __forceinline__ int ts_count(const double2* __restrict__ de, int n, double x) {
-  double p0 = 1.0, p1 = ts_nonzero(de[0].x - x, 1.0);
+  double p0 = 1.0, p1 = ts_pivot(de[0].x - x, 1.0, 0);
   unsigned cnt = (unsigned)__double2hiint(p1) >> 31;
   int k = 1;
-  auto step = [&](double2 v) {
-    const double p2 = ts_nonzero(fma(v.x - x, p1, -v.y * p0), p1);
+  auto step = [&](double2 v, int u) {
+    const double p2 = ts_pivot(fma(v.x - x, p1, -v.y * p0), p1, u + 1);
     cnt += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
     p0 = p1;
     p1 = p2;
@@ -56,10 +70,10 @@ __device__ __forceinline__ int ts_count(const double2* __restrict__ de, int n, d
   for (; k + 8 <= n; k += 8) {
     ts_rescale(p0, p1);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) step(de[k + u]);
+    for (int u = 0; u < 8; ++u) step(de[k + u], u);
   }
   ts_rescale(p0, p1);
-  for (; k < n; ++k) step(de[k]);
+  for (int u = 0; k < n; ++k, ++u) step(de[k], u);
   return (int)cnt;
 }
 
@@ -176,17 +190,6 @@ tridiag_values_kernel(const double* __restrict__ dIn, const double* __restrict__
   if (act && j == 0) lam[i] = 0.5 * (a + c) / scale;
 }
 
-// a / x to about a rounding: reciprocal by Newton's iteration from the hardware estimate, the
-// quotient corrected by its residual; a and x are normal numbers within 2^+-600 here
-__device__ __forceinline__ double ts_div(double a, double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  y = fma(y, fma(-x, y, 1.0), y);
-  const double q = a * y;
-  return fma(fma(-x, q, a), y, q);
-}
-
 // Eigenvectors of the eigenvalues range[2b] .. range[2b+1]-1 of matrix b (trimmed to
 // [vecLo, vecHi] by value), by the twisted factorisation of T - lambda I at the index of
 // the smallest |gamma|. CTA (c, r): 64 eigenvectors, lanes of the first half of the CTA
@@ -247,8 +250,8 @@ tridiag_vectors_kernel(const double* __restrict__ dIn, const double* __restrict_
     auto one = [&](int t) {
       const int k = role ? n - 2 - t : t;
       const double ek = de[k].y, dn = de[role ? k : k + 1].x;
-      p1 = ts_nonzero(p1, p0);
-      if (act) *out = ts_div(ek * p0, p1);
+      p1 = ts_pivot(p1, p0);
+      if (act) *out = ek * p0 / p1;
       out += step;
       const double p2 = fma(dn - l, p1, -(ek * ek) * p0);
       p0 = p1;
@@ -258,7 +261,7 @@ tridiag_vectors_kernel(const double* __restrict__ dIn, const double* __restrict_
     for (; t + 4 <= n - 1; t += 4) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) one(t + u);
-      p1 = ts_nonzero(p1, p0);
+      p1 = ts_pivot(p1, p0);
       ts_rescale(p0, p1);
     }
     for (; t < n - 1; ++t) one(t);

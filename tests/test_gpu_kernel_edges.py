@@ -214,3 +214,23 @@ def test_fft_lines_with_several_odd_factors(ctx, px):
         lmn = np.stack([l, m, np.sqrt(1 - l * l - m * m)], 1).astype(np.float32)
         uvw, c = _points(rng, 500, 400.0, 20.0, 1)
         _check_nufft(ctx, lmn, uvw, c, 1e-6, 2e-5)
+
+
+@pytest.mark.parametrize("n", [24, 40, 130, 300])
+@pytest.mark.parametrize("power", [-60, -300, -505, -514, -517, -519, -522, -600])
+def test_nearly_decoupled_tridiagonal(ctx, n, power):
+    """Tridiagonal FP64 matrices whose couplings are tiny, so that eigenvalues meet diagonal
+    entries exactly and products of pivots pass the smallest numbers. The eigenvalues are the
+    diagonal to a rounding of the norm each way (4 eps), the eigenvectors unit vectors to 64
+    eps (the couplings, below 2^-60, over gaps of 1 / 2 n, are far less)."""
+    import bipp_b200 as bipp
+
+    d0 = 0.5 + (np.arange(n) * 7 % n + 0.25) / (2.0 * n) if n % 7 else 0.5 + np.arange(n) / (2.0 * n)
+    e = np.full(n - 1, 2.0 ** power)
+    s = np.diag(d0) + np.diag(e, -1) + np.diag(e, 1)
+    v, d, nred, _ = bipp.eigh(2.0, s.astype(np.complex128), np.eye(n), ctx=ctx, full=True)
+    eps = np.finfo(np.float64).eps
+    order = np.argsort(d0)
+    assert nred == n
+    assert np.abs(d - d0[order]).max() <= 4 * eps
+    assert np.abs(np.abs(v[order, :]) - np.eye(n)).max() <= 64 * eps
