@@ -173,7 +173,10 @@ tridiag_values_kernel(const double* __restrict__ dIn, const double* __restrict__
   const unsigned group = (M == 32 ? 0xffffffffu : ((1u << M) - 1u)) << ((tid & 31) / M * M);
   bool done = !act;
   for (int it = 0; it < 64; ++it) {
-    done = done || c - a <= fmax(2.0 * eps * fmax(fabs(a), fabs(c)), eps * tnorm);
+    // half the width at which halving would end (between eps / 2 and eps of the norm): a cut
+    // into many parts can stop anywhere below the bound, and the eigenvectors, which are as
+    // exact as the eigenvalue over its gap, were up to 1.7 times further off for it
+    done = done || c - a <= fmax(eps * fmax(fabs(a), fabs(c)), 0.5 * eps * tnorm);
     if (!__any_sync(0xffffffffu, !done)) break;
     const double x = a + (c - a) * (f * (j + 1));
     const bool above = done ? false : ts_count(de, n, x) > i;

@@ -234,3 +234,24 @@ def test_nearly_decoupled_tridiagonal(ctx, n, power):
     assert nred == n
     assert np.abs(d - d0[order]).max() <= 4 * eps
     assert np.abs(np.abs(v[order, :]) - np.eye(n)).max() <= 64 * eps
+
+
+@pytest.mark.parametrize("n", [100, 301, 512])
+@pytest.mark.parametrize("top", [3.0, 4.0, 8.0, 100.0])
+def test_eigenvalue_width(ctx, n, top):
+    """Eigenvalues of the second difference matrix, 2 cos(pi k / (n + 1)), beside one decoupled
+    entry that sets the norm, in FP64. Bisection ends at a width of half a rounding of the
+    norm, so the error is uniform within eps / 4 of it: 0.144 eps in the mean square, and 0.2
+    eps allowed with the counts' own roundings (ending at a whole one gives up to 0.289)."""
+    import bipp_b200 as bipp
+
+    ld = np.longdouble
+    exact = np.sort(2 * np.cos(np.arange(1, n + 1).astype(ld) * (4 * np.arctan(ld(1))) / (n + 1)))
+    s = np.zeros((n + 1, n + 1), dtype=np.complex128)
+    s[np.arange(1, n), np.arange(n - 1)] = 1.0
+    s[np.arange(n - 1), np.arange(1, n)] = 1.0
+    s[n, n] = top
+    _, d, nred, _ = bipp.eigh(2.0, s, np.eye(n + 1), ctx=ctx, full=True)
+    assert nred == n + 1
+    err = (d[:n].astype(ld) - exact)[np.abs(exact) <= top / 2]
+    assert np.sqrt(np.mean(err ** 2)) <= 0.2 * np.finfo(np.float64).eps * top
