@@ -255,3 +255,36 @@ def test_eigenvalue_width(ctx, n, top):
     assert nred == n + 1
     err = (d[:n].astype(ld) - exact)[np.abs(exact) <= top / 2]
     assert np.sqrt(np.mean(err ** 2)) <= 0.2 * np.finfo(np.float64).eps * top
+
+
+@pytest.mark.parametrize("umax", [10.0, 900.0, 3e4])
+def test_direct_sum_double_phases(ctx, umax):
+    """FP64 direct sums against 80-bit ones: no further off than the plain FP64 form of the
+    phase, alpha x rounded and every product and sum of it, which rounds more often than the
+    kernel's multiply-adds; 1.1 for the sampling of 600 outputs of 2000 terms."""
+    import bipp_b200 as bipp
+
+    ld = np.longdouble
+    twopi = 8 * np.arctan(ld(1))
+    got, plain = [], []
+    for seed in range(12):
+        rng = np.random.default_rng(seed)
+        u, x = rng.uniform(-umax, umax, (3, 2000)), rng.uniform(-1, 1, (3, 50))
+        v = rng.standard_normal(2000) + 1j * rng.standard_normal(2000)
+        alpha = 1.25 * (1 + 0.3 * rng.random())
+
+        def total(phase):
+            phase = phase.astype(ld)
+            phase = phase - twopi * np.round(phase / twopi)
+            return (np.cos(phase) * v.real - np.sin(phase) * v.imag).sum(1)
+
+        ref = total(ld(alpha) * (x.astype(ld).T @ u.astype(ld)))
+        xa = (alpha * x).T
+        p = xa[:, 0, None] * u[0] + xa[:, 1, None] * u[1] + xa[:, 2, None] * u[2]
+        out = bipp.nuft_sum(alpha, v, u[0], u[1], u[2], x[0], x[1], x[2], ctx=ctx)
+        # the sum itself rounds too, in FP64 on either side: a real and an imaginary product per
+        # term, added in turn
+        both = np.stack([np.cos(p) * v.real, -np.sin(p) * v.imag], 2).reshape(len(p), -1)
+        plain.append((total(p) - ref) + (both.cumsum(1)[:, -1] - both.astype(ld).sum(1)))
+        got.append(out - ref)
+    assert np.sqrt(np.mean(np.square(got))) <= 1.1 * np.sqrt(np.mean(np.square(plain)))
