@@ -39,6 +39,7 @@
 namespace bippb200 {
 
 constexpr int kHtSeg = 128;   // rows per unit when a cluster shares a matrix
+constexpr int kHtAlign = 256;   // of the panel: its widest row (HtPanel::kRow)
 
 // rows in shared memory: whole blocks of 32
 __host__ __device__ constexpr int ht_pad(int nmax) { return (nmax + 31) & ~31; }
@@ -81,7 +82,9 @@ template <typename C, int NB> struct HtPanel;
 template <int NB> struct HtPanel<float2, NB> {   // piece q = (V, W)
   static constexpr int kRow = NB * 16;
   static constexpr uint32_t kMask = NB * 16 - 16;
-  uint32_t base;   // shared address, 128-byte aligned
+  // the exclusive or must not reach the base's bits, nor leave the row
+  static_assert(kRow <= kHtAlign && kHtAlign % kRow == 0, "rows aligned to their own size");
+  uint32_t base;   // shared address, aligned to kHtAlign
   __device__ __forceinline__ uint32_t row(int r) const { return base + (uint32_t)r * kRow + (((uint32_t)r << 4) & kMask); }
   static __device__ __forceinline__ void get(uint32_t row, int q, float2& v, float2& w) {
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -99,6 +102,7 @@ template <int NB> struct HtPanel<float2, NB> {   // piece q = (V, W)
 };
 template <int NB> struct HtPanel<double2, NB> {   // pieces 2 q = V_q, 2 q + 1 = W_q
   static constexpr int kRow = NB * 32;
+  static_assert(kRow <= kHtAlign && kHtAlign % kRow == 0, "rows aligned to their own size");
   uint32_t base;
   __device__ __forceinline__ uint32_t row(int r) const { return base + (uint32_t)r * kRow + (((uint32_t)r << 4) & 112u); }
   static __device__ __forceinline__ double2 one(uint32_t row, int q, int w) {
@@ -490,7 +494,7 @@ __global__ void __launch_bounds__(T, sizeof(C) == 8 && T == 256 ? 2 : 1)
 hetrd_cluster_kernel(C* __restrict__ A, const int* __restrict__ nred, int ld, double* __restrict__ dOut,
                      double* __restrict__ eOut, C* __restrict__ tauOut, const int* __restrict__ order, int nBatch,
                      int nmax) {
-  extern __shared__ __align__(128) unsigned char ht_smem_raw[];
+  extern __shared__ __align__(kHtAlign) unsigned char ht_smem_raw[];
   const uint32_t rank = CS > 1 ? ht_cluster_rank() : 0;
   for (int w = blockIdx.x / CS; w < nBatch; w += gridDim.x / CS) {
     const int b = order[w], n = nred[b];
