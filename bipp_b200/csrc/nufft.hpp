@@ -62,6 +62,9 @@ public:
   // grid written by the spreading (all slabs), work items, tiles split into several
   // parts (more points than the spread.items_cap tunable; their parts accumulate with atomics)
   long long lastPoints = 0, lastSlabs = 0, lastGridBytes = 0, lastItems = 0, lastSplitTiles = 0;
+  // the transform's accumulators, free between transforms: 2 floats per pixel and channel
+  float* scratch() const { return acc_.get<float>(); }
+  long long scratch_floats() const { return (long long)(acc_.bytes() / sizeof(float)); }
   long long num_pixels() const { return (long long)g_.Na * g_.Nb; }
   bool sincos64() const { return eps_ < 1e-6; }
   double su() const { return su_; }

@@ -585,14 +585,19 @@ BippError bipp_pipeline_images(bipp_pipeline_t pl, float* images, int normalize,
     bipp_ctx_s* ctx = pl->ctx;
     const long long n = (long long)pl->nLevels * pl->P;
     if (normalize && pl->stepsDone > 0) {
-      // one pass from the accumulated images to the caller's, or to a buffer that is copied out
-      DevBuf host;
-      if (!onDevice) host.alloc(ctx, n * sizeof(float));
-      float* out = onDevice ? images : host.get<float>();
-      count_launch();
-      scale_images_kernel<<<2048, 256, 0, ctx->stream>>>(pl->images.get<float>(), n, 1.0f / (float)pl->stepsDone, out);
-      B2_CHECK_LAUNCH();
-      if (!onDevice) d2h(ctx, images, out, n * sizeof(float));
+      // one pass from the accumulated images to the caller's, or piece by piece through the
+      // transform's accumulators, idle here, so that images on the host need no more memory
+      // on the device
+      const float scale = 1.0f / (float)pl->stepsDone;
+      const long long piece = onDevice ? n : std::min(n, pl->core.scratch_floats());
+      for (long long i = 0; i < n; i += piece) {
+        const long long m = std::min(piece, n - i);
+        float* out = onDevice ? images : pl->core.scratch();
+        count_launch();
+        scale_images_kernel<<<2048, 256, 0, ctx->stream>>>(pl->images.get<float>() + i, m, scale, out);
+        B2_CHECK_LAUNCH();
+        if (!onDevice) d2h(ctx, images + i, out, m * sizeof(float));
+      }
     } else {
       B2_CUDA(cudaMemcpyAsync(images, pl->images.get(), n * sizeof(float),
                               onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream));

@@ -498,3 +498,30 @@ def test_pipeline_fully_flagged_steps(ctx, empty):
     else:
         assert not first.any() and not again.any()
     pl.close()
+
+
+@pytest.mark.parametrize("mode", ["batched", "plain"])
+def test_pipeline_images_need_no_device_memory(ctx, mode):
+    """Normalised images read back to the host allocate nothing on the device (the high-water
+    mark of its memory pool stays where it was) and equal the sums over the steps divided by
+    their number to a rounding each."""
+    import ctypes as C
+
+    import bipp_b200 as bipp
+
+    cfg, obs, s, xyz = _pipeline_case(n_ant=24, n_steps=3, image=301)
+    intervals = np.array([[0.0, 0.3], [0.3, 1.0], [1.0, 3.0], [3.0, np.inf]])
+    pl = bipp.Pipeline(ctx, cfg.n_antenna, intervals, _lattice(obs, cfg.image_size), obs.lmn[:, 2], obs.basis,
+                       tolerance=1e-4, mode=mode)
+    pl.process(s, xyz, np.full(3, cfg.wl))
+    cu = C.CDLL("libcuda.so.1")
+    pool, used, high = C.c_void_p(), C.c_uint64(), C.c_uint64(0)
+    in_use, in_use_high = 7, 8   # bytes of the pool in use, and their high-water mark
+    assert cu.cuDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+    assert cu.cuMemPoolSetAttribute(pool, in_use_high, C.byref(high)) == 0
+    assert cu.cuMemPoolGetAttribute(pool, in_use, C.byref(used)) == 0
+    img = pl.images()
+    assert cu.cuMemPoolGetAttribute(pool, in_use_high, C.byref(high)) == 0
+    assert high.value == used.value > 0
+    assert np.array_equal(img, pl.images(normalize=False) * np.float32(1.0 / 3.0))
+    pl.close()
