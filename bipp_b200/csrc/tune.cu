@@ -19,6 +19,7 @@
 #include <mutex>
 #include <sstream>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "bipp_b200.h"
@@ -89,29 +90,50 @@ Param* find(const char* name) {
   return nullptr;
 }
 
-void set_value(const char* name, int value) {
+Param* check_value(const char* name, int value) {
   Param* p = find(name);
   if (!p) throw Error(BIPP_INVALID_PARAMETER_ERROR, std::string("unknown tunable parameter: ") + name);
   if (std::find(p->candidates.begin(), p->candidates.end(), value) == p->candidates.end())
     throw Error(BIPP_INVALID_PARAMETER_ERROR, std::string("value not among the candidates of ") + name);
-  p->value = value;
+  return p;
 }
+
+void set_value(const char* name, int value) { check_value(name, value)->value = value; }
+
+// Written as "format 2". In files without that line the parameters below still count threads
+// of a matrix's one CTA; their values say nothing about the present kernels and are not taken
+// over (256 would hold a matrix to one CTA, 128 the search for its eigenvalues to an eighth of
+// the lanes).
+constexpr int kFileFormat = 2;
+constexpr const char* kNewMeaning[] = {"hetrd.threads", "tridiag.threads"};
 
 // "name value" lines; '#' starts a comment
 void load_file(const char* path) {
   std::ifstream in(path);
   if (!in) throw Error(BIPP_INVALID_PARAMETER_ERROR, std::string("cannot read tuning file: ") + path);
-  std::string line;
-  while (std::getline(in, line)) {
+  std::vector<std::pair<std::string, int>> entries;
+  std::string line, malformed;
+  int format = 1;
+  while (malformed.empty() && std::getline(in, line)) {
     const auto hash = line.find('#');
     if (hash != std::string::npos) line.resize(hash);
     std::istringstream ls(line);
     std::string name;
     int value;
     if (!(ls >> name)) continue;
-    if (!(ls >> value)) throw Error(BIPP_INVALID_PARAMETER_ERROR, "malformed tuning line: " + line);
-    set_value(name.c_str(), value);
+    if (!(ls >> value)) malformed = line;
+    else if (name == "format") format = value;
+    else entries.emplace_back(name, value);
   }
+  if (format < 1 || format > kFileFormat)
+    throw Error(BIPP_INVALID_PARAMETER_ERROR, "tuning file of an unknown format: " + std::to_string(format));
+  for (const auto& [name, value] : entries) {
+    check_value(name.c_str(), value);
+    const bool old = format < 2 && std::any_of(std::begin(kNewMeaning), std::end(kNewMeaning),
+                                               [&](const char* k) { return name == k; });
+    if (!old) set_value(name.c_str(), value);
+  }
+  if (!malformed.empty()) throw Error(BIPP_INVALID_PARAMETER_ERROR, "malformed tuning line: " + malformed);
 }
 
 void ensure_file_loaded() {
@@ -190,7 +212,7 @@ BippError bipp_tuning_save(const char* path) {
     ensure_file_loaded();
     std::ofstream out(path);
     require((bool)out, "cannot write the tuning file");
-    out << "# bipp_b200 tuned launch parameters (name value)\n";
+    out << "# bipp_b200 tuned launch parameters (name value)\nformat " << kFileFormat << "\n";
     for (const auto& p : table()) out << p.name << " " << p.value << "\n";
   });
 }

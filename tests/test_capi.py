@@ -176,6 +176,34 @@ def test_tuning_table_without_a_gpu(tmp_path):
     bipp.tuning_reset()
 
 
+def test_tuning_file_of_the_earlier_format(tmp_path):
+    """A file saved before hetrd.threads and tridiag.threads changed their meaning (threads of
+    a matrix's one CTA) has no format line: its other values are taken over, those two are
+    checked but not applied. Saved files name the format and come back whole."""
+    import bipp_b200 as bipp
+
+    f = tmp_path / "tune.txt"
+    old = "# bipp_b200 tuned launch parameters (name value)\nspread.items_cap 4096\nhetrd.threads 256\n" \
+          "hetrd.ctas_pct 75\ntridiag.threads 128\nvv.ctas_per_sm 2\n"
+
+    def load(text):
+        bipp.tuning_reset()
+        f.write_text(text)
+        bipp.tuning_load(str(f))
+        return [bipp.tuning_get(k) for k in ("spread.items_cap", "hetrd.threads", "hetrd.ctas_pct", "tridiag.threads",
+                                             "vv.ctas_per_sm")]
+
+    assert load(old) == [4096, 0, 75, 0, 2]
+    assert load(old + "format 2\n") == [4096, 256, 75, 128, 2]
+    bipp.tuning_save(str(f))
+    assert "format 2" in f.read_text().splitlines()
+    assert load(f.read_text()) == [4096, 256, 75, 128, 2]
+    for bad in ("hetrd.threads 300\n", "format 3\n", "tridiag.threads\n"):
+        with pytest.raises(bipp.InvalidParameterError):
+            load(bad)
+    bipp.tuning_reset()
+
+
 def test_cxx_shell_image_reduction_over_three_ranks(tmp_path):
     """The C++ API's Communicator::world() sums float arrays of three ranks (processes)
     into rank 0 over TCP, exactly; custom() runs the caller's reduction
