@@ -1,0 +1,105 @@
+"""Eigenvectors of the generalised eigensolver, judged one by one against the matrices they
+belong to: G-orthonormality and the residual of every pair."""
+import math
+
+import numpy as np
+import pytest
+import scipy.linalg
+
+gpu = pytest.mark.gpu
+
+
+def _failures(s, g, x, d, eps):
+    """Pairs of S x = d G x (columns of x, ascending d) outside their bounds, as text.
+
+    With L L^H = G and y = L^H x the solver works on C = L^-1 S L^-H in precision eps: its
+    orthogonal transformations and products leave errors of eps sqrt(n) normwise, taken 32
+    times. Orthonormality X^H G X = Y^H Y: the rounded L^-1 and the last product act on
+    columns of length ||L|| ||L^-1|| = sqrt(cond G); eigenvectors of the tridiagonal matrix,
+    found in FP64 from eigenvalues good to a rounding of the norm, are orthogonal to that
+    over their gap (and re-orthogonalised below gaps of 1e-10). Residual in the same frame,
+    L^-1 (S x - d G x) = C y - d y: relative to ||S|| ||G^-1||, the size of the terms of C."""
+    n = s.shape[0]
+    tol = 32 * eps * math.sqrt(n)
+    g = np.asarray(g, dtype=np.complex128)
+    low = np.linalg.cholesky(g)
+    y = low.conj().T @ x
+    gap = np.abs(d[:, None] - d[None])
+    gap64 = np.minimum(8 * np.finfo(np.float64).eps * np.abs(d).max() / np.maximum(gap, 1e-300), 1e-5)
+    np.fill_diagonal(gap64, 0.0)
+    orth = np.abs(y.conj().T @ y - np.eye(x.shape[1]))
+    bad = ["orthonormality %.2e at %s" % (orth[i, j], (i, j))
+           for i, j in zip(*np.nonzero(~(orth <= tol * math.sqrt(np.linalg.cond(g)) + gap64)))]
+    size = np.linalg.norm(s, 2) * np.linalg.norm(np.linalg.inv(g), 2)
+    res = np.linalg.norm(scipy.linalg.solve_triangular(low, s @ x - (g @ x) * d, lower=True), axis=0) / size
+    bad += ["residual %.2e of %d" % (res[i], i) for i in np.nonzero(~(res <= tol))[0]]
+    return bad
+
+
+def _antennas(rng, n):
+    """Positions with every pair at least half a wavelength (of 2) apart."""
+    side = int(math.ceil(math.sqrt(n)))
+    grid = np.stack(np.meshgrid(np.arange(side), np.arange(side)), -1).reshape(-1, 2)[:n] * 3.0
+    xyz = np.zeros((n, 3))
+    xyz[:, :2] = grid + rng.uniform(-0.9, 0.9, (n, 2))
+    return xyz
+
+
+def _sources(rng, xyz):
+    """Visibilities of 8 sources and noise, Hermitian."""
+    a = np.exp(1j * np.pi * xyz @ (rng.standard_normal((8, 3)) * 0.1).T)
+    noise = rng.standard_normal((len(xyz),) * 2) + 1j * rng.standard_normal((len(xyz),) * 2)
+    return (a * rng.uniform(1, 20, 8)) @ a.conj().T + 0.05 * (noise + noise.conj().T)
+
+
+def _gram(xyz):
+    return np.sinc(np.linalg.norm(xyz[:, None] - xyz[None], axis=2))
+
+
+def _hermitian(s):
+    s = np.tril(s).astype(np.complex128)
+    s = s + np.tril(s, -1).conj().T
+    np.fill_diagonal(s, s.diagonal().real)
+    return s
+
+
+@pytest.mark.parametrize("n", [2, 40, 129, 321])
+@pytest.mark.parametrize("eps", [np.finfo(np.float32).eps, np.finfo(np.float64).eps])
+def test_checks_see_wrong_vectors(n, eps):
+    """The checks pass for scipy's solution rounded to the precision and see a zero, a
+    repeated, a turned and an unnormalised eigenvector, of noise and of sources alike."""
+    rng = np.random.default_rng(n)
+    xyz = _antennas(rng, n)
+    s, g = _hermitian(_sources(rng, xyz)), _gram(xyz)
+    d, x = scipy.linalg.eigh(s, g)
+    if eps > 1e-10:
+        d, x = d.astype(np.float32).astype(np.float64), x.astype(np.complex64).astype(np.complex128)
+    assert not _failures(s, g, x, d, eps)
+    for i in (0, n // 2, n - 1):
+        for change in ("zero", "repeat", "turn", "scale"):
+            z = x.copy()
+            z[:, i] = {"zero": 0 * x[:, i], "repeat": x[:, i - 1], "turn": x[:, i] + 0.02 * x[:, i - 1],
+                       "scale": 1.02 * x[:, i]}[change]
+            assert _failures(s, g, z, d, eps), (i, change)
+
+
+@gpu
+@pytest.mark.parametrize("n,b", [(2, 3), (31, 2), (64, 2), (65, 1), (96, 40), (97, 3), (129, 1), (200, 2), (257, 1),
+                                 (300, 20), (321, 1), (513, 1), (130, 160)])
+@pytest.mark.parametrize("precision", ["single", "double"])
+def test_eigenvectors_of_batches(ctx, n, b, precision):
+    """W = I: single matrices on clusters of CTAs, batches on one CTA each."""
+    import bipp_b200 as bipp
+
+    dbl = precision == "double"
+    rng = np.random.default_rng(100 * n + b)
+    x0 = np.stack([_antennas(rng, n) for _ in range(min(b, 3))])
+    s0 = np.stack([_sources(rng, x) for x in x0]).astype(np.complex128 if dbl else np.complex64)
+    at = np.arange(b) % len(x0)
+    v, d, nred, _ = bipp.eigh_gram_batched(np.full(b, 2.0), s0[at], x0[at], ctx=ctx, precision=precision)
+    assert (nred == n).all()
+    for k in sorted({0, b // 2, b - 1}):
+        x = x0[at[k]] if dbl else x0[at[k]].astype(np.float32).astype(np.float64)
+        bad = _failures(_hermitian(s0[at[k]]), _gram(x), v[k].astype(np.complex128), d[k].astype(np.float64),
+                        np.finfo(np.float64 if dbl else np.float32).eps)
+        assert not bad, (k, len(bad), bad[:4])
