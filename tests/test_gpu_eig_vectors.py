@@ -103,3 +103,41 @@ def test_eigenvectors_of_batches(ctx, n, b, precision):
         bad = _failures(_hermitian(s0[at[k]]), _gram(x), v[k].astype(np.complex128), d[k].astype(np.float64),
                         np.finfo(np.float64 if dbl else np.float32).eps)
         assert not bad, (k, len(bad), bad[:4])
+
+
+@gpu
+@pytest.mark.parametrize("beams", [1, 2, 31, 63, 64, 65, 130])
+@pytest.mark.parametrize("flagged", [0, 1, 7])
+@pytest.mark.parametrize("double", [False, True])
+def test_beamformed_eigenvectors(ctx, beams, flagged, double):
+    """Orthonormal complex beams of more antennas than beams, some of them flagged: the
+    complex factor and inverse at and beside the 64 rows of its one-launch form."""
+    import bipp_b200 as bipp
+
+    if flagged >= beams:
+        pytest.skip("no beam left")
+    rng = np.random.default_rng(10 * beams + flagged)
+    rt, ct = (np.float64, np.complex128) if double else (np.float32, np.complex64)
+    n = beams + 20
+    xyz = _antennas(rng, n).astype(rt)
+    w = np.linalg.qr(rng.standard_normal((n, beams)) + 1j * rng.standard_normal((n, beams)))[0].astype(ct)
+    s = _sources(rng, xyz.astype(np.float64))
+    s = (w.conj().T @ s @ w).astype(ct)
+    off = rng.choice(beams, flagged, replace=False)
+    s[off] = 0
+    s[:, off] = 0
+    keep = np.setdiff1d(np.arange(beams), off)
+    v, d, nred, _ = bipp.eigh_gram_full(rt(2.0), s, w, xyz, ctx=ctx)
+    assert nred == len(keep)
+    wk = w[:, keep].astype(np.complex128)
+    g = wk.conj().T @ _gram(xyz.astype(np.float64)) @ wk
+    g = 0.5 * (g + g.conj().T)
+    sk = _hermitian(s[np.ix_(keep, keep)])
+    x = np.linalg.lstsq(wk, v[:, :nred].astype(np.complex128), rcond=None)[0]
+    eps = np.finfo(rt).eps
+    ref = scipy.linalg.eigh(sk, g, eigvals_only=True)
+    size = np.linalg.norm(sk, 2) * np.linalg.norm(np.linalg.inv(g), 2)
+    assert np.abs(d[:nred] - ref).max() <= 32 * eps * math.sqrt(nred) * size
+    assert not d[nred:].any() and not v[:, nred:].any()
+    bad = _failures(sk, g, x, d[:nred].astype(np.float64), eps)
+    assert not bad, (len(bad), bad[:4])
