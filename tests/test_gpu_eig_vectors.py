@@ -1,5 +1,6 @@
 """Eigenvectors of the generalised eigensolver, judged one by one against the matrices they
 belong to: G-orthonormality and the residual of every pair."""
+import ctypes as C
 import math
 
 import numpy as np
@@ -141,3 +142,32 @@ def test_beamformed_eigenvectors(ctx, beams, flagged, double):
     assert not d[nred:].any() and not v[:, nred:].any()
     bad = _failures(sk, g, x, d[:nred].astype(np.float64), eps)
     assert not bad, (len(bad), bad[:4])
+
+
+@gpu
+@pytest.mark.parametrize("double", [False, True])
+def test_batched_column_major_entries(ctx, double):
+    """bipp_eigh_gram_batched_s/_d take the matrices column-major, the _rows_ forms row-major:
+    the same results bit for bit, with flagged antennas and over two chunks of steps."""
+    import bipp_b200 as bipp
+    from bipp_b200._lib import check
+
+    rng = np.random.default_rng(5)
+    b, n = 300, 33
+    rt, ct = (np.float64, np.complex128) if double else (np.float32, np.complex64)
+    xyz = np.stack([_antennas(rng, n) for _ in range(b)]).astype(rt)
+    s = np.stack([_sources(rng, x.astype(np.float64)) for x in xyz]).astype(ct)
+    for k in range(0, b, 3):
+        off = rng.choice(n, 1 + k % 5, replace=False)
+        s[k][off] = 0
+        s[k][:, off] = 0
+    wl = np.full(b, 2.0, dtype=rt)
+    v, d, nred, scale = bipp.eigh_gram_batched(wl, s, xyz, ctx=ctx, precision="double" if double else "single")
+    fn = ctx._lib.bipp_eigh_gram_batched_d if double else ctx._lib.bipp_eigh_gram_batched_s
+    columns, pos = np.ascontiguousarray(s.transpose(0, 2, 1)), np.ascontiguousarray(xyz.transpose(0, 2, 1))
+    v2, d2 = np.empty((b, n, n), dtype=ct), np.empty((b, n), dtype=rt)
+    nred2, scale2 = np.empty(b, dtype=np.uint64), np.empty(b, dtype=rt)
+    check(fn(ctx.handle, b, n, *(a.ctypes.data_as(C.c_void_p) for a in (wl, columns, pos, d2, v2, nred2, scale2))))
+    assert np.array_equal(nred, nred2) and len(set(nred2.tolist())) > 3
+    assert np.array_equal(scale, scale2) and np.array_equal(d, d2)
+    assert np.array_equal(v, v2.transpose(0, 2, 1))
