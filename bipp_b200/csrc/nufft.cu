@@ -486,28 +486,32 @@ static void launch_spread(const NufftGeom& g, int nItems, size_t smem, cudaStrea
 
 // tensor-core spreading (4 or 8 channels): persistent CTAs, as many per SM as tensor
 // memory allows
-template <int CH, int STAGES, bool AT, bool F16>
+template <int CH, int STAGES, bool AT, bool F16, bool DRAIN = false>
 static void launch_spread_tc(const NufftGeom& g, int nItems, cudaStream_t st, const int* offs, const char* pts,
                              int stride, int ch0, int nch, const SpreadItem* items, int tw0, int slabPlanes, float2* out, int* errFlag, int* workCounter, const unsigned* valScale) {
-  using S = TcShape<CH, STAGES, AT, F16>;
+  using S = TcShape<CH, STAGES, AT, F16, DRAIN>;
   int dev = 0, sms = 148;
   B2_CUDA(cudaGetDevice(&dev));
   B2_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  smem_optin(spread_tc_kernel<CH, STAGES, AT, F16>, S::Smem);
+  smem_optin(spread_tc_kernel<CH, STAGES, AT, F16, DRAIN>, S::Smem);
   // never more CTAs per SM than tensor memory holds (a CTA beyond that would wait in its
   // allocation until another one exits)
   const int grid = std::max(1, std::min(nItems, sms * std::min(S::MinBlocks, tuned("spread.ctas_per_sm"))));
   count_launch();
-  spread_tc_kernel<CH, STAGES, AT, F16><<<grid, kTcThreads, S::Smem, st>>>(
+  spread_tc_kernel<CH, STAGES, AT, F16, DRAIN><<<grid, kTcThreads, S::Smem, st>>>(
       g, offs, pts, stride, ch0, nch, items, nItems, tw0, slabPlanes, out, errFlag, workCounter, valScale);
 }
 
 // BIPP_B200_SPREAD=warp selects the shared-memory-atomic spreader for every channel count.
-// More than 8 channels (four images with their first-order lattice channels: 12) take one
-// tensor-core launch of 8 and one of 4; the points' kernel values are then formed twice,
-// which still leaves the atomics of the other spreader far behind (1024^2 px, 16 x 512^2
-// points: 40.5 ms). Below a tolerance of 1e-5 the FP16 hi/lo operands show beside the
-// transform's own error (2 % of it at 1e-6, 0.02 % at 1e-5), so those keep FP32 sums.
+// More than 8 channels (three or four images with their first-order lattice channels) had FP32
+// products and sums there, and keep their precision on the tensor cores: the tf32 split, whose
+// lo parts hold their bits at any magnitude, and the accumulators drained into FP32 registers
+// every phase, in launches of 4 channels each. (Accumulated in tensor memory over a whole tile,
+// which cuts every addition off, images of point sources at a tolerance of 1e-5 were 9.4e-6 off
+// the FP64 sum against 6.7e-6; FP16 hi/lo operands alone lose 2-8 % where values span 1e3 or
+// more. So: 6.7e-6, within the repeats of the other spreader.) 1024^2 px, 16 x 512^2 points, 12
+// channels: 10.4 ms a transform, 43.7 with the atomics, 6.7 with neither of the two. Below a
+// tolerance of 1e-5, where 2^-22 of a product begins to show, the atomics stay.
 static bool use_tensor_core_spread(int nch, double eps) {
   const char* e = std::getenv("BIPP_B200_SPREAD");
   if (e && std::string(e) == "warp") return false;
@@ -564,6 +568,7 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
   // ones unless the pruned FFT, which reads by the tiles' bits, leaves them out; the warp
   // spreader works on a cleared slab
   const bool tc = use_tensor_core_spread(nch_, eps_);
+  const int groupCh = nch_ > kTcMaxChan ? 4 : kTcMaxChan;   // channels of a tensor-core launch
   const bool prunedFft = fftPlansOk_ && tuned("nufft.fft") == 1;
   const int tb = std::min(8192, (ntiles + 255) / 256);
   clearFlag_.ensure(ctx_, (size_t)ntiles * sizeof(int));
@@ -647,7 +652,7 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
     B2_CUDA(cudaMemcpyAsync(items_.get(), itemsAlt_.get(), (size_t)nItemsAll * sizeof(SpreadItem),
                             cudaMemcpyDeviceToDevice, ctx_->stream));
     // a counter per slab and channel group
-    const size_t counters = (size_t)std::max(1, nslab) * ((nch_ + kTcMaxChan - 1) / kTcMaxChan);
+    const size_t counters = (size_t)std::max(1, nslab) * ((nch_ + groupCh - 1) / groupCh);
     workCounters_.ensure(ctx_, counters * sizeof(int));
     B2_CUDA(cudaMemsetAsync(workCounters_.get(), 0, counters * sizeof(int), ctx_->stream));
   }
@@ -687,9 +692,10 @@ void NufftCore::execute(float* image, long long ldImage, double* stageMs) {
           {{launch_spread_tc<8, 1, false, false>, launch_spread_tc<8, 2, false, false>},
            {launch_spread_tc<8, 1, true, false>, launch_spread_tc<8, 2, true, false>},
            {launch_spread_tc<8, 1, false, true>, launch_spread_tc<8, 2, false, true>}}};
-      for (int c0 = 0, grp = 0; c0 < nch_; c0 += kTcMaxChan, ++grp) {
-        const int nc = std::min(kTcMaxChan, nch_ - c0);
-        const L launch = table[nc <= 4 ? 0 : 1][operands][two ? 1 : 0];
+      for (int c0 = 0, grp = 0; c0 < nch_; c0 += groupCh, ++grp) {
+        const int nc = std::min(groupCh, nch_ - c0);
+        const L launch = nch_ > kTcMaxChan ? launch_spread_tc<4, 2, false, false, true>
+                                           : table[nc <= 4 ? 0 : 1][operands][two ? 1 : 0];
         launch(g_, nItems, ctx_->stream, offsets_.get<int>(), pts_.get<char>(), pt_bytes(nch_), c0, nc,
                items_.get<SpreadItem>() + slabBegin[sl], tw0, slabPlanes,
                grid_.get<float2>() + slab_index(g_, nch_, slabPlanes, c0, 0, 0, 0), errFlag_.get<int>(),

@@ -26,7 +26,7 @@ constexpr int kTcThreads = 128;
 constexpr int kTcVisits = 16;                 // visits per phase
 constexpr int kTcSteps = kTcVisits / 8;       // MMA K-steps per phase (K = 8 for tf32)
 constexpr int kTcM = kTX * kTY;               // 128 accumulator rows (cells)
-constexpr int kTcMaxChan = 8;                 // channels of one launch of the tensor-core kernel
+constexpr int kTcMaxChan = 8;                 // channels of one launch of the tensor-core kernel (4 with DRAIN)
 // shared-memory layout (bytes); one K-step of A is 128 rows x 8 tf32
 constexpr int kTcAStep = kTcM * 8 * 4;
 // per-visit kernel values at every tile position (zero outside the support) and the
@@ -48,14 +48,19 @@ static_assert(kTX == 16 && kTY == 8 && kTW == 8 && kTcVisits == 16, "prep mappin
 // phase; half the operand bytes and MMAs of the tf32 split, so that two stages fit the
 // shared memory of 8 CTAs per SM). B is built from values scaled per channel into
 // [-1, 1] (FP16 range), the epilogue scales back.
+// DRAIN: every stage has an accumulator of its own, started anew by its phase and added to
+// FP32 sums in registers before the stage's next one. The tensor core cuts its additions off
+// instead of rounding, which over the hundreds of phases of a heavy tile adds up to 5e-6 of
+// the sums; drained, what is left is the rounding of FP32 additions.
 constexpr int tc_pow2_cols(int c) { return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : c <= 256 ? 256 : 512; }
-template <int CH, int STAGES = 1, bool AT = false, bool F16 = false>
+template <int CH, int STAGES = 1, bool AT = false, bool F16 = false, bool DRAIN = false>
 struct TcShape {
   static constexpr int N = kTW * 2 * CH;
   static constexpr int KSteps = F16 ? 1 : kTcSteps;              // MMA K-steps per phase
   static constexpr int AStageCols = AT ? 2 * kTcSteps * 8 : 0;   // A_hi, A_lo of a phase (K = 16 each)
-  static constexpr int AColBase = N;                             // A of stage s at AColBase + s AStageCols
-  static constexpr int Cols = tc_pow2_cols(N + STAGES * AStageCols);   // tensor-memory columns per CTA
+  static constexpr int AccCols = DRAIN ? STAGES * N : N;         // accumulators: one, or one per stage
+  static constexpr int AColBase = AccCols;                       // A of stage s at AColBase + s AStageCols
+  static constexpr int Cols = tc_pow2_cols(AccCols + STAGES * AStageCols);   // tensor-memory columns per CTA
   static constexpr int BStep = N * 8 * 4;
   static constexpr int OffAhi = 0;                // operands of stage 0; stage s at + s StageBytes
   static constexpr int OffAlo = OffAhi + (AT ? 0 : KSteps * kTcAStep);
@@ -77,6 +82,7 @@ struct TcShape {
   static_assert(N % 16 == 0 && N <= 256, "MMA N for M = 128");
   static_assert(OffEx % 1024 == 0, "operand blocks 1 KB aligned");
   static_assert(STAGES == 1 || STAGES == 2, "one or two operand stages");
+  static_assert(!DRAIN || (CH == 4 && !AT && !F16), "tf32 split; N sums per thread in registers");
   static_assert(MinBlocks >= 1 && MinBlocks * (Smem + 256 + 1024) <= 233472,
                 "shared memory (dynamic + static <= 256 B + 1 KB reserved) for MinBlocks CTAs per SM");
 };
@@ -117,17 +123,17 @@ __device__ __forceinline__ int tc_range_pair(int j) {
 }
 
 // The nch <= CH channels of one launch are consecutive ones of a point's, from ch0: more than
-// 8 channels are spread by several launches, valScale and grid pointing at
-// each launch's first channel.
+// 8 channels are spread by several launches, valScale and grid pointing at each launch's first
+// channel.
 // Persistent: each CTA takes work items blockIdx.x, blockIdx.x + gridDim.x, ... or, with
 // a work counter, the next item of the (load-ordered) list whenever it is free
-template <int CH, int STAGES, bool AT = false, bool F16 = false>
-static __global__ void __launch_bounds__(kTcThreads, TcShape<CH, STAGES, AT, F16>::MinBlocks)
+template <int CH, int STAGES, bool AT = false, bool F16 = false, bool DRAIN = false>
+static __global__ void __launch_bounds__(kTcThreads, TcShape<CH, STAGES, AT, F16, DRAIN>::MinBlocks)
 spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const char* __restrict__ pts, int stride, int ch0,
                  int nch, const SpreadItem* __restrict__ items,
                  int nItems, int tw0, int slabPlanes, float2* __restrict__ grid, int* __restrict__ errFlag,
                  int* __restrict__ workCounter, const unsigned* __restrict__ valScale = nullptr) {
-  using S = TcShape<CH, STAGES, AT, F16>;
+  using S = TcShape<CH, STAGES, AT, F16, DRAIN>;
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ __align__(8) uint64_t mbar[STAGES];   // MMA completion of the phases of each stage
   __shared__ uint32_t tmemSlot;
@@ -258,6 +264,23 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const char* __res
       }
     };
     fetch(0);
+    // DRAIN: this row's sums
+    float acc[DRAIN ? S::N : 1];
+    if constexpr (DRAIN) {
+#pragma unroll
+      for (int i = 0; i < S::N; ++i) acc[i] = 0.f;
+    }
+    auto drain = [&](int st) {
+      if constexpr (DRAIN) {
+#pragma unroll
+        for (int q = 0; q < S::N / 16; ++q) {
+          float r[16];
+          tmem_ld16(tmemWarp + (uint32_t)(st * S::N + q * 16), r);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[q * 16 + i] += r[i];
+        }
+      }
+    };
     for (int v0 = 0; v0 < nvis; v0 += kTcVisits) {
       const int nk = min(kTcVisits, nvis - v0);
       const int steps = F16 ? 1 : (nk + 7) >> 3;
@@ -311,8 +334,11 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const char* __res
       if (tid == 0 && !wait_stage(stg)) sOk = 0;
       if constexpr (AT) tc_fence_before();
       __syncthreads();
-      if constexpr (AT) tc_fence_after();   // the stage's tensor memory is free to rewrite
+      if constexpr (AT || DRAIN) tc_fence_after();   // the stage's tensor memory is free to rewrite or read
       if (!sOk) break;
+      if constexpr (DRAIN) {
+        if (v0 >= STAGES * kTcVisits) drain(stg);   // the sums of this stage's previous phase
+      }
       if (v0 + kTcVisits < nvis) fetch(v0 + kTcVisits);
       // A: row tid (cell xm, ym), 8 visits per K-step
       if constexpr (F16) {
@@ -422,10 +448,21 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const char* __res
         tmem_st_wait();
         tc_fence_before();
       }
+      if constexpr (DRAIN) tc_fence_before();   // the drained accumulator is free to rewrite
       __syncthreads();
       if (tid == 0) {
         tc_fence_after();
-        for (int s = 0; s < steps; ++s) {
+        if constexpr (DRAIN) {
+          // the small products first: the large ones are cut off once per K-step, not thrice
+          const uint32_t d = tmem + (uint32_t)(stg * S::N);
+          for (int t = 0; t < 3; ++t)
+            for (int s = 0; s < steps; ++s) {
+              const uint64_t dA = tc_desc(sstage + (t == 1 ? S::OffAlo : S::OffAhi) + s * kTcAStep, kTcAStep / 2, 128);
+              const uint64_t dB = tc_desc(sstage + (t == 0 ? S::OffBlo : S::OffBhi) + s * S::BStep, S::BStep / 2, 128);
+              tc_mma(d, dA, dB, S::Idesc, (t > 0 || s > 0) ? 1u : 0u);
+            }
+        }
+        for (int s = 0; s < (DRAIN ? 0 : steps); ++s) {
           const uint64_t dBh = tc_desc(sstage + S::OffBhi + s * S::BStep, S::BStep / 2, 128);
           const uint64_t dBl = tc_desc(sstage + S::OffBlo + s * S::BStep, S::BStep / 2, 128);
           if constexpr (F16) {
@@ -461,13 +498,23 @@ spread_tc_kernel(NufftGeom g, const int* __restrict__ offsets, const char* __res
     __syncthreads();
     tc_fence_after();
     if (!sOk) break;
+    if constexpr (DRAIN) {
+#pragma unroll
+      for (int st = 0; st < STAGES; ++st)
+        if (nvis > st * kTcVisits) drain(st);
+    }
     if (nvis > 0) {
       const int twl = tw - tw0;
       constexpr int PPB = 16 / (2 * CH);   // planes per 16-column block
 #pragma unroll
       for (int q = 0; q < S::N / 16; ++q) {
         float r[16];
-        tmem_ld16(tmemWarp + (uint32_t)(q * 16), r);
+        if constexpr (DRAIN) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = acc[q * 16 + i];
+        } else {
+          tmem_ld16(tmemWarp + (uint32_t)(q * 16), r);
+        }
 #pragma unroll
         for (int pl = 0; pl < PPB; ++pl) {
           const int plane = twl * kTW + q * PPB + pl;

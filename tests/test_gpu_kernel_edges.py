@@ -288,3 +288,62 @@ def test_direct_sum_double_phases(ctx, umax):
         plain.append((total(p) - ref) + (both.cumsum(1)[:, -1] - both.astype(ld).sum(1)))
         got.append(out - ref)
     assert np.sqrt(np.mean(np.square(got))) <= 1.1 * np.sqrt(np.mean(np.square(plain)))
+
+
+def _both_spreaders(ctx, monkeypatch, lmn, uvw, c, tol):
+    """Images of more than 8 channels by default and with the shared-memory atomics."""
+    import bipp_b200 as bipp
+
+    out = []
+    for warp in (False, True):
+        if warp:
+            monkeypatch.setenv("BIPP_B200_SPREAD", "warp")
+        plan = bipp.NufftSynthesis(ctx, bipp.NufftSynthesisOptions().set_tolerance(tol), lmn, c.shape[1], uvw.shape[0])
+        plan.add(uvw, c)
+        out.append(np.stack([plan.get_image(i) for i in range(c.shape[1])]).astype(np.float64))
+        plan.close()
+    return out
+
+
+@pytest.mark.parametrize("images,tol", [(3, 1e-5), (4, 1e-4), (4, 1e-5)])
+@pytest.mark.parametrize("values", ["sky", "noise", "heavy"])
+def test_more_than_eight_channels_keep_single_precision(ctx, monkeypatch, images, tol, values):
+    """9 and 12 channels on the tensor cores against the spreader with FP32 products and sums,
+    whose transform they share, so that only operands and sums differ: dropped products of
+    2^-22, FP32 additions on either side, 1e-6 (2^-20) in all. Heavy tiles of short baselines,
+    point sources whose values add up in phase, and values that span four decades."""
+    from bipp_b200 import simulate as sim
+
+    rng = np.random.default_rng(31)
+    n = 20000
+    lmn = sim.make_lmn_grid(64, math.radians(12.0)).astype(np.float32)
+    r, a = np.exp(rng.uniform(np.log(20), np.log(4000), n)), rng.uniform(0, 2 * np.pi, n)
+    uvw = np.stack([r * np.cos(a), r * np.sin(a), rng.uniform(-200, 200, n)], 1).astype(np.float32)
+    c = rng.standard_normal((n, images)) + 1j * rng.standard_normal((n, images))
+    if values == "sky":
+        lm = rng.uniform(-0.1, 0.1, (12, 2))
+        at = np.concatenate([lm, np.sqrt(1 - (lm ** 2).sum(1))[:, None]], 1)
+        c = np.exp(-1j * uvw.astype(np.float64) @ at.T) @ np.exp(rng.uniform(-4, 2, (12, images)))
+    elif values == "heavy":
+        c[20:] *= 1e-4
+    tc, warp = _both_spreaders(ctx, monkeypatch, lmn, uvw, c.astype(np.complex64), tol)
+    for i in range(images):
+        assert _rel_l2(tc[i], warp[i]) <= 1e-6, i
+    assert not np.array_equal(tc, warp)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 17, 32, 33, 48, 49, 2049, 5000])
+def test_more_than_eight_channels_point_counts(ctx, monkeypatch, n):
+    """Points of one place of the grid, so that its tiles get exactly n: phases that are not
+    full, one or two accumulators in use, tiles spread in parts. Bound as above, of the terms'
+    mean square (the same phase at every point lets an image's terms cancel)."""
+    from bipp_b200 import simulate as sim
+
+    rng = np.random.default_rng(n)
+    lmn = sim.make_lmn_grid(40, math.radians(12.0)).astype(np.float32)
+    uvw = (np.array([1234.0, -777.0, 111.0]) + rng.uniform(-0.5, 0.5, (n, 3))).astype(np.float32)
+    c = (rng.standard_normal((n, 4)) + 1j * rng.standard_normal((n, 4))).astype(np.complex64)
+    tc, warp = _both_spreaders(ctx, monkeypatch, lmn, uvw, c, 1e-5)
+    size = np.linalg.norm(c, axis=0) * math.sqrt(lmn.shape[0] / 2)
+    for i in range(4):
+        assert np.linalg.norm(tc[i] - warp[i]) <= 1e-6 * size[i], i
