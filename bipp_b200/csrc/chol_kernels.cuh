@@ -87,9 +87,10 @@ __device__ __forceinline__ void ct_each(double (&acc)[2][4][2], F f) {
 // too): 64 elimination steps on [D | X], each a pivot column scaled by every thread for itself
 // and one update of the entries to its right and of X, thread = row tid % 64, columns tid / 64
 // + 4 k. Bound by the chain of pivots (root, two barriers, update); for real blocks the
-// register form below is twice as fast. False when a pivot was not positive.
-template <typename E>
-__device__ __forceinline__ bool ct_eliminate(E* __restrict__ D, E* __restrict__ X, E* __restrict__ lcol) {
+// register form below is twice as fast, and complex ones take this. False when a pivot was not positive.
+__device__ __forceinline__ bool ct_eliminate(double2* __restrict__ D, double2* __restrict__ X,
+                                             double2* __restrict__ lcol) {
+  using E = double2;
   const int r = threadIdx.x % kCtB, g = threadIdx.x / kCtB;
   constexpr int G = kCtThreads / kCtB;
   bool ok = true;

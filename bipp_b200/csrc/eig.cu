@@ -235,7 +235,7 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
     smem_optin(k, smem);
     count_launch();
     k<<<nb, kPrepThreads, smem, st>>>(L.nBeam, L.S, L.sStride, L.lds, L.xyz, L.xyzStride, L.ldxyz, L.wl, L.mode,
-                                      L.eps, 0, Nmax, L.idx, L.nred, L.nvis, nullptr, nullptr, L.status, 1, 0,
+                                      L.eps, 0, Nmax, L.idx, L.nred, L.nvis, nullptr, nullptr, L.status, 0,
                                       L.batchOffset);
     B2_CHECK_LAUNCH();
   }
@@ -244,8 +244,9 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
     const int t = (Nmax + 31) / 32;
     count_launch();
     compact_kernel<T><<<dim3(t * (t + 1) / 2, nb), 256, 0, st>>>(L.S, L.sStride, L.lds, L.xyz, L.xyzStride, L.ldxyz, L.wl,
-                                                               (L.gram && L.identityW) ? 2 : 0, Nmax, L.idx, L.nred, A,
-                                                               G, L.batchOffset);
+                                                               Nmax, L.idx, L.nred, A,
+                                                               L.gram && L.identityW ? reinterpret_cast<double*>(G) : nullptr,
+                                                               L.batchOffset);
     B2_CHECK_LAUNCH();
   }
   if (L.gram && !L.identityW) {
@@ -284,13 +285,13 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
       B2_CHECK_LAUNCH();
       mark(2);
     } else {
-      auto k = cholesky_kernel<double2>;
+      auto k = cholesky_kernel;
       smem_optin(k, kCholSmem);
       count_launch();
       k<<<nb, kCholThreads, kCholSmem, st>>>(G, nred, Nmax, L.status + L.batchOffset, sizeOrder);
       B2_CHECK_LAUNCH();
       mark(2);
-      auto ki = trinv_kernel<double2, C>;
+      auto ki = trinv_kernel<C>;
       smem_optin(ki, kTrinvSmem);
       count_launch();
       ki<<<nb, 256, kTrinvSmem, st>>>(G, W64, Linv, nred, Nmax, sizeOrder);
@@ -598,7 +599,7 @@ static void eigh_host(bipp_ctx_s* ctx, bool gram, T wl, size_t nAntenna, size_t 
     count_launch();
     k<<<1, kPrepThreads, smem, ctx->stream>>>(F.nBeam, F.S, F.sStride, F.lds, F.xyz, F.xyzStride, F.ldxyz, F.wl,
                                               F.mode, F.eps, 0, Nmax, F.idx, F.nred, F.nvis,
-                                              work.A.template get<C>(), work.G.template get<double2>(), F.status, 1, 0, 0);
+                                              nullptr, nullptr, F.status, 0, 0);
     B2_CHECK_LAUNCH();
     int nr = 0;
     d2h(ctx, &nr, dNred.get(), sizeof(int));

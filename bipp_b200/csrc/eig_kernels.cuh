@@ -1,18 +1,23 @@
 // Batched generalized Hermitian eigensolver kernels (sm_100a).
 //
-// Pipeline per matrix b of a batch (sizes vary per matrix after flagging):
-//   prep_kernel        flag non-zero rows/cols of S, compact S -> A (working precision),
-//                      Gram G_ij = sinc(2|p_i-p_j|/wl) -> G (FP64)       [src/eigensolver.cpp:148-207,
-//                                                                          src/host/gram_matrix.cpp:23-56]
-//   cholesky_kernel    G = L L^H in FP64                                   [LAPACK potrf inside ?hegv]
-//   trinv_kernel       Linv = L^-1 in FP64, rounded to working precision
-//   gemm_kernel        C = Linv S Linv^H (two triangular products)         [hegst]
-//   hetrd_kernel       C = Q T Q^H, T real tridiagonal (Householder)        [hetrd]
-//   tridiag_kernel     eigenpairs of T in FP64: bisection + twisted factorisation
-//   backtransform      Y = Q Z                                              [unmtr]
-//   gemm_kernel        X = Linv^H Y                                         [trsm back-transform]
-// One CTA owns one matrix in the sequential stages; matrices live in HBM with
-// leading dimension Nmax (the batch's padded size).
+// Pipeline of a batch (sizes vary per matrix after flagging), with the file of each kernel
+// where it is not this one:
+//   prep_kernel        flag non-zero rows/cols of S                        [src/eigensolver.cpp:148-207]
+//   compact_kernel     S compacted -> A (working precision), W = I: Gram matrix G_ij =
+//                      sinc(2|p_i-p_j|/wl) -> G (FP64 reals)               [src/host/gram_matrix.cpp:23-56]
+//   chol_kernels.cuh   G = L L^H in FP64, Linv = L^-1 rounded to working precision
+//                      (cholesky_kernel, trinv_kernel: general W above 64 beams)
+//                                                                          [LAPACK potrf inside ?hegv]
+//   gemm_kernel        C = Linv S Linv^H (two triangular products; gemm_tc.cuh in FP32)   [hegst]
+//   hetrd_kernels.cuh  C = Q T Q^H, T real tridiagonal (Householder; hetrd_blk_kernel and
+//                      hetrd_kernel where that says so)                    [hetrd]
+//   tridiag_kernels.cuh eigenpairs of T in FP64: bisection + twisted factorisation
+//                      (tridiag_kernel: the predicted partial solve)
+//   bt_*_kernel        Y = Q Z                                             [unmtr]
+//   gemm_kernel        X = Linv^H Y                                        [trsm back-transform]
+// The allocation-free entry point runs the one-CTA-per-matrix kernels of this file alone
+// (prep_kernel then compacts and forms G too). Matrices live in HBM with leading dimension
+// Nmax (the batch's padded size).
 #pragma once
 
 #include "common.cuh"
@@ -33,7 +38,7 @@ prep_kernel(int nBeam, const typename Cplx<T>::type* __restrict__ S, long long s
             const double* __restrict__ wl, int mode, T eps, int withGram, int Nmax,
             int* __restrict__ idxOut, int* __restrict__ nredOut, long long* __restrict__ nvisOut,
             typename Cplx<T>::type* __restrict__ A, double2* __restrict__ G, int* __restrict__ status,
-            int doFlag, int doCompact, int batchOffset) {
+            int doCompact, int batchOffset) {
   using C = typename Cplx<T>::type;
   extern __shared__ int smem_i[];
   int* flags = smem_i;                 // [Nmax]
@@ -44,7 +49,7 @@ prep_kernel(int nBeam, const typename Cplx<T>::type* __restrict__ S, long long s
   const int bg = b + batchOffset;           // matrix within the flag/index arrays
   const C* Sb = S + b * sStride;
   int* idxB = idxOut + (long long)bg * Nmax;
-  if (doFlag) {
+  {
     for (int i = threadIdx.x; i < nBeam; i += blockDim.x) flags[i] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
@@ -101,11 +106,6 @@ prep_kernel(int nBeam, const typename Cplx<T>::type* __restrict__ S, long long s
       nvisOut[bg] = nvis;
     }
     for (int i = threadIdx.x; i < s_nred; i += blockDim.x) idxB[i] = idx[i];
-  } else {
-    if (threadIdx.x == 0) s_nred = nredOut[bg];
-    __syncthreads();
-    for (int i = threadIdx.x; i < s_nred; i += blockDim.x) idx[i] = idxB[i];
-    __syncthreads();
   }
   if (!doCompact) return;
   const int nr = s_nred;
@@ -150,14 +150,13 @@ prep_kernel(int nBeam, const typename Cplx<T>::type* __restrict__ S, long long s
 // sinc(2 |p_i - p_j| / wl); the conjugate upper triangle of A goes out through shared memory.
 // Bound by the FP64 sine, root and quotient of G and by reading S through the index. One CTA
 // per matrix, with 64-bit divisions per element and an uncoalesced upper triangle, took 5.0 ms
-// for 2048 matrices of 380-512 rows and 0.50 for one of 550. gram: 0 none, 1 complex
-// storage, 2 real storage.
+// for 2048 matrices of 380-512 rows and 0.50 for one of 550. G may be null: no Gram matrix.
 template <typename T>
 __global__ void __launch_bounds__(256)
 compact_kernel(const typename Cplx<T>::type* __restrict__ S, long long sStride, int lds, const double* __restrict__ xyz,
-               long long xyzStride, int ldxyz, const double* __restrict__ wl, int gram, int Nmax,
+               long long xyzStride, int ldxyz, const double* __restrict__ wl, int Nmax,
                const int* __restrict__ idx, const int* __restrict__ nred, typename Cplx<T>::type* __restrict__ A,
-               double2* __restrict__ G, int batchOffset) {
+               double* __restrict__ G, int batchOffset) {
   using C = typename Cplx<T>::type;
   __shared__ C tile[32][33];
   __shared__ int id[2][32];
@@ -173,13 +172,13 @@ compact_kernel(const typename Cplx<T>::type* __restrict__ S, long long sStride, 
     const int k = (y ? c0 : r0) + x;
     const int i = k < n ? idx[(long long)bg * Nmax + k] : 0;
     id[y][x] = i;
-    if (gram)
+    if (G)
       for (int c = 0; c < 3; ++c) pos[y][c][x] = xyz[bg * xyzStride + i + (long long)c * ldxyz];
   }
   __syncthreads();
   const C* Sb = S + b * sStride;
   C* Ab = A + (long long)b * Nmax * Nmax;
-  const double w = gram ? wl[bg] : 1.0;
+  const double w = G ? wl[bg] : 1.0;
   const int r = r0 + x;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -190,7 +189,7 @@ compact_kernel(const typename Cplx<T>::type* __restrict__ S, long long sStride, 
       tile[cc][x] = v;
       const long long at = (long long)b * Nmax * Nmax + r + (long long)c * Nmax;
       A[at] = v;
-      if (gram) {
+      if (G) {
         double g = 1.0;
         if (r != c) {
           const double dx = pos[0][0][x] - pos[1][0][cc], dy = pos[0][1][x] - pos[1][1][cc],
@@ -198,10 +197,7 @@ compact_kernel(const typename Cplx<T>::type* __restrict__ S, long long sStride, 
           const double q = 2.0 * sqrt(dx * dx + dy * dy + dz * dz) / w;
           g = (q != 0.0) ? sinpi(q) / (3.14159265358979323846 * q) : 1.0;
         }
-        if (gram == 2)
-          reinterpret_cast<double*>(G)[at] = g;
-        else
-          G[at] = make_double2(g, 0.0);
+        G[at] = g;
       }
     }
   }
@@ -219,58 +215,47 @@ compact_kernel(const typename Cplx<T>::type* __restrict__ S, long long sStride, 
 constexpr int kCholNB = 32;
 constexpr int kCholThreads = 256;
 // shared memory: diagonal block D, its inverse Dinv, and two 64-row panel tiles
-template <typename E>
-constexpr size_t chol_smem() { return (size_t)(2 * kCholNB + 128) * (kCholNB + 1) * sizeof(E); }
-constexpr size_t kCholSmem = chol_smem<double2>();
+constexpr size_t kCholSmem = (size_t)(2 * kCholNB + 128) * (kCholNB + 1) * sizeof(double2);
 
-// FP64 element helpers: E = double2 (complex Hermitian G) or double (real symmetric G,
-// identity beamforming)
+// FP64 element helpers (E = double2, complex Hermitian G; chol_kernels.cuh also E = double)
 template <typename E> __device__ __forceinline__ E e_zero();
 template <> __device__ __forceinline__ double2 e_zero<double2>() { return make_double2(0.0, 0.0); }
 template <> __device__ __forceinline__ double e_zero<double>() { return 0.0; }
 __device__ __forceinline__ double e_re(double2 a) { return a.x; }
-__device__ __forceinline__ double e_re(double a) { return a; }
 __device__ __forceinline__ double2 e_real(double2, double v) { return make_double2(v, 0.0); }
 __device__ __forceinline__ double e_real(double, double v) { return v; }
 __device__ __forceinline__ double2 e_scale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-__device__ __forceinline__ double e_scale(double a, double s) { return a * s; }
 __device__ __forceinline__ double2 e_neg(double2 a) { return make_double2(-a.x, -a.y); }
-__device__ __forceinline__ double e_neg(double a) { return -a; }
 // acc -= a conj(b)
 __device__ __forceinline__ void e_sub_mulc(double2& acc, double2 a, double2 b) {
   acc.x -= a.x * b.x + a.y * b.y;
   acc.y -= a.y * b.x - a.x * b.y;
 }
-__device__ __forceinline__ void e_sub_mulc(double& acc, double a, double b) { acc -= a * b; }
 // acc -= a b
 __device__ __forceinline__ void e_sub_mul(double2& acc, double2 a, double2 b) {
   acc.x -= a.x * b.x - a.y * b.y;
   acc.y -= a.x * b.y + a.y * b.x;
 }
-__device__ __forceinline__ void e_sub_mul(double& acc, double a, double b) { acc -= a * b; }
 // acc += a conj(b)
 __device__ __forceinline__ void e_add_mulc(double2& acc, double2 a, double2 b) {
   acc.x += a.x * b.x + a.y * b.y;
   acc.y += a.y * b.x - a.x * b.y;
 }
-__device__ __forceinline__ void e_add_mulc(double& acc, double a, double b) { acc += a * b; }
 // acc += a b
 __device__ __forceinline__ void e_add_mul(double2& acc, double2 a, double2 b) { cfma(acc, a, b); }
-__device__ __forceinline__ void e_add_mul(double& acc, double a, double b) { acc += a * b; }
 // a / d
 __device__ __forceinline__ double2 e_div(double2 a, double2 d) {
   const double den = d.x * d.x + d.y * d.y;
   return make_double2((a.x * d.x + a.y * d.y) / den, (a.y * d.x - a.x * d.y) / den);
 }
-__device__ __forceinline__ double e_div(double a, double d) { return a / d; }
 
 // Panel rows below the diagonal block are X = A L_kk^-H with L_kk^-1 formed in shared
 // memory (as the triangular inverse does per block). For the Gram matrices of general
 // beamforming above 64 beams and the allocation-free entry point.
-template <typename E>
-__global__ void __launch_bounds__(kCholThreads)
-cholesky_kernel(E* __restrict__ G, const int* __restrict__ nred, int Nmax, int* __restrict__ status,
+static __global__ void __launch_bounds__(kCholThreads)
+cholesky_kernel(double2* __restrict__ G, const int* __restrict__ nred, int Nmax, int* __restrict__ status,
                 const int* __restrict__ order = nullptr) {
+  using E = double2;
   const int b = order ? order[blockIdx.x] : blockIdx.x;
   const int n = nred[b];
   E* Gb = G + (long long)b * Nmax * Nmax;
@@ -435,14 +420,13 @@ __device__ __forceinline__ void store_conv(double* p, double v) { *p = v; }
 // Linv[I,J] = -Linv[I,I] sum_{K=J}^{I-1} L[I,K] Linv[K,J]. The FP64 inverse goes to W64
 // (read back for the later block rows) and, rounded, to LinvOut. O = the
 // working-precision output element.
-template <typename E>
-constexpr size_t trinv_smem() { return 3 * 32 * 33 * sizeof(E); }
-constexpr size_t kTrinvSmem = trinv_smem<double2>();
+constexpr size_t kTrinvSmem = 3 * 32 * 33 * sizeof(double2);
 
-template <typename E, typename O>
+template <typename O>
 __global__ void __launch_bounds__(256)
-trinv_kernel(const E* __restrict__ L, E* __restrict__ W64, O* __restrict__ LinvOut, const int* __restrict__ nred,
-             int Nmax, const int* __restrict__ order = nullptr) {
+trinv_kernel(const double2* __restrict__ L, double2* __restrict__ W64, O* __restrict__ LinvOut,
+             const int* __restrict__ nred, int Nmax, const int* __restrict__ order = nullptr) {
+  using E = double2;
   constexpr int NB = 32;
   const int b = order ? order[blockIdx.x] : blockIdx.x;
   const int n = nred[b];
@@ -1667,7 +1651,7 @@ backtransform_kernel(const C* __restrict__ A, const C* __restrict__ taus, const 
 // (one CTA per block and matrix); bt_apply_kernel keeps a 16-column slice of Y in
 // registers (thread: one column, every 16th row) for all blocks. A block of V is read by a
 // warp per reflector (no division per element), and the partial sums of V^H Y over a warp's
-// row groups are added by exchanges that halve what each lane keeps, 8 instead of 24 shuffles
+// row groups are added by exchanges that halve what each lane keeps, 7 instead of 24 shuffles
 // of a value: 2048 complex FP32 matrices of 512 rows 26.5 -> 22.1 ms, 64 of 1024 rows
 // 6.3 -> 4.7 ms, 256 of 256 rows 0.77 -> 0.62 ms.
 constexpr int kBtNB = 16;             // reflectors per block

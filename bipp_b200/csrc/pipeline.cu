@@ -408,7 +408,7 @@ static void pipeline_process(bipp_pipeline_s* p, size_t nSteps, const void* s, c
     k<<<T, kPrepThreads, smem, ctx->stream>>>(N, p->Sin, n2, N, p->xyzT.get<double>(), 3ll * N, N,
                                               p->wl.get<double>(), 0, std::numeric_limits<float>::epsilon(), 1, N,
                                               p->idx.get<int>(), p->nred.get<int>(), p->nvis.get<long long>(),
-                                              nullptr, nullptr, p->status.get<int>(), 1, 0, 0);
+                                              nullptr, nullptr, p->status.get<int>(), 0, 0);
     B2_CHECK_LAUNCH();
   }
   std::vector<int> nredH(T);
