@@ -326,8 +326,8 @@ def spread_roofline(stats, spread_ms, n_levels):
             "peak_source": label, "traffic": traffic, "algorithmic_bytes_per_launch": int(per_launch),
             "launches_per_step": slabs, "launch_ms": round(dur_s * 1000.0, 3),
             "flops_per_launch": int(flops), "achieved_tflops": round(flops / dur_s / 1e12, 3),
-            "note": spread_operands_note() + "; bound by building the dense operands (latency at "
-                    "32 warps per SM), the HBM fraction is its floor"}
+            "note": spread_operands_note() + "; bound by building the dense operands (the shared-memory "
+                    "pipe at 32 warps per SM), the HBM fraction is its floor"}
 
 
 def spread_operands_note():
@@ -586,7 +586,7 @@ def main():
             parity = verify.check_batch(ctx, S[sel].contiguous(), xyz[sel].contiguous(), wl[sel].contiguous(), obs,
                                         n, intervals, cfg.eps, n_pix=args.check_pixels,
                                         chunk_steps=min(args.chunk_steps, len(sel)), vv_precision=args.vv_precision)
-            parity["reference"] = ("FP64: bipp_eigh_gram_batched_d + FP64 V diag(d) V^H + direct sum with FP64 "
+            parity["reference"] = ("FP64: bipp_eigh_gram_batched_rows_d + FP64 V diag(d) V^H + direct sum with FP64 "
                                    "phase and trigonometry (the library's FP64 pieces pinned to the compiled "
                                    "reference)")
         except bipp.GPUError as err:

@@ -15,7 +15,9 @@
 //                  the block below the diagonal of each pair is -X22 (L21 X11), two launches
 //                  per level and log2(n / 64) levels
 // The products run on the FP64 tensor instruction (m8n8k4; 256 multiply-adds per issue, 6
-// shared-memory loads per 8 of them), which is bound by the FP64 pipe rather than by loads.
+// shared-memory loads per 8 of them). In a batch of 128 matrices of 380-512 rows that pipe is
+// 60-65 % busy in the inverse, 29 % in the trailing update, whose tile loads precede each
+// product without overlap and one of whose CTAs goes on through a chain of pivots.
 // All arithmetic and accumulation is FP64 as before.
 #pragma once
 

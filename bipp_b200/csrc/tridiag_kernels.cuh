@@ -19,6 +19,10 @@
 //    more lanes only repeat work when the batch fills it already;
 //  - the two factorisations of an eigenvector, from the top and from the bottom, run in two
 //    lanes at once, their quotients off the chain.
+// One matrix of 550 rows takes 0.46 ms, 64 of 256 0.37, 512 of 380-512 2.4 for all three
+// launches; in 128 of 380-512 the search is bound by the latency of its recurrence and the
+// integer comparisons around it, the eigenvectors by reading their quotients back with the few
+// lanes that the level range leaves (profiled at 41 % and 19 % of the issue slots).
 #pragma once
 
 #include "common.cuh"

@@ -4,7 +4,7 @@ The FP32 pipeline (the form the benchmark times) images a batch of time steps; t
 same steps are then imaged in FP64 by this library's own FP64 pieces, each pinned to
 the reference's CPU code by the parity tests:
 
-- eigenpairs: ``bipp_eigh_gram_batched_d`` (the reference's eigh_gram<double>, i.e.
+- eigenpairs: ``bipp_eigh_gram_batched_rows_d`` (the reference's eigh_gram<double>, i.e.
   zhegv after flagging, src/eigensolver.cpp:129-225);
 - virtual visibilities: VV_l = V diag(scale * d * [lo_l <= d <= hi_l]) V^H in FP64
   (src/host/virtual_vis.cpp:19-73, the level mask of python/bipp/filter.py:45-47);

@@ -404,6 +404,8 @@ BIPP_B200_EXPORT BippError bipp_autotune_pipeline(bipp_pipeline_t pl, size_t nSt
 /* The tuning table: get or set one parameter (a value outside its candidates fails with
  * BIPP_INVALID_PARAMETER_ERROR), describe all (one line each: name, value, candidates,
  * meaning), save to or load from a file of "name value" lines, or reset to the defaults.
+ * Saved files carry a "format 2" line; in files without it hetrd.threads and
+ * tridiag.threads, whose meaning has changed, are checked but not applied.
  * BIPP_B200_TUNING_FILE, when set, is loaded on first use. No device is needed. */
 BIPP_B200_EXPORT BippError bipp_tuning_get(const char* name, int* value);
 BIPP_B200_EXPORT BippError bipp_tuning_set(const char* name, int value);
