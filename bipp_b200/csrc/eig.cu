@@ -428,9 +428,14 @@ void eig_launch(bipp_ctx_s* ctx, const EigLaunch<T>& L, EigWork<T>& w) {
         w.d.template get<double>(), w.e.template get<double>(), nred, Nmax, lam, L.vecLo, L.vecHi, range, krange, Z,
         reinterpret_cast<double*>(W64), sizeOrder);
     B2_CHECK_LAUNCH();
+  }
+  {
+    const size_t smem = (size_t)Nmax * sizeof(double);
+    smem_optin(tridiag_clusters_kernel<R>, smem);
     count_launch();
-    tridiag_clusters_kernel<R><<<nb, 256, 0, st>>>(w.d.template get<double>(), w.e.template get<double>(), nred, Nmax,
-                                                   lam, krange, Z, L.status + L.batchOffset);
+    tridiag_clusters_kernel<R><<<nb, 256, smem, st>>>(w.d.template get<double>(), w.e.template get<double>(), nred, Nmax,
+                                                      lam, krange, Z, reinterpret_cast<double*>(W64),
+                                                      L.status + L.batchOffset);
     B2_CHECK_LAUNCH();
   }
   // 5. back-transform Y = Q Z -> T1

@@ -12,7 +12,7 @@
 //   hetrd_kernels.cuh  C = Q T Q^H, T real tridiagonal (Householder; hetrd_blk_kernel and
 //                      hetrd_kernel where that says so)                    [hetrd]
 //   tridiag_kernels.cuh eigenpairs of T in FP64: bisection + twisted factorisation
-//                      (tridiag_kernel: the predicted partial solve)
+//                      (tridiag_kernel: the predicted partial solve; clusters there too)
 //   bt_*_kernel        Y = Q Z                                             [unmtr]
 //   gemm_kernel        X = Linv^H Y                                        [trsm back-transform]
 // The allocation-free entry point runs the one-CTA-per-matrix kernels of this file alone
@@ -1540,42 +1540,6 @@ tridiag_kernel(const double* __restrict__ dIn, const double* __restrict__ eIn, c
       if (threadIdx.x == 0 && krange) krange[2 * b] = 0;
       __syncthreads();
     }
-  }
-  // re-orthogonalise tight clusters (relative gap below 1e-10 of |T|): modified
-  // Gram-Schmidt inside each cluster, in eigenvalue order.
-  const double ctol = 1e-10 * fmax(tnorm, 1e-300);
-  __shared__ int s_any;
-  if (threadIdx.x == 0) {
-    int any = 0;
-    for (int i = kLo + 1; i < kHi; ++i) any |= (lam[i] - lam[i - 1] < ctol);
-    s_any = any;
-  }
-  __syncthreads();
-  if (!s_any) return;
-  if (threadIdx.x == 0) atomicOr(status + b, (int)kStatusClusterFix);
-  for (int i = kLo + 1; i < kHi; ++i) {
-    if (!(lam[i] - lam[i - 1] < ctol)) continue;
-    int j0 = i - 1;
-    while (j0 > kLo && lam[j0] - lam[j0 - 1] < ctol) --j0;
-    for (int j = j0; j < i; ++j) {
-      double part = 0.0;
-      for (int k = threadIdx.x; k < n; k += blockDim.x)
-        part += (double)Zb[(long long)k * Nmax + i] * (double)Zb[(long long)k * Nmax + j];
-      const double dot = block_sum(part, red);
-      for (int k = threadIdx.x; k < n; k += blockDim.x)
-        Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] - dot * (double)Zb[(long long)k * Nmax + j]);
-      __syncthreads();
-    }
-    double part = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      const double zv = (double)Zb[(long long)k * Nmax + i];
-      part += zv * zv;
-    }
-    const double nr = sqrt(block_sum(part, red));
-    const double inv = nr > 0 ? 1.0 / nr : 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x)
-      Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] * inv);
-    __syncthreads();
   }
 }
 

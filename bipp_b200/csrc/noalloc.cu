@@ -15,6 +15,7 @@
 #include "bipp_b200.h"
 #include "context.hpp"
 #include "eig_kernels.cuh"
+#include "tridiag_kernels.cuh"
 
 namespace bippb200 {
 namespace {
@@ -191,6 +192,8 @@ extern "C" BippError bipp_eigh_gram_noalloc_s(int device, void* stream, float wl
       smem_optin(tridiag_kernel<float>, smem);
       tridiag_kernel<float><<<1, kTriThreads, smem, st>>>(w.d, w.e, nred, N, lam, w.Z,
                                                            reinterpret_cast<double*>(w.W64), status);
+      tridiag_clusters_kernel<float><<<1, 256, (size_t)N * sizeof(double), st>>>(
+          w.d, w.e, nred, N, lam, nullptr, w.Z, reinterpret_cast<double*>(w.W64), status);
     }
     {
       const size_t smem = ((size_t)N * 16 + N + kBtThreads) * sizeof(float2);

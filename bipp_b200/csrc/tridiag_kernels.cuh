@@ -114,7 +114,7 @@ __device__ __forceinline__ void ts_load(const double* __restrict__ d, const doub
 // two Sturm counts give; the others come out as zero. CTA (c, r): chunk c of
 // kTsThreads / M eigenvalues of the matrix of rank r in `order`. range[2b], range[2b+1]:
 // the index range. Dynamic shared memory: Nmax double2.
-__global__ void __launch_bounds__(kTsThreads)
+static __global__ void __launch_bounds__(kTsThreads)
 tridiag_values_kernel(const double* __restrict__ dIn, const double* __restrict__ eIn, const int* __restrict__ nred,
                       int Nmax, double vecLo, double vecHi, int allValues, int M, double* __restrict__ lamOut,
                       int* __restrict__ range, const int* __restrict__ order) {
@@ -340,53 +340,164 @@ tridiag_vectors_kernel(const double* __restrict__ dIn, const double* __restrict_
   }
 }
 
-// Clusters (neighbours closer than 1e-10 of the norm): modified Gram-Schmidt inside each,
-// in eigenvalue order. One CTA per matrix, which returns at once when there is none.
+// fixed pseudo-random number in (-1, 1) for row k of eigenvector i (multiply-and-shift mixing)
+__device__ __forceinline__ double ts_random(int i, int k) {
+  unsigned h = (unsigned)i * 0x9e3779b1u ^ ((unsigned)k + 1u) * 0x85ebca77u;
+  h ^= h >> 15;
+  h *= 0x2c1b3c6du;
+  h ^= h >> 12;
+  h *= 0x297a2d39u;
+  h ^= h >> 15;
+  return ((double)(int)h + 0.5) * 4.656612873077393e-10;   // 2^-31
+}
+
+// One step of inverse iteration: z <- (T - l)^-1 z, normalised, or, at the start, of a vector of
+// its own, by Gaussian elimination with partial pivoting (row k of U: u0, u1, u2) and pivots of
+// at least `tiny`. One thread; at(a, k): its workspace, a = 0..2 the rows of U, 3 the
+// right-hand side and the solution.
+template <typename R, typename At>
+__device__ __forceinline__ void ts_inverse_step(const double* __restrict__ d, const double* __restrict__ e, int n,
+                                                double l, double tiny, bool start, int i, At at, R* __restrict__ z,
+                                                long long ldz) {
+  auto rhs = [&](int k) { return start ? ts_random(i, k) : (double)z[(long long)k * ldz]; };
+  double a = d[0] - l, b = n > 1 ? e[0] : 0.0, r = rhs(0);
+  for (int k = 0; k < n - 1; ++k) {
+    const double s = e[k], q = d[k + 1] - l, t = k + 2 < n ? e[k + 1] : 0.0, rn = rhs(k + 1);
+    if (fabs(a) >= fabs(s)) {
+      if (fabs(a) < tiny) a = copysign(tiny, a);
+      const double m = s / a;
+      at(0, k) = a;
+      at(1, k) = b;
+      at(2, k) = 0.0;
+      at(3, k) = r;
+      a = fma(-m, b, q);
+      b = t;
+      r = fma(-m, r, rn);
+    } else {
+      const double m = a / s;
+      at(0, k) = fabs(s) < tiny ? copysign(tiny, s) : s;
+      at(1, k) = q;
+      at(2, k) = t;
+      at(3, k) = rn;
+      a = fma(-m, q, b);
+      b = -m * t;
+      r = fma(-m, rn, r);
+    }
+  }
+  at(0, n - 1) = fabs(a) < tiny ? copysign(tiny, a) : a;
+  at(1, n - 1) = at(2, n - 1) = 0.0;
+  at(3, n - 1) = r;
+  double x1 = 0.0, x2 = 0.0, big = 0.0, f = 1.0;
+  for (int k = n - 1; k >= 0; --k) {
+    double x = (at(3, k) * f - at(1, k) * x1 - at(2, k) * x2) / at(0, k);
+    if (fabs(x) > 1e150) {   // several vanishing pivots in a row
+      x *= 1e-150;
+      x1 *= 1e-150;
+      f *= 1e-150;
+      big *= 1e-150;
+      for (int j = k + 1; j < n; ++j) at(3, j) *= 1e-150;
+    }
+    at(3, k) = x;
+    big = fmax(big, fabs(x));
+    x2 = x1;
+    x1 = x;
+  }
+  const double scale = big > 0.0 ? 1.0 / big : 1.0;
+  double norm2 = 0.0;
+  for (int k = 0; k < n; ++k) {
+    const double x = at(3, k) * scale;
+    norm2 = fma(x, x, norm2);
+  }
+  const double inv = scale / sqrt(norm2);
+  for (int k = 0; k < n; ++k) z[(long long)k * ldz] = (R)(at(3, k) * inv);
+}
+
+// Clusters: runs of eigenvalues whose neighbours are closer than 1e-10 of the norm. Twisted
+// factorisations at equal eigenvalues give the same vector, so the members are found anew: a
+// step of inverse iteration from vectors of their own, one thread each, orthogonalised in
+// eigenvalue order (classical Gram-Schmidt, twice), and both once more, since the first
+// orthogonalisation of unrelated vectors enlarges what they hold of other eigenvectors. The
+// shift lies 8 roundings of the norm beside the eigenvalue: at equal eigenvalues, which come
+// out a rounding apart, every direction of their space is then enlarged alike. One CTA per
+// matrix, which returns at once when it has no cluster. work: 2 Nmax^2 doubles per matrix. krange null: all n. Dynamic
+// shared memory: Nmax doubles.
 template <typename R>
 __global__ void __launch_bounds__(256)
 tridiag_clusters_kernel(const double* __restrict__ dIn, const double* __restrict__ eIn, const int* __restrict__ nred,
                         int Nmax, const double* __restrict__ lamIn, const int* __restrict__ krange, R* __restrict__ Z,
-                        int* __restrict__ status) {
+                        double* __restrict__ work, int* __restrict__ status) {
   const int b = blockIdx.x;
   const int n = nred[b];
   if (n <= 0) return;
-  __shared__ double red[32];
+  extern __shared__ __align__(16) double ts_dots[];
+  __shared__ double red[32], part[8][33];
   const double* d = dIn + (long long)b * Nmax;
   const double* e = eIn + (long long)b * Nmax;
   const double* lam = lamIn + (long long)b * Nmax;
   R* Zb = Z + (long long)b * Nmax * Nmax;
-  const int kLo = krange[2 * b], kHi = krange[2 * b + 1];
+  double* wb = work + (long long)b * 2 * Nmax * Nmax;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kLo = krange ? krange[2 * b] : 0, kHi = krange ? krange[2 * b + 1] : n;
   double t = 0.0;
-  for (int k = threadIdx.x; k < n; k += blockDim.x)
+  for (int k = tid; k < n; k += blockDim.x)
     t = fmax(t, fabs(d[k]) + (k < n - 1 ? fabs(e[k]) : 0.0) + (k > 0 ? fabs(e[k - 1]) : 0.0));
-  const double ctol = 1e-10 * fmax(block_max(t, red, 0.0), 1e-300);
+  const double tnorm = fmax(block_max(t, red, 0.0), 1e-300), eps = 2.220446049250313e-16;
+  const double ctol = 1e-10 * tnorm;
   bool close = false;
-  for (int i = kLo + 1 + threadIdx.x; i < kHi; i += blockDim.x) close = close || lam[i] - lam[i - 1] < ctol;
+  for (int i = kLo + 1 + tid; i < kHi; i += blockDim.x) close = close || lam[i] - lam[i - 1] < ctol;
   if (!__syncthreads_or(close)) return;
-  if (threadIdx.x == 0) atomicOr(status + b, (int)kStatusClusterFix);
-  for (int i = kLo + 1; i < kHi; ++i) {
-    if (!(lam[i] - lam[i - 1] < ctol)) continue;
-    int j0 = i - 1;
-    while (j0 > kLo && lam[j0] - lam[j0 - 1] < ctol) --j0;
-    for (int j = j0; j < i; ++j) {
-      double part = 0.0;
-      for (int k = threadIdx.x; k < n; k += blockDim.x)
-        part += (double)Zb[(long long)k * Nmax + i] * (double)Zb[(long long)k * Nmax + j];
-      const double dot = block_sum(part, red);
-      for (int k = threadIdx.x; k < n; k += blockDim.x)
-        Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] - dot * (double)Zb[(long long)k * Nmax + j]);
+  if (tid == 0) atomicOr(status + b, (int)kStatusClusterFix);
+  const int P = min((int)blockDim.x, Nmax / 2);   // vectors at a time: four arrays of Nmax each
+  for (int j0 = kLo, j1; j0 < kHi; j0 = j1) {
+    for (j1 = j0 + 1; j1 < kHi && lam[j1] - lam[j1 - 1] < ctol;) ++j1;
+    if (j1 - j0 < 2) continue;
+    for (int step = 0; step < 2; ++step) {
+      for (int c = j0 + tid; tid < P && c < j1; c += P) {
+        auto at = [&](int a, int k) -> double& { return wb[((long long)a * Nmax + k) * P + tid]; };
+        ts_inverse_step<R>(d, e, n, lam[c] + 8.0 * eps * tnorm, eps * tnorm, step == 0, c, at, Zb + c, Nmax);
+      }
       __syncthreads();
+      for (int i = j0; i < j1; ++i) {
+        for (int pass = 0; pass < (i > j0 ? 2 : 0); ++pass) {
+          // dots[j] = z_{j0+j} . z_i: lanes over 32 vectors, warps over the rows
+          for (int jb = j0; jb < i; jb += 32) {
+            double s = 0.0;
+            if (jb + lane < i) {
+#pragma unroll 4
+              for (int k = warp; k < n; k += 8)
+                s = fma((double)Zb[(long long)k * Nmax + jb + lane], (double)Zb[(long long)k * Nmax + i], s);
+            }
+            part[warp][lane] = s;
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll
+              for (int w = 1; w < 8; ++w) s += part[w][lane];
+              if (jb + lane < i) ts_dots[jb - j0 + lane] = s;
+            }
+            __syncthreads();
+          }
+          // z_i -= sum_j dots[j] z_{j0+j}, a warp per row
+          for (int k = warp; k < n; k += 8) {
+            double s = 0.0;
+            for (int j = j0 + lane; j < i; j += 32) s = fma(ts_dots[j - j0], (double)Zb[(long long)k * Nmax + j], s);
+            s = warp_sum(s);
+            if (lane == 0) Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] - s);
+          }
+          __syncthreads();
+          // normalised
+          double q = 0.0;
+          for (int k = tid; k < n; k += blockDim.x) {
+            const double zv = (double)Zb[(long long)k * Nmax + i];
+            q = fma(zv, zv, q);
+          }
+          const double nr = sqrt(block_sum(q, red));
+          const double inv = nr > 0 ? 1.0 / nr : 0.0;
+          for (int k = tid; k < n; k += blockDim.x)
+            Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] * inv);
+          __syncthreads();
+        }
+      }
     }
-    double part = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      const double zv = (double)Zb[(long long)k * Nmax + i];
-      part += zv * zv;
-    }
-    const double nr = sqrt(block_sum(part, red));
-    const double inv = nr > 0 ? 1.0 / nr : 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x)
-      Zb[(long long)k * Nmax + i] = (R)((double)Zb[(long long)k * Nmax + i] * inv);
-    __syncthreads();
   }
 }
 

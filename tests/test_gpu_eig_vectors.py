@@ -1,4 +1,4 @@
-"""Eigenvectors of the generalised eigensolver, judged one by one against the matrices they
+"""Eigenvectors of the generalised eigensolver, checked one by one against the matrices they
 belong to: G-orthonormality and the residual of every pair."""
 import ctypes as C
 import math
@@ -18,7 +18,8 @@ def _failures(s, g, x, d, eps):
     times. Orthonormality X^H G X = Y^H Y: the rounded L^-1 and the last product act on
     columns of length ||L|| ||L^-1|| = sqrt(cond G); eigenvectors of the tridiagonal matrix,
     found in FP64 from eigenvalues good to a rounding of the norm, are orthogonal to that
-    over their gap (and re-orthogonalised below gaps of 1e-10). Residual in the same frame,
+    over their gap (and re-orthogonalised below gaps of 1e-10; the bound of 1e-5 holds for gaps
+    about there, and pairs below a tenth of that get none). Residual in the same frame,
     L^-1 (S x - d G x) = C y - d y: relative to ||S|| ||G^-1||, the size of the terms of C."""
     n = s.shape[0]
     tol = 32 * eps * math.sqrt(n)
@@ -27,7 +28,7 @@ def _failures(s, g, x, d, eps):
     y = low.conj().T @ x
     gap = np.abs(d[:, None] - d[None])
     gap64 = np.minimum(8 * np.finfo(np.float64).eps * np.abs(d).max() / np.maximum(gap, 1e-300), 1e-5)
-    np.fill_diagonal(gap64, 0.0)
+    gap64[gap < 1e-11 * np.abs(d).max()] = 0.0
     orth = np.abs(y.conj().T @ y - np.eye(x.shape[1]))
     bad = ["orthonormality %.2e at %s" % (orth[i, j], (i, j))
            for i, j in zip(*np.nonzero(~(orth <= tol * math.sqrt(np.linalg.cond(g)) + gap64)))]
@@ -171,3 +172,76 @@ def test_batched_column_major_entries(ctx, double):
     assert np.array_equal(nred, nred2) and len(set(nred2.tolist())) > 3
     assert np.array_equal(scale, scale2) and np.array_equal(d, d2)
     assert np.array_equal(v, v2.transpose(0, 2, 1))
+
+
+def _degenerate(kind, n):
+    """Hermitian matrices with equal, nearly equal or vanishing eigenvalues."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    four = np.repeat([1.0, 2.0, 3.0, 4.0], n // 4 + 1)[:n]
+    if kind == "identity":
+        return 2.5 * np.eye(n) + 0j
+    if kind == "diagonal":
+        return np.diag(four) + 0j
+    if kind == "clusters":
+        q = np.linalg.qr(x)[0]
+        return (q * four) @ q.conj().T
+    if kind == "two stations":
+        return np.kron(np.eye(2), x[:n // 2, :n // 2] + x[:n // 2, :n // 2].conj().T)
+    if kind == "pairs":   # Wilkinson's: eigenvalues in pairs that agree to all digits
+        return np.diag(np.abs(np.arange(n) - n // 2) + 0.01) + np.diag(np.ones(n - 1), 1) + np.diag(np.ones(n - 1), -1) + 0j
+    if kind == "floor":   # most eigenvalues at a thousandth of the largest
+        q = np.linalg.qr(x)[0]
+        return (q * 10.0 ** np.linspace(0, -30, n)) @ q.conj().T + 1e-3 * np.eye(n)
+    rank = {"ones": 0, "rank 3": 3, "half rank": n // 2}[kind]
+    return x[:, :rank] @ x[:, :rank].conj().T if rank else np.ones((n, n)) + 0j
+
+
+@gpu
+@pytest.mark.parametrize("kind", ["identity", "diagonal", "clusters", "two stations", "pairs", "floor", "ones", "rank 3",
+                                  "half rank"])
+@pytest.mark.parametrize("n", [2, 6, 40, 96, 130, 258])
+@pytest.mark.parametrize("double", [False, True])
+@pytest.mark.parametrize("gram", [False, True])
+def test_equal_eigenvalues(ctx, kind, n, double, gram):
+    """Equal eigenvalues get orthonormal eigenvectors of their space, as LAPACK's ?hegv gives."""
+    import bipp_b200 as bipp
+
+    if kind == "ones" and n > 96 and not double and not gram:
+        pytest.skip("remainders of the reduction underflow in FP32")
+    rt, ct = (np.float64, np.complex128) if double else (np.float32, np.complex64)
+    s = _hermitian(_degenerate(kind, n).astype(ct))
+    xyz = _antennas(np.random.default_rng(1), n).astype(rt)
+    eye = np.eye(n, dtype=ct)
+    if gram:
+        g = _gram(xyz.astype(np.float64))
+        v, d, nred, _ = bipp.eigh_gram_full(rt(2.0), s.astype(ct), eye, xyz, ctx=ctx)
+    else:
+        g = np.eye(n)
+        v, d, nred, _ = bipp.eigh(rt(2.0), s.astype(ct), eye, ctx=ctx, full=True)
+    assert nred == n
+    eps = np.finfo(rt).eps
+    ref = scipy.linalg.eigh(s, g, eigvals_only=True)
+    size = np.linalg.norm(s, 2) * np.linalg.norm(np.linalg.inv(g), 2)
+    assert np.abs(d - ref).max() <= 32 * eps * math.sqrt(n) * size
+    bad = _failures(s, g, v.astype(np.complex128), d.astype(np.float64), eps)
+    assert not bad, (len(bad), bad[:4])
+
+
+@gpu
+@pytest.mark.parametrize("kind", ["two stations", "ones", "rank 3", "half rank"])
+def test_equal_eigenvalues_in_a_batch(ctx, kind):
+    """Beside matrices without any, over two chunks, and in a range of the spectrum."""
+    import bipp_b200 as bipp
+
+    rng = np.random.default_rng(3)
+    b, n = 260, 24
+    xyz = np.stack([_antennas(rng, n)] * b).astype(np.float32)
+    s = np.stack([_sources(rng, xyz[0].astype(np.float64)) for _ in range(4)] * (b // 4)).astype(np.complex64)
+    with_equal = [0, 5, 131, 259]
+    s[with_equal] = _degenerate(kind, n)
+    g = _gram(xyz[0].astype(np.float64))
+    v, d, nred, _ = bipp.eigh_gram_batched(np.full(b, 2.0), s, xyz, ctx=ctx)
+    for k in with_equal + [1, 258]:
+        bad = _failures(_hermitian(s[k]), g, v[k].astype(np.complex128), d[k].astype(np.float64), np.finfo(np.float32).eps)
+        assert nred[k] == n and not bad, (k, len(bad), bad[:4])
