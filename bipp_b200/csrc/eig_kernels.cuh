@@ -707,32 +707,54 @@ constexpr int kTrdThreads = 1024;   // upper bound (launch bounds); see trd_thre
 // at barriers, so several CTAs share an SM and hide each other's barrier waits
 inline int trd_threads(int Nmax) { return Nmax <= 256 ? 256 : Nmax <= 512 ? 512 : 1024; }
 
+// Reflector I - tau v v^H that takes (alpha, x), |x|^2 = xnorm2, to (beta, 0): v = (1, sc x)
+template <typename C, typename R>
+__device__ __forceinline__ void hh_reflector(C alpha, R xnorm2, C& tau, C& sc, R& beta) {
+  tau = sc = mk(R(0), R(0));
+  beta = alpha.x;
+  if (!(xnorm2 == R(0) && alpha.y == R(0))) {
+    const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2);
+    beta = (alpha.x >= R(0)) ? -nrm : nrm;
+    tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
+    const C am = mk(alpha.x - beta, alpha.y);
+    const R den = am.x * am.x + am.y * am.y;
+    sc = mk(am.x / den, -am.y / den);
+  }
+}
+
+// FP32 columns whose squares come near the underflow (the remainders of exactly low-rank
+// matrices shrink by a rounding per column) would give reflectors that are not unitary: below
+// kHhTiny the squared norm is formed again from the entries times kHhUp, which tau does not
+// depend on, and a column still below it is taken as zero
+constexpr float kHhTiny = 1e-24f, kHhUp = 1.152921504606846976e18f, kHhDown = 1.0f / kHhUp;   // 2^60
+template <typename C, typename R>
+__device__ __forceinline__ bool hh_underflows(C alpha, R xnorm2) {
+  return sizeof(R) == 4 && cabs2(alpha) + xnorm2 < R(kHhTiny);
+}
+
 template <typename C, typename R>
 __device__ __forceinline__ void householder(C* __restrict__ col, int m, C* __restrict__ v, R* red,
                                             C& tauOut, R& betaOut) {
   // col[0..m): alpha = col[0], x = col[1..m). Produces v[0..m) in smem (v[0] = 1).
   R part = 0;
   for (int r = 1 + threadIdx.x; r < m; r += blockDim.x) part += cabs2(col[r]);
-  const R xnorm2 = block_sum(part, red);
-  const C alpha = col[0];
-  C tau;
-  R beta;
-  if (xnorm2 == R(0) && alpha.y == R(0)) {
-    tau = mk(R(0), R(0));
-    beta = alpha.x;
-    for (int r = threadIdx.x; r < m; r += blockDim.x) v[r] = mk(r == 0 ? R(1) : R(0), R(0));
-  } else {
-    const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2);
-    beta = (alpha.x >= R(0)) ? -nrm : nrm;
-    tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
-    // scale = 1 / (alpha - beta)
-    const C am = mk(alpha.x - beta, alpha.y);
-    const R den = am.x * am.x + am.y * am.y;
-    const C sc = mk(am.x / den, -am.y / den);
-    for (int r = threadIdx.x; r < m; r += blockDim.x) v[r] = (r == 0) ? mk(R(1), R(0)) : cmul(col[r], sc);
+  R xnorm2 = block_sum(part, red), up = R(1), down = R(1);
+  const C zero = mk(R(0), R(0));
+  C alpha = col[0];
+  if (hh_underflows(alpha, xnorm2)) {
+    up = R(kHhUp), down = R(kHhDown);
+    part = 0;
+    for (int r = 1 + threadIdx.x; r < m; r += blockDim.x) part += cabs2(cscale(col[r], up));
+    xnorm2 = block_sum(part, red);
+    alpha = cscale(alpha, up);
+    if (hh_underflows(alpha, xnorm2)) alpha = zero, xnorm2 = R(0);
   }
+  C tau, sc;
+  R beta;
+  hh_reflector(alpha, xnorm2, tau, sc, beta);
+  for (int r = threadIdx.x; r < m; r += blockDim.x) v[r] = r == 0 ? mk(R(1), R(0)) : cmul(cscale(col[r], up), sc);
   tauOut = tau;
-  betaOut = beta;
+  betaOut = beta * down;
 }
 
 // Reduce G per-lane values over the 32 lanes of a warp so that column k's total ends in

@@ -327,27 +327,39 @@ __device__ __forceinline__ void ht_matrix(C* __restrict__ A, int n, int ld, doub
       if (lane == 0) sNorm[warp] = part2;
       __syncthreads();
       // reflector
-      const C alpha = sAlpha;
-      R xnorm2 = 0;
+      C alpha = sAlpha;
+      R xnorm2 = 0, up = R(1), down = R(1);
 #pragma unroll
       for (int w = 0; w < kHtWarps; ++w) xnorm2 += sNorm[w];
-      C tau = zero, sc = zero;
-      R beta = alpha.x;
-      if (!(xnorm2 == R(0) && alpha.y == R(0))) {
-        const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2);
-        beta = (alpha.x >= R(0)) ? -nrm : nrm;
-        tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
-        const C am = mk(alpha.x - beta, alpha.y);
-        const R den = am.x * am.x + am.y * am.y;
-        sc = mk(am.x / den, -am.y / den);
+      if (hh_underflows(alpha, xnorm2)) {   // the same in every thread of the cluster
+        up = R(kHhUp), down = R(kHhDown);
+        part2 = 0;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const int r = tid + kHtThreads * i;
+          if (r > c + 1 && r < n) part2 += cabs2(cscale(col[i], up));
+        }
+        part2 = warp_sum(part2);
+        __syncthreads();
+        if (lane == 0) sNorm[warp] = part2;
+        __syncthreads();
+        xnorm2 = 0;
+#pragma unroll
+        for (int w = 0; w < kHtWarps; ++w) xnorm2 += sNorm[w];
+        alpha = cscale(alpha, up);
+        if (hh_underflows(alpha, xnorm2)) alpha = zero, xnorm2 = R(0);
       }
+      C tau, sc;
+      R beta;
+      hh_reflector(alpha, xnorm2, tau, sc, beta);
+      beta *= down;
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
         const int r = tid + kHtThreads * i;
         v[i] = zero;
         if (r == c) x[r] = zero;   // leaves the trailing block
         if (r > c && r < n) {
-          v[i] = r == c + 1 ? mk(R(1), R(0)) : cmul(col[i], sc);
+          v[i] = r == c + 1 ? mk(R(1), R(0)) : cmul(cscale(col[i], up), sc);
           x[r] = v[i];
           P.set(P.row(r), j, 0, v[i]);
         }
@@ -549,22 +561,28 @@ hetrd_small_kernel(C* __restrict__ A, const int* __restrict__ nred, int ld, doub
     part = warp_sum(part);
     if (lane == 0) sNorm[warp] = part;
     __syncthreads();
-    R xnorm2 = 0;
+    R xnorm2 = 0, up = R(1), down = R(1);
 #pragma unroll
     for (int w = 0; w < NW; ++w) xnorm2 += sNorm[w];
-    const C alpha = col[c + 1];
-    C tau = zero, sc = zero;
-    R beta = alpha.x;
-    if (!(xnorm2 == R(0) && alpha.y == R(0))) {
-      const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2);
-      beta = (alpha.x >= R(0)) ? -nrm : nrm;
-      tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
-      const C am = mk(alpha.x - beta, alpha.y);
-      const R den = am.x * am.x + am.y * am.y;
-      sc = mk(am.x / den, -am.y / den);
+    C alpha = col[c + 1];
+    if (hh_underflows(alpha, xnorm2)) {   // the same in every thread
+      up = R(kHhUp), down = R(kHhDown);
+      part = warp_sum(p == 0 && i > c + 1 && i < n ? cabs2(cscale(col[i], up)) : R(0));
+      __syncthreads();
+      if (lane == 0) sNorm[warp] = part;
+      __syncthreads();
+      xnorm2 = 0;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) xnorm2 += sNorm[w];
+      alpha = cscale(alpha, up);
+      if (hh_underflows(alpha, xnorm2)) alpha = zero, xnorm2 = R(0);
     }
+    C tau, sc;
+    R beta;
+    hh_reflector(alpha, xnorm2, tau, sc, beta);
+    beta *= down;
     const bool in = i > c && i < n;
-    const C v = in ? (i == c + 1 ? mk(R(1), R(0)) : cmul(col[i], sc)) : zero;
+    const C v = in ? (i == c + 1 ? mk(R(1), R(0)) : cmul(cscale(col[i], up), sc)) : zero;
     if (p == 0) {
       vs[i] = v;
       if (in) Ab[i + (long long)c * ld] = i == c + 1 ? mk(beta, R(0)) : v;

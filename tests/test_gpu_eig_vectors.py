@@ -207,8 +207,6 @@ def test_equal_eigenvalues(ctx, kind, n, double, gram):
     """Equal eigenvalues get orthonormal eigenvectors of their space, as LAPACK's ?hegv gives."""
     import bipp_b200 as bipp
 
-    if kind == "ones" and n > 96 and not double and not gram:
-        pytest.skip("remainders of the reduction underflow in FP32")
     rt, ct = (np.float64, np.complex128) if double else (np.float32, np.complex64)
     s = _hermitian(_degenerate(kind, n).astype(ct))
     xyz = _antennas(np.random.default_rng(1), n).astype(rt)
@@ -245,3 +243,17 @@ def test_equal_eigenvalues_in_a_batch(ctx, kind):
     for k in with_equal + [1, 258]:
         bad = _failures(_hermitian(s[k]), g, v[k].astype(np.complex128), d[k].astype(np.float64), np.finfo(np.float32).eps)
         assert nred[k] == n and not bad, (k, len(bad), bad[:4])
+
+
+@gpu
+@pytest.mark.parametrize("n", [130, 500, 700, 1030])
+def test_reduction_of_an_exact_low_rank_matrix(ctx, n):
+    """All ones in FP32: what is left of the matrix shrinks by a rounding per column, and its
+    squares underflow after three (1030 rows: the panel kernel, 130 and more the clusters)."""
+    import bipp_b200 as bipp
+
+    s = np.ones((n, n), np.complex64)
+    v, d, nred, _ = bipp.eigh(np.float32(2.0), s, np.eye(n, dtype=np.complex64), ctx=ctx, full=True)
+    bad = _failures(s.astype(np.complex128), np.eye(n), v.astype(np.complex128), d.astype(np.float64),
+                    np.finfo(np.float32).eps)
+    assert nred == n and not bad, (len(bad), bad[:4])
